@@ -107,18 +107,6 @@ __device__ inline C32 load_pos(const PartC32& a, long long p) {
   return r;
 }
 
-// The same with streaming (evict-first) loads: for the passes that read every
-// particle once, so that the 7.8 GB particle stream does not push the E table
-// or the density accumulators out of L2.
-__device__ inline C32 load_pos_cs(const PartC32& a, long long p) {
-  C32 r;
-  unpack_cell(__ldcs(a.cell + p), r.i, r.j, r.k);
-  r.f[0] = __ldcs(a.fx + p);
-  r.f[1] = __ldcs(a.fy + p);
-  r.f[2] = __ldcs(a.fz + p);
-  return r;
-}
-
 // Move one axis by d cells (FP32, in cell units) in 32-bit fixed point: d is
 // scaled to 2^-32 cells (exact when |d| >= 2^-9, else rounded to the nearest
 // 2^-32), added to the offset, and the whole cells of the sum move the index.
@@ -588,113 +576,255 @@ __global__ void deposit_c32_kernel(KParams P, PartC32 a, long long n, unsigned l
 // ParticlesGridify.f90:65-123, shared-memory tiled, one tile per warp.
 // Particles are stored in cell order (initialisation and every append go cell
 // by cell; compaction keeps the order) and move a small fraction of a cell per
-// step, so a warp's kDepWarpChunk consecutive particles (one or two cells
-// at 64 per cell) touch a small box of nodes.  Each warp takes the bounding
-// box of its particles' CIC stencils (base node + 1 on every axis, by
-// species) with warp reductions, accumulates the fixed-point weights in its
-// own slice of shared memory with 32-bit atomics -- weights lie in [0, 2^40],
-// split into 20-bit halves so neither half-sum can overflow -- and adds every
-// touched node to global memory once, with the ghost folds applied.  A warp
-// whose box does not fit its slice (a row or plane boundary, or a particle
-// far from the rest after BCoutflow filled a hole) falls back to one global
-// atomic per particle corner.  Warps synchronise only with themselves: no
-// block barrier holds a warp's loads behind another warp's atomics.
-// Integer sums are exact and order-independent: N is bit-identical to the
-// warp-aggregated kernel's.
-constexpr int kDepPer = 2;                       // particles per lane
-constexpr int kDepWarpChunk = 32 * kDepPer;      // particles per warp iteration
-constexpr int kDepWarpTile = 512;                // tile entries per warp (two u32 halves each: 4 KB)
-constexpr int kDepWarps = 8;                     // warps per CTA
+// step, so a warp's 32 PER consecutive particles touch a small box of nodes.
+// Each warp takes the bounding box of its particles' CIC stencils (base node
+// + 1 on every axis, by species) with warp reductions, accumulates the
+// fixed-point weights in its own slice of shared memory with 32-bit atomics --
+// weights lie in [0, 2^40], split into 20-bit halves so neither half-sum can
+// overflow -- and adds every touched node to global memory once, with the
+// ghost folds applied.  Warps synchronise only with themselves: no block
+// barrier holds a warp's loads behind another warp's atomics.  Integer sums
+// are exact and order-independent: N is bit-identical to the warp-aggregated
+// kernel's.
+//
+// What bounds it is the shared-memory pipe (16 atomics per particle, each
+// warp-level atomic taking as many wavefronts as lanes meet in one bank) and
+// instruction issue.  So
+// - a lane takes PER consecutive particles (16-byte loads) rather than every
+//   32nd: at one time the lanes stand in several cells;
+// - lane l visits the eight corners in the order q ^ (l & 7), so lanes that
+//   share a base node add to different nodes (the weights of the swapped
+//   corners come from |x - c| with a per-lane c: no extra instructions);
+// - the loop over a lane's groups of four stays rolled: with eight particles
+//   and the far path unrolled, warps waited on instruction fetches most;
+// - the flush clears what it reads, so no pass zeroes the tile.
+// Before: every 32nd particle to a lane, two per lane, corners in one order.
+// ParticlesGridify in us, before and now: 67 M particles at 64 per cell (128 x
+// 128 x 64) 984 and 687, 11.9 M at 26 per cell (77^3) 228 and 154, 8.0 M at 10
+// per cell (93^3) 212 and 143, 3.5 M at 128 per cell, 60 steps of a tenth of a
+// cell after their creation (30^3), 292 and 145.
+// A warp whose box does not fit its slice (a row boundary, or a particle that
+// filled a hole of BCoutflow far from where it was created) takes the
+// particles within a window around its own cells first, those around the
+// first one left over in a second pass when there are many, and adds the
+// corners of what then remains to global memory directly.
+constexpr int kDepTile = 768;   // tile entries per warp (two u32 halves each: 6 KB)
+constexpr int kDepWarps = 8;    // warps per CTA
+constexpr int kDepCtas = 4;     // CTAs per SM (64 registers, 48 KB)
+constexpr unsigned kDepFew = 16;  // not worth a pass over the tile
+constexpr int kDepSide = 2;     // the window: x +- reach, y and z +- kDepSide
 
-__global__ void __launch_bounds__(256, 4) deposit_tile_c32_kernel(KParams P, PartC32 a, long long n,
-                                                                  unsigned long long* Nacc) {
-  extern __shared__ unsigned int dep_tile[];  // per warp: [2][kDepWarpTile] low and high 20-bit halves
+__device__ __forceinline__ uint32_t cell_x(uint32_t c) { return c & kCellMaskX; }
+__device__ __forceinline__ uint32_t cell_y(uint32_t c) { return (c >> kCellBitsX) & kCellMaskY; }
+__device__ __forceinline__ uint32_t cell_z(uint32_t c) { return c >> (kCellBitsX + kCellBitsY); }
+
+// v / d = (v small_inv(d)) >> 16 for 0 <= v < 1024 and 1 <= d <= 64: the
+// excess of the rounded-up reciprocal adds less than v d / 65536 < 1.
+__device__ __forceinline__ uint32_t small_inv(int d) { return (65535u + uint32_t(d)) / uint32_t(d); }
+
+// 1 + f / 2^32 in one 32 x 32 + 64-bit multiply-add (the bits of off_one_plus).
+__device__ __forceinline__ double one_plus(uint32_t f) {
+  return __longlong_as_double((long long)((unsigned long long)f * 1048576ull + 0x3FF0000000000000ull));
+}
+
+// Bounding box of a warp's CIC base nodes (packed cell fields) by species.
+struct DepBox {
+  int imin, imax, jmin, jmax, kmin, kmax, smin, smax;
+};
+
+// One particle into the lane's running box: z, y and x are compared as the top
+// bits of the packed word shifted up by 0, 10 and 21.
+struct DepBoxLane {
+  uint32_t zl = ~0u, zh = 0, yl = ~0u, yh = 0, xl = ~0u, xh = 0, sl = ~0u, sh = 0;
+  __device__ __forceinline__ void add(uint32_t c, uint32_t s) {
+    const uint32_t y = c << kCellBitsZ, x = c << (kCellBitsY + kCellBitsZ);
+    zl = min(zl, c), zh = max(zh, c);
+    yl = min(yl, y), yh = max(yh, y);
+    xl = min(xl, x), xh = max(xh, x);
+    sl = min(sl, s), sh = max(sh, s);
+  }
+  __device__ __forceinline__ DepBox reduce() const {
+    constexpr int sy = kCellBitsX + kCellBitsZ, sx = kCellBitsY + kCellBitsZ;
+    DepBox B;
+    B.kmin = int(cell_z(__reduce_min_sync(0xffffffffu, zl))), B.kmax = int(cell_z(__reduce_max_sync(0xffffffffu, zh)));
+    B.jmin = int(__reduce_min_sync(0xffffffffu, yl) >> sy), B.jmax = int(__reduce_max_sync(0xffffffffu, yh) >> sy);
+    B.imin = int(__reduce_min_sync(0xffffffffu, xl) >> sx), B.imax = int(__reduce_max_sync(0xffffffffu, xh) >> sx);
+    B.smin = int(__reduce_min_sync(0xffffffffu, sl)), B.smax = int(__reduce_max_sync(0xffffffffu, sh));
+    return B;
+  }
+};
+
+// Tile entries of a box, 0 when it does not fit a warp's slice.
+__device__ __forceinline__ int dep_volume(const DepBox& B) {
+  const int bi = B.imax - B.imin + 2, bj = B.jmax - B.jmin + 2, bk = B.kmax - B.kmin + 2, bs = B.smax - B.smin + 1;
+  if (bi > 64 || bj > 64 || bk > 64) return 0;
+  const int vol = bi * bj * bk * bs;  // at most 64^3 * 8
+  return vol <= kDepTile ? vol : 0;
+}
+
+// V consecutive words of a lane (V = 4 by a 16-byte load, 2 by an 8-byte one).
+template <int V>
+__device__ __forceinline__ uint4 load_group(const uint32_t* p) {
+  if (V == 4) return __ldcs(reinterpret_cast<const uint4*>(p));
+  const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p));
+  return make_uint4(v.x, v.y, 0u, 0u);
+}
+template <int V>
+__device__ __forceinline__ uint32_t load_species(const int8_t* p) {
+  if (V == 4) return __ldcs(reinterpret_cast<const uint32_t*>(p));
+  return __ldcs(reinterpret_cast<const uint16_t*>(p));
+}
+
+__device__ __forceinline__ uint32_t word4(const uint4& v, int m) { return m == 0 ? v.x : m == 1 ? v.y : m == 2 ? v.z : v.w; }
+
+template <int PER>
+__global__ void __launch_bounds__(256, kDepCtas) deposit_tile_c32_kernel(KParams P, PartC32 a, long long n,
+                                                                   unsigned long long* Nacc, uint32_t reach) {
+  static_assert(PER == 2 || PER == 4 || PER == 8, "loads of two or four particles");
+  constexpr int V = PER < 4 ? PER : 4, kGroups = PER / V;
+  constexpr unsigned kAll = (1u << PER) - 1u;
+  extern __shared__ unsigned int dep_tile[];  // per warp: [2][kDepTile] low and high 20-bit halves
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned int* lo = dep_tile + warp * 2 * kDepWarpTile;
-  unsigned int* hi = lo + kDepWarpTile;
+  unsigned int* lo = dep_tile + warp * 2 * kDepTile;
+  constexpr int kHi = kDepTile;  // lo[e + kHi]: the high half of entry e
+  int zeroed = 0;  // entries below this are zero between chunks: the flush clears what it reads
+  // weight of the corner that the lane visits first on an axis: |(1 + f) - c|,
+  // c = 2 for the lower node (1 - f), 1 for the upper one (f)
+  const bool sx = lane & 1, sy = lane & 2, sz = lane & 4;
+  const double cx = sx ? 1.0 : 2.0, cy = sy ? 1.0 : 2.0, cz = sz ? 1.0 : 2.0;
   const long long warps = (long long)gridDim.x * kDepWarps;
-  for (long long base = ((long long)blockIdx.x * kDepWarps + warp) * kDepWarpChunk; base < n;
-       base += warps * kDepWarpChunk) {
-    C32 c[kDepPer];
-    int sp[kDepPer];
-    bool act[kDepPer];
-    int imin = INT_MAX, imax = INT_MIN, jmin = INT_MAX, jmax = INT_MIN, kmin = INT_MAX, kmax = INT_MIN;
-    int smin = INT_MAX, smax = INT_MIN;
-#pragma unroll
-    for (int m = 0; m < kDepPer; ++m) {
-      const long long p = base + lane + 32 * m;
-      act[m] = p < n;
-      if (act[m]) {
-        c[m] = load_pos_cs(a, p);
-        sp[m] = __ldcs(a.sp + p);
-        imin = min(imin, c[m].i), imax = max(imax, c[m].i);
-        jmin = min(jmin, c[m].j), jmax = max(jmax, c[m].j);
-        kmin = min(kmin, c[m].k), kmax = max(kmax, c[m].k);
-        smin = min(smin, sp[m]), smax = max(smax, sp[m]);
-      }
-    }
-    // the warp's bounding box (lane 0 always holds a particle: base < n)
-    imin = __reduce_min_sync(0xffffffffu, imin), imax = __reduce_max_sync(0xffffffffu, imax);
-    jmin = __reduce_min_sync(0xffffffffu, jmin), jmax = __reduce_max_sync(0xffffffffu, jmax);
-    kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
-    smin = __reduce_min_sync(0xffffffffu, smin), smax = __reduce_max_sync(0xffffffffu, smax);
-    const long long bi = (long long)imax - imin + 2, bj = (long long)jmax - jmin + 2, bk = (long long)kmax - kmin + 2,
-                    bs = (long long)smax - smin + 1;
-    const long long vol = bi * bj * bk * bs;
-    if (vol <= kDepWarpTile) {
-      const int vi = int(vol);
-      for (int e = lane; e < vi; e += 32) lo[e] = 0u, hi[e] = 0u;
-      __syncwarp();
-#pragma unroll
-      for (int m = 0; m < kDepPer; ++m) {
-        if (!act[m]) continue;
-        long long w[8];
-        double F[8];
-        cic_fixed_c32(c[m], w, F);
-        const int b0 = (((sp[m] - smin) * int(bk) + (c[m].k - kmin)) * int(bj) + (c[m].j - jmin)) * int(bi) +
-                       (c[m].i - imin);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const unsigned long long wq = (unsigned long long)w[q];
-          const int e = b0 + (corner(q, 2) * int(bj) + corner(q, 1)) * int(bi) + corner(q, 0);
-          atomicAdd(lo + e, unsigned(wq & 0xFFFFFu));
-          atomicAdd(hi + e, unsigned(wq >> 20));
-        }
-      }
-      __syncwarp();
-      for (int e = lane; e < vi; e += 32) {
-        const unsigned l = lo[e], h = hi[e];
-        if ((l | h) == 0u) continue;
-        int r = e;
-        const int ii = r % int(bi) + imin;
-        r /= int(bi);
-        const int jj = r % int(bj) + jmin;
-        r /= int(bj);
-        const int kk = r % int(bk) + kmin;
-        const int ss = r / int(bk) + smin;
-        const int i = fold_index(ii, P.nx, P.xflow), j = fold_index(jj, P.ny, P.yflow),
-                  k = fold_index(kk, P.nz, P.zflow);
-        const unsigned long long v = ((unsigned long long)h << 20) + (unsigned long long)l;
-        atomicAdd(Nacc + (long long)ss * P.nodes + node_index(P, i, j, k), v);
-      }
-      __syncwarp();
+  for (long long base = ((long long)blockIdx.x * kDepWarps + warp) * (32 * PER); base < n; base += warps * (32 * PER)) {
+    // the lane's group g of V consecutive particles starts at p0 + 16 g: four
+    // lanes read 64 contiguous bytes of every array at a time (PER = 8)
+    const long long p0 = base + V * ((lane >> 2) * 4 * kGroups + (lane & 3));
+    unsigned left = kAll;  // this lane's particles not deposited yet
+    if (base + 32 * PER > n) {  // the last, partial chunk of the array
+#pragma unroll 1
+      for (int m = 0; m < PER; ++m)
+        if (p0 + 16 * (m / V) + m % V >= n) left &= ~(1u << m);
     } else {
+      uint4 cell[kGroups];
+      uint32_t sp[kGroups];
+      DepBoxLane L;
 #pragma unroll
-      for (int m = 0; m < kDepPer; ++m) {
-        if (!act[m]) continue;
-        long long w[8];
-        double F[8];
-        cic_fixed_c32(c[m], w, F);
-        unsigned long long* plane = Nacc + (long long)sp[m] * P.nodes;
+      for (int g = 0; g < kGroups; ++g) {
+        cell[g] = load_group<V>(a.cell + p0 + 16 * g);
+        sp[g] = load_species<V>(a.sp + p0 + 16 * g);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int i = fold_index(c[m].i + corner(q, 0), P.nx, P.xflow),
-                    j = fold_index(c[m].j + corner(q, 1), P.ny, P.yflow),
-                    k = fold_index(c[m].k + corner(q, 2), P.nz, P.zflow);
-          atomicAdd(plane + node_index(P, i, j, k), (unsigned long long)w[q]);
+        for (int m = 0; m < V; ++m) L.add(word4(cell[g], m), (sp[g] >> (8 * m)) & 0xFFu);
+      }
+      DepBox B = L.reduce();
+      unsigned near = kAll;
+      int vol = dep_volume(B);
+      for (int pass = 0; pass < 2; ++pass) {
+        if (vol == 0) {
+          // too large: only what lies around the middle one of three cells (so
+          // that one far particle among them does not place the window), or in
+          // the second pass around the first one left
+          uint32_t mid;
+          if (pass == 0) {
+            const uint32_t w0 = a.cell[base], w1 = a.cell[base + 16 * PER], w2 = a.cell[base + 32 * PER - 1];
+            mid = max(min(w0, w1), min(max(w0, w1), w2));
+          } else {
+            const int src = __ffs(__ballot_sync(0xffffffffu, left != 0u)) - 1;
+            const int m = __ffs(left) - 1;
+            mid = a.cell[__shfl_sync(0xffffffffu, p0 + 16 * (m / V) + m % V, src)];
+          }
+          const uint32_t wx = cell_x(mid) - reach, wy = cell_y(mid) - kDepSide, wz = cell_z(mid) - kDepSide;
+          DepBoxLane W;
+          near = 0u;
+#pragma unroll
+          for (int m = 0; m < PER; ++m) {
+            const uint32_t c = word4(cell[m / V], m % V);
+            if ((left >> m & 1u) && cell_x(c) - wx <= 2 * reach && cell_y(c) - wy <= 2 * kDepSide &&
+                cell_z(c) - wz <= 2 * kDepSide) {
+              near |= 1u << m;
+              W.add(c, (sp[m / V] >> (8 * (m % V))) & 0xFFu);
+            }
+          }
+          if (__reduce_add_sync(0xffffffffu, unsigned(__popc(near))) <= kDepFew) break;
+          B = W.reduce();
+          vol = dep_volume(B);
+          if (vol == 0) break;
         }
+        const int bi = B.imax - B.imin + 2, bj = B.jmax - B.jmin + 2, bk = B.kmax - B.kmin + 2;
+        const int sj = bi, sk = bi * bj, ss = sk * bk;
+        if (vol > zeroed) {
+          for (int e = zeroed + lane; e < vol; e += 32) lo[e] = 0u, lo[e + kHi] = 0u;
+          zeroed = vol;
+          __syncwarp();
+        }
+        const int first = (sx ? 1 : 0) + (sy ? sj : 0) + (sz ? sk : 0) - (B.imin + B.jmin * sj + B.kmin * sk + B.smin * ss);
+        const int dx = sx ? -1 : 1, dy = sy ? -sj : sj, dz = sz ? -sk : sk;
+#pragma unroll 1
+        for (int g = 0; g < kGroups; ++g) {
+          const uint4 c4 = g > 0 ? cell[kGroups - 1] : cell[0];
+          const uint32_t s4 = g > 0 ? sp[kGroups - 1] : sp[0];
+          const uint4 fx = load_group<V>(a.fx + p0 + 16 * g);
+          const uint4 fy = load_group<V>(a.fy + p0 + 16 * g);
+          const uint4 fz = load_group<V>(a.fz + p0 + 16 * g);
+#pragma unroll
+          for (int m = 0; m < V; ++m) {
+            if (!(near >> (V * g + m) & 1u)) continue;
+            const uint32_t c = word4(c4, m), s = (s4 >> (8 * m)) & 0xFFu;
+            const double x0 = fabs(one_plus(word4(fx, m)) - cx), y0 = fabs(one_plus(word4(fy, m)) - cy),
+                         z0 = fabs(one_plus(word4(fz, m)) - cz);
+            const double ax[2] = {x0, 1.0 - x0}, ay[2] = {y0, 1.0 - y0}, az[2] = {z0, 1.0 - z0};
+            unsigned int* e0 = lo + (first + int(cell_x(c)) + int(cell_y(c)) * sj + int(cell_z(c)) * sk + int(s) * ss);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const double F = (ax[q & 1] * ay[q >> 1 & 1]) * az[q >> 2];
+              // the bits of 1.5 2^52 + round(F 2^40): the weight's low 20 bits,
+              // and its high ones under a constant top bit that the sum masks off
+              const long long u = __double_as_longlong(fma(F, 1099511627776.0, 6755399441055744.0));
+              unsigned int* e = e0 + ((q & 1) ? dx : 0) + ((q & 2) ? dy : 0) + ((q & 4) ? dz : 0);
+              atomicAdd(e, unsigned(u) & 0xFFFFFu);
+              atomicAdd(e + kHi, unsigned(u >> 20));
+            }
+          }
+        }
+        __syncwarp();
+        // nodes of the box, (field value - 1) a 0-based node; interior boxes need no fold
+        const bool inside = B.imin >= 2 && B.imax < P.nx + 1 && B.jmin >= 2 && B.jmax < P.ny + 1 && B.kmin >= 2 &&
+                            B.kmax < P.nz + 1;
+        const uint32_t ri = small_inv(bi), rj = small_inv(bj), rk = small_inv(bk);
+        for (int e = lane; e < vol; e += 32) {
+          const unsigned l = lo[e], h = lo[e + kHi];
+          if ((l | h) == 0u) continue;
+          lo[e] = 0u, lo[e + kHi] = 0u;
+          const int r1 = int((uint32_t(e) * ri) >> 16), r2 = int((uint32_t(r1) * rj) >> 16),
+                    r3 = int((uint32_t(r2) * rk) >> 16);
+          int i = e - r1 * bi + B.imin - 1, j = r1 - r2 * bj + B.jmin - 1, k = r2 - r3 * bk + B.kmin - 1;
+          if (!inside) {
+            i = fold_index(i, P.nx, P.xflow);
+            j = fold_index(j, P.ny, P.yflow);
+            k = fold_index(k, P.nz, P.zflow);
+          }
+          const unsigned long long v = ((unsigned long long)(h & 0x7FFFFFFFu) << 20) + (unsigned long long)l;
+          atomicAdd(Nacc + (long long)(r3 + B.smin) * P.nodes + node_index(P, i, j, k), v);
+        }
+        __syncwarp();
+        left &= ~near;
+        if (__reduce_add_sync(0xffffffffu, unsigned(__popc(left))) <= kDepFew) break;
+        vol = 0;
       }
     }
+    while (left) {  // one by one, straight to global memory
+      const int m = __ffs(left) - 1;
+      const long long p = p0 + 16 * (m / V) + m % V;
+      left &= left - 1;
+      const C32 c = load_pos(a, p);
+      unsigned long long* plane = Nacc + (long long)a.sp[p] * P.nodes;
+      const double x = one_plus(c.f[0]), y = one_plus(c.f[1]), z = one_plus(c.f[2]);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const double F = (((q & 1) ? x - 1.0 : 2.0 - x) * ((q & 2) ? y - 1.0 : 2.0 - y)) * ((q & 4) ? z - 1.0 : 2.0 - z);
+        const int i = fold_index(c.i + (q & 1), P.nx, P.xflow), j = fold_index(c.j + (q >> 1 & 1), P.ny, P.yflow),
+                  k = fold_index(c.k + (q >> 2), P.nz, P.zflow);
+        atomicAdd(plane + node_index(P, i, j, k), (unsigned long long)fixed40_rn(F));
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -808,25 +938,30 @@ cudaError_t launch_deposit_c32(const KParams& P, PartC32 a, long long n, unsigne
                                unsigned long long* Facc, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (!Facc) {
-    const size_t smem = size_t(kDepWarps) * 2 * sizeof(unsigned int) * kDepWarpTile;
-    static bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(deposit_tile_c32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
-    static int per_sm = 0;
-    if (!per_sm) {
-      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, deposit_tile_c32_kernel, 256, smem);
-      if (e != cudaSuccess) return e;
-      if (per_sm < 1) per_sm = 1;
-    }
-    const long long chunks = (n + kDepWarps * kDepWarpChunk - 1) / (kDepWarps * kDepWarpChunk),
-                    full = 148LL * per_sm;
+    // Eight particles per lane spread a warp's lanes over more cells (fewer
+    // bank conflicts) and flush a box less often; four where that box would be
+    // mostly empty (few particles per cell) or the array has no two chunks of
+    // eight for every resident warp.  Both, us per ParticlesGridify: 64 per
+    // cell, 67 M particles 687 against 786; 26 per cell, 11.9 M 154 / 162; 24
+    // per cell, 1.56 M 46 / 43; 10 per cell, 8.0 M 172 / 139.
+    // Particles per lane.  Eight spread a warp's lanes over more cells (fewer
+    // bank conflicts) and flush a box less often, four where that box would be
+    // mostly empty (few particles per cell), two where the array has not two
+    // chunks of eight for every resident warp.  us per ParticlesGridify with
+    // 8 / 4 / 2: 64 per cell, 67 M particles 687 / 786 / -; 26 per cell, 11.9 M
+    // 154 / 162 / -; 10 per cell, 8.0 M 172 / 143 / 165; 24 per cell, 1.56 M
+    // 46 / 44 / 40; 8 per cell, 33 k 21.7 / 19.7 / 16.7.
+    const long long cells = (long long)P.nx * P.ny * P.nz, lanes = 148LL * kDepCtas * kDepWarps * 32;
+    const int per = n < 16 * lanes ? 2 : n >= 16 * cells ? 8 : 4;
+    auto* kernel = per == 8 ? deposit_tile_c32_kernel<8> : per == 4 ? deposit_tile_c32_kernel<4> : deposit_tile_c32_kernel<2>;
+    const size_t smem = size_t(kDepWarps) * 2 * sizeof(unsigned int) * kDepTile;  // within the default 48 KB
+    const long long chunk = (long long)kDepWarps * 32 * per;
+    const long long chunks = (n + chunk - 1) / chunk, full = 148LL * kDepCtas;
     const int grid = int(chunks < full ? chunks : full);
     note_launch();
-    deposit_tile_c32_kernel<<<grid, 256, smem, st>>>(P, a, n, Nacc);
+    // the window reaches as far along x as the particles of one warp at this density, and a cell to either side
+    const long long span = (chunk / kDepWarps) * cells / n + 2;
+    kernel<<<grid, 256, smem, st>>>(P, a, n, Nacc, uint32_t(span < 15 ? span : 15));
     return cudaGetLastError();
   }
   note_launch();
