@@ -31,18 +31,21 @@ struct SortBuf {
 // FFT BCpotentials (bcpot_fft.cu): slice transforms of D and stage buffers.
 struct BcFft;
 
-// Closed-form Jacobi solve (spectral.cu): per-axis orthonormal bases of the
-// sweep operator and the compact FP64 interior arrays the transforms use.
+// One axis of the closed-form Jacobi solve (spectral.cu): the orthonormal basis
+// of the sweep operator, folded by its even / odd symmetry (folded_basis).
+struct AxisBasis {
+  int ne = 0, no = 0, s = 0;  // even and odd functions; 0 open, 1 periodic
+  double* Pe = nullptr;       // [ne][ne] even functions, row = mode
+  double* PeT = nullptr;
+  double* Po = nullptr;       // [no][no] odd functions
+  double* PoT = nullptr;
+};
+
+// Closed-form Jacobi solve (spectral.cu): the axis bases and the compact FP64
+// interior arrays the transforms use.  Modes of an axis in the order [even |
+// odd].
 struct SpectralPlan {
-  double* Q[3] = {nullptr, nullptr, nullptr};   // periodic axes: [n_d][n_d], row = mode
-  double* QT[3] = {nullptr, nullptr, nullptr};  // transposes
-  // open axes: the sine basis folded by its even/odd symmetry (spectral.cu
-  // folded_basis), modes in the order [even | odd]
-  int folded[3] = {0, 0, 0};
-  double* Qe[3] = {nullptr, nullptr, nullptr};
-  double* QeT[3] = {nullptr, nullptr, nullptr};
-  double* QoR[3] = {nullptr, nullptr, nullptr};
-  double* QoRT[3] = {nullptr, nullptr, nullptr};
+  AxisBasis ax[3];
   double* om[3] = {nullptr, nullptr, nullptr};  // a_d (2 - sigma_d) per mode
   double* T[2] = {nullptr, nullptr};            // nx*ny*nz each
   double* partial = nullptr;                    // [norm_blocks][32]

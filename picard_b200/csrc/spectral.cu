@@ -24,11 +24,11 @@
 // ||r_d|| <= maxerr ||b|| -- is found by a bracketing search: each launch
 // evaluates the Parseval sum at up to kSpecPoints sweep counts.
 //
-// The transforms are dense per-axis products (FP64, 2n flops per node and
-// axis): the z and y passes multiply Q_d from the left onto planes/rows of
-// the compact interior array, the x pass multiplies rows by Q_x^T from the
-// right.  Everything is FP64; the result equals the FP64 sweeps' iterate to
-// rounding (the sweeps themselves round each of their d updates).
+// The transforms are per-axis products, one launch each, on the FP64 tensor
+// cores (spec_axis_kernel).  Every axis basis is folded by its even / odd
+// symmetry, which halves the flops.  Everything is FP64; the result equals the
+// FP64 sweeps' iterate to rounding (the sweeps themselves round each of their
+// d updates).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -46,17 +46,30 @@ namespace {
 
 constexpr int kSpecPoints = 32;     // sweep counts per evaluation launch
 constexpr int kSpecThreads = 256;
-constexpr int kGemmBM = 64, kGemmBN = 64, kGemmBK = 16;
+constexpr int kAxTile = 64, kAxK = 16;  // spec_axis_kernel: 64 x 64 outputs per parity, K chunks of 16
+
+// Element t of a compact nx x ny array of planes -> (i, j, k).  T is 32 bits
+// wherever the element count allows: the two divisions by run-time extents are
+// most of the integer work of the passes below.
+template <class T>
+__device__ __forceinline__ void split3(T t, int nx, int ny, int& i, int& j, int& k) {
+  const T r = t / T(nx), q = r / T(ny);
+  i = int(t - r * T(nx));
+  j = int(r - q * T(ny));
+  k = int(q);
+}
+inline bool fits32(long long n) { return n < (1LL << 31); }
 
 // r_0 = b - L U over the interior, compact x-fastest (CalcEpotential.f90:83-92;
 // periodic axes read the wrapped interior instead of the ghost).
+template <class T>
 __global__ void spec_r0_kernel(KParams P, double idx2, double idy2, double idz2, const double* __restrict__ U,
                                const double* __restrict__ b, double* __restrict__ R) {
-  const long long n = (long long)P.nx * P.ny * P.nz;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = int(t % P.nx) + 1;
-    const int j = int((t / P.nx) % P.ny) + 1;
-    const int k = int(t / ((long long)P.nx * P.ny)) + 1;
+  const T n = T(P.nx) * T(P.ny) * T(P.nz);
+  for (T t = T(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += T(gridDim.x) * blockDim.x) {
+    int i, j, k;
+    split3(t, P.nx, P.ny, i, j, k);
+    ++i, ++j, ++k;
     const int im = (i == 1 && !P.xflow) ? P.nx : i - 1, ip = (i == P.nx && !P.xflow) ? 1 : i + 1;
     const int jm = (j == 1 && !P.yflow) ? P.ny : j - 1, jp = (j == P.ny && !P.yflow) ? 1 : j + 1;
     const int km = (k == 1 && !P.zflow) ? P.nz : k - 1, kp = (k == P.nz && !P.zflow) ? 1 : k + 1;
@@ -68,70 +81,210 @@ __global__ void spec_r0_kernel(KParams P, double idx2, double idy2, double idz2,
   }
 }
 
-// C[o] (M x N) = A[o] (M x K, K contiguous: A[m*lda + k]) * B[o] (K x N),
-// B[k*ldb + n] (N contiguous) or, with KB, B[n*ldb + k] (K contiguous).
-// Tiles of 64 x 64, K chunks of 16, 256 threads with 4 x 4 outputs each (rows
-// ty + 16a, columns tx + 16c).  Batch o = blockIdx.z with element strides
-// sa, sb, sc.
-template <bool KB>
-__global__ void __launch_bounds__(256) spec_gemm_kernel(const double* __restrict__ A, int lda, long long sa,
-                                                        const double* __restrict__ B, int ldb, long long sb,
-                                                        double* __restrict__ C, int ldc, long long sc, int M, int N,
-                                                        int K) {
-  __shared__ double As[kGemmBK][kGemmBM + 2];
-  __shared__ double Bs[kGemmBK][kGemmBN + 2];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * kGemmBM, n0 = blockIdx.x * kGemmBN;
-  A += sa * blockIdx.z;
-  B += sb * blockIdx.z;
-  C += sc * blockIdx.z;
-  double acc[4][4];
+// D += A B for one 8 x 4 by 4 x 8 FP64 tile: lane l holds A[l / 4][l % 4],
+// B[l % 4][l / 4] and D[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d0), "+d"(d1)
+      : "d"(a), "d"(b));
+}
+
+// One axis pass of the transform.  An axis of length n has `ne` even and `no`
+// odd basis functions about the reflection i -> n - 1 - i + s (s = 0 open, 1
+// periodic, indices mod n): element i < ne stands for itself and, when s <= i
+// < no + s, for its partner n - 1 - i + s, so
+//   forward: out[m] = sum_i Pe[m][i] (x[i] + x[partner]),
+//            out[ne + m] = sum_i Po[m][i - s] (x[i] - x[partner]);
+//   inverse: out[i] = E[i] + O[i], out[partner] = E[i] - O[i], with
+//            E[i] = sum_k Pe[k][i] in[k] and O[i] = sum_k Po[k][i - s] in[ne + k].
+// Both halves read the same input, so one block computes the 64 x 64 outputs
+// of both: warps 0-3 the even half, warps 4-7 the odd one, 32 x 32 each as 4 x
+// 4 tiles of mma.m8n8k4.  The fold is done while the input is staged and the
+// unfold while the output is written, so a pass reads and writes the array
+// once.
+//
+// X: the axis is contiguous (rows of n, `rows` of them): A = data, B = matrix
+// (Pe, Po given as [k][output]).  Else the axis has stride I and the block
+// takes 64 of the I contiguous columns of slab blockIdx.z: A = matrix ([output]
+// [k]), B = data.  APPLY (x, inverse): adds the outputs to U's interior instead
+// of storing them.
+//
+// What bounds it: FP64 (4.3 GFLOP of products for both transforms of 256 x 128
+// x 128, 0.12 ms at 37 TFLOP/s), the fragments being read from shared memory
+// once per 4 x 4 tiles (64 of 256 cycles); small grids are bound by the launch.
+// Both transforms of 256 x 128 x 128 with the update of U: 286 us in 6 launches,
+// against 498 us in 19 for products with 4 x 4 outputs per thread (as many
+// shared-memory as FP64 cycles), in-place butterflies and a pass of its own for
+// the update; 24^3: 28 us against 55 us.
+template <bool INV, bool X, bool APPLY>
+__global__ void __launch_bounds__(256, 2) spec_axis_kernel(const double* __restrict__ in, double* __restrict__ out,
+                                                           const double* __restrict__ Pe,
+                                                           const double* __restrict__ Po, int n, int ne, int no, int s,
+                                                           long long I, int rows, KParams P, double* __restrict__ U) {
+  // row strides 4 mod 16 doubles: the 16 lanes of a half-warp read 16 banks
+  __shared__ double sh[2 * kAxTile * (kAxK + 4) + 2 * kAxK * (kAxTile + 4)];
+  double(*As)[kAxTile][kAxK + 4] = reinterpret_cast<double(*)[kAxTile][kAxK + 4]>(sh);
+  double(*Bs)[kAxK][kAxTile + 4] = reinterpret_cast<double(*)[kAxK][kAxTile + 4]>(sh + 2 * kAxTile * (kAxK + 4));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int par = warp >> 2, wm = (warp >> 1) & 1, wn = warp & 1;
+  const int c0 = blockIdx.x * kAxTile, r0 = blockIdx.y * kAxTile;  // first output column and row of the tile
+  // outputs run over rows (not X) or columns (X); the other index is the data's
+  const int o0 = X ? c0 : r0;
+  const long long v0 = X ? r0 : c0, vn = X ? rows : I;
+  const long long slab = X ? 0 : (long long)blockIdx.z * n * I;
+  in += slab;
+  if (!APPLY) out += slab;
+  const int K = ne;
+  // data element `i` of vector v: even and odd value (i - s: the odd index)
+  auto data = [&](long long v, int i, double& e, double& o) {
+    e = o = 0.0;
+    if (v >= vn || i >= ne) return;
+    const double* x = X ? in + v * n : in + v;
+    const long long st = X ? 1 : I;
+    if (INV) {
+      e = x[(long long)i * st];
+      if (i < no) o = x[(long long)(ne + i) * st];
+    } else {
+      const double a = x[(long long)i * st];
+      if (i >= s && i < no + s) {
+        const double b = x[(long long)(n - 1 - i + s) * st];
+        e = a + b;
+        o = a - b;
+      } else {
+        e = a;
+      }
+    }
+  };
+  // matrix entry of output q (a mode, or INV an element) and summation index k
+  auto matrix = [&](int q, int k, double& e, double& o) {
+    const int qo = INV ? q - s : q, ko = INV ? k : k - s;
+    e = (q < ne && k < ne) ? (X ? Pe[(long long)k * ne + q] : Pe[(long long)q * ne + k]) : 0.0;
+    o = (qo >= 0 && qo < no && ko >= 0 && ko < no) ? (X ? Po[(long long)ko * no + qo] : Po[(long long)qo * no + ko]) : 0.0;
+  };
+  double acc[4][4][2];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = 0.0;
-  for (int k0 = 0; k0 < K; k0 += kGemmBK) {
+    for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+  // rows of this warp's parity that exist at all (uniform per warp)
+  const int lim = INV ? ne : (par ? no : ne);
+  const bool live = X ? (c0 + wn * 32 < lim && r0 + wm * 32 < rows) : (r0 + wm * 32 < lim && v0 + wn * 32 < I);
+  double ae[4], ao[4], be[4], bo[4];
+  auto fetch = [&](int k0) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int q = tid + 256 * e;
-      const int m = q >> 4, k = q & 15;  // A: k fastest
-      const int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < M && gk < K) ? A[(long long)gm * lda + gk] : 0.0;
-      if (KB) {
-        const int n = q >> 4, kk = q & 15;
-        const int gn = n0 + n, gkk = k0 + kk;
-        Bs[kk][n] = (gn < N && gkk < K) ? B[(long long)gn * ldb + gkk] : 0.0;
+      if (X) {
+        data(v0 + (q >> 4), k0 + (q & 15), ae[e], ao[e]);
+        matrix(o0 + (q & 63), k0 + (q >> 6), be[e], bo[e]);
       } else {
-        const int kk = q >> 6, n = q & 63;
-        const int gn = n0 + n, gkk = k0 + kk;
-        Bs[kk][n] = (gn < N && gkk < K) ? B[(long long)gkk * ldb + gn] : 0.0;
+        matrix(o0 + (q >> 4), k0 + (q & 15), ae[e], ao[e]);
+        data(v0 + (q & 63), k0 + (q >> 6), be[e], bo[e]);
+      }
+    }
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += kAxK) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int q = tid + 256 * e;
+      As[0][q >> 4][q & 15] = ae[e];
+      As[1][q >> 4][q & 15] = ao[e];
+      Bs[0][q >> 6][q & 63] = be[e];
+      Bs[1][q >> 6][q & 63] = bo[e];
+    }
+    __syncthreads();
+    if (k0 + kAxK < K) fetch(k0 + kAxK);
+    if (live) {
+#pragma unroll
+      for (int kk = 0; kk < kAxK; kk += 4) {
+        double a[4], b[4];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) a[f] = As[par][wm * 32 + 8 * f + (lane >> 2)][kk + (lane & 3)];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) b[f] = Bs[par][kk + (lane & 3)][wn * 32 + 8 * f + (lane >> 2)];
+#pragma unroll
+        for (int fa = 0; fa < 4; ++fa)
+#pragma unroll
+          for (int fb = 0; fb < 4; ++fb) mma_f64(acc[fa][fb][0], acc[fa][fb][1], a[fa], b[fb]);
       }
     }
     __syncthreads();
+  }
+  if constexpr (INV) {  // the odd half goes to the even warps
+    double(*Os)[kAxTile + 2] = reinterpret_cast<double(*)[kAxTile + 2]>(sh);
+    if (par == 1) {
 #pragma unroll
-    for (int k = 0; k < kGemmBK; ++k) {
-      double av[4], bv[4];
+      for (int fa = 0; fa < 4; ++fa)
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[k][ty + 16 * a];
+        for (int fb = 0; fb < 4; ++fb)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) bv[c] = Bs[k][tx + 16 * c];
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[a][c] = fma(av[a], bv[c], acc[a][c]);
+          for (int t = 0; t < 2; ++t)
+            Os[wm * 32 + 8 * fa + (lane >> 2)][wn * 32 + 8 * fb + 2 * (lane & 3) + t] = acc[fa][fb][t];
     }
     __syncthreads();
-  }
+    if (par == 1) return;
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int gm = m0 + ty + 16 * a;
-    if (gm >= M) continue;
+    for (int fa = 0; fa < 4; ++fa) {
+      const int row = wm * 32 + 8 * fa + (lane >> 2);
+      double* y = nullptr;  // x: the row's first output
+      if constexpr (X) {
+        const unsigned v = unsigned(v0) + row, vk = v / unsigned(P.ny);
+        if (v >= unsigned(rows)) continue;
+        y = APPLY ? U + node_index(P, 1, 1 + int(v - vk * P.ny), 1 + int(vk)) : out + (long long)v * n;
+      }
+      double u0[4][2], u1[4][2];  // APPLY: all of a row's loads before its first store
+      if constexpr (APPLY) {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int gn = n0 + tx + 16 * c;
-      if (gn < N) C[(long long)gm * ldc + gn] = acc[a][c];
+        for (int fb = 0; fb < 4; ++fb)
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const int i = o0 + wn * 32 + 8 * fb + 2 * (lane & 3) + t;
+            u0[fb][t] = i < ne ? y[i] : 0.0;
+            u1[fb][t] = i < ne && i >= s && i < no + s ? y[n - 1 - i + s] : 0.0;
+          }
+      }
+#pragma unroll
+      for (int fb = 0; fb < 4; ++fb)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const int col = wn * 32 + 8 * fb + 2 * (lane & 3) + t;
+          const int i = o0 + (X ? col : row);
+          const double E = acc[fa][fb][t], O = Os[row][col];
+          const bool pair = i >= s && i < no + s;
+          const int j = n - 1 - i + s;
+          if (i >= ne) continue;
+          if constexpr (APPLY) {
+            y[i] = u0[fb][t] + (pair ? E + O : E);
+            if (pair) y[j] = u1[fb][t] + (E - O);
+          } else if constexpr (X) {
+            y[i] = pair ? E + O : E;
+            if (pair) y[j] = E - O;
+          } else {
+            const long long v = v0 + col;
+            if (v >= I) continue;
+            out[(long long)i * I + v] = pair ? E + O : E;
+            if (pair) out[(long long)j * I + v] = E - O;
+          }
+        }
     }
+  } else {
+#pragma unroll
+    for (int fa = 0; fa < 4; ++fa)
+#pragma unroll
+      for (int fb = 0; fb < 4; ++fb)
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const int row = wm * 32 + 8 * fa + (lane >> 2), col = wn * 32 + 8 * fb + 2 * (lane & 3) + t;
+          const int m = o0 + (X ? col : row);
+          const long long v = v0 + (X ? row : col);
+          if (m >= lim || v >= vn) continue;
+          const long long q = (par ? ne : 0) + m;
+          if (X)
+            out[v * n + q] = acc[fa][fb][t];
+          else
+            out[q * I + v] = acc[fa][fb][t];
+        }
   }
 }
 
@@ -146,12 +299,17 @@ __device__ inline double ipow(double x, long long e) {
   return r;
 }
 
+// What bounds it: the FP64 powers at large sizes, the final sum at small ones.
+// 256 x 128 x 128 37 us (76 with 64-bit element indices, 160 shuffles a warp
+// and a last block that read the partials one point at a time), 77^3 14 us (42).
+//
 // Parseval sums f(d_t) = sum_m g_m^(2 d_t) rh_m^2 at the sweep counts
 // d_t = d0 + t*step (doubling == 0) or d_t = d0 * 2^t (doubling == 1), for
 // t < count.  Modes with g^2 <= g2_skip add nothing (the caller bounds what
 // they could add far below the stop test's resolution).  Per-block partials
 // in a fixed order; the last block to finish sums them (in block order) into
 // out[t] and re-arms the counter.
+template <class T>
 __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* __restrict__ Rh, int nx, int ny,
                                                                   int nz, const double* __restrict__ omx,
                                                                   const double* __restrict__ omy,
@@ -162,9 +320,10 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
   double acc[kSpecPoints];
 #pragma unroll
   for (int t = 0; t < kSpecPoints; ++t) acc[t] = 0.0;
-  const long long n = (long long)nx * ny * nz;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    const int mx = int(q % nx), my = int((q / nx) % ny), mz = int(q / ((long long)nx * ny));
+  const T n = T(nx) * T(ny) * T(nz);
+  for (T q = T(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += T(gridDim.x) * blockDim.x) {
+    int mx, my, mz;
+    split3(q, nx, ny, mx, my, mz);
     const double g = 1.0 - (omx[mx] + omy[my] + omz[mz]);
     const double g2 = g * g;
     if (g2 <= g2_skip) continue;
@@ -198,12 +357,17 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
   __shared__ double sh[kSpecThreads / 32][kSpecPoints];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // transposed butterfly: 31 exchanges leave point `lane` of the warp in
+  // acc[0], where 32 separate trees would take 160
 #pragma unroll
-  for (int t = 0; t < kSpecPoints; ++t) {
-    double v = acc[t];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[wid][t] = v;
-  }
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int t = 0; t < o; ++t) {
+      const bool up = lane & o;
+      const double give = up ? acc[t] : acc[t + o];
+      acc[t] = (up ? acc[t + o] : acc[t]) + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  sh[wid][lane] = acc[0];
   __syncthreads();
   if (threadIdx.x < kSpecPoints) {
     double s = 0.0;
@@ -216,12 +380,17 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // the last block: out[t] = sum_b partial[b][t], warp w taking points w, w + 8, ...
-  for (int t = wid; t < kSpecPoints; t += kSpecThreads / 32) {
-    double s = 0.0;
-    for (int b2 = lane; b2 < (int)gridDim.x; b2 += 32) s += __ldcg(partial + (long long)b2 * kSpecPoints + t);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[t] = s;
+  // the last block: out[t] = sum_b partial[b][t], warp w taking blocks w, w +
+  // 8, ... (a row of 32 points per load) and the warps' sums added in order
+  double s = 0.0;
+#pragma unroll 8
+  for (int b2 = wid; b2 < (int)gridDim.x; b2 += kSpecThreads / 32) s += __ldcg(partial + (long long)b2 * kSpecPoints + lane);
+  sh[wid][lane] = s;
+  __syncthreads();
+  if (threadIdx.x < kSpecPoints) {
+    double v = 0.0;
+    for (int w2 = 0; w2 < kSpecThreads / 32; ++w2) v += sh[w2][threadIdx.x];
+    out[threadIdx.x] = v;
   }
   if (threadIdx.x == 0) *counter = 0u;
 }
@@ -229,16 +398,21 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
 // rh -> -af (1 - g^d)/(1 - g) rh in place.  For g > 0 the factor is
 // -expm1(d log1p(-omg))/omg (no cancellation near g = 1); a mode with
 // omg == 0 (every axis periodic, the constant mode) takes d.
+template <class T>
 __global__ void spec_scale_kernel(double* __restrict__ Rh, int nx, int ny, int nz, const double* __restrict__ omx,
                                   const double* __restrict__ omy, const double* __restrict__ omz, long long d,
                                   double af) {
-  const long long n = (long long)nx * ny * nz;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-    const int mx = int(q % nx), my = int((q / nx) % ny), mz = int(q / ((long long)nx * ny));
+  const T n = T(nx) * T(ny) * T(nz);
+  for (T q = T(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += T(gridDim.x) * blockDim.x) {
+    int mx, my, mz;
+    split3(q, nx, ny, mx, my, mz);
     const double omg = omx[mx] + omy[my] + omz[mz];
+    // |g|^d <= exp(-d (1 - |g|)): below exp(-40) < 2^-57 it is nothing beside 1
     double f;
     if (omg == 0.0) {
       f = (double)d;
+    } else if ((double)d * fmin(omg, 2.0 - omg) > 40.0) {
+      f = 1.0 / omg;
     } else if (omg < 1.0) {
       f = -expm1((double)d * log1p(-omg)) / omg;
     } else {
@@ -249,193 +423,93 @@ __global__ void spec_scale_kernel(double* __restrict__ Rh, int nx, int ny, int n
   }
 }
 
-// U(interior) += D (compact).
-__global__ void spec_apply_kernel(KParams P, const double* __restrict__ D, double* __restrict__ U) {
-  const long long n = (long long)P.nx * P.ny * P.nz;
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-    const int i = int(t % P.nx) + 1;
-    const int j = int((t / P.nx) % P.ny) + 1;
-    const int k = int(t / ((long long)P.nx * P.ny)) + 1;
-    U[node_index(P, i, j, k)] += D[t];
-  }
-}
-
-// In-place fold along one axis of an (O, n, I) array (element (o, i, t) at
-// (o n + i) I + t): for i < n/2, x[i] <- x[i] + x[n-1-i] and x[n-1-i] <-
-// x[i] - x[n-1-i] (the middle of an odd n unchanged); unfold is the same
-// butterfly after the inverse products (E + O, E - O).
-__global__ void spec_fold_kernel(double* __restrict__ x, long long O, int n, long long I) {
-  const int h = n / 2;
-  const long long pairs = O * h * I;
-  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < pairs;
-       q += (long long)gridDim.x * blockDim.x) {
-    const long long t = q % I;
-    const long long r = q / I;
-    const int i = int(r % h);
-    const long long o = r / h;
-    double* row = x + o * n * I + t;
-    const double a = row[(long long)i * I], b = row[(long long)(n - 1 - i) * I];
-    row[(long long)i * I] = a + b;
-    row[(long long)(n - 1 - i) * I] = a - b;
-  }
-}
-
 int stream_blocks(long long n) {
   long long b = (n + kSpecThreads - 1) / kSpecThreads;
   return int(std::max<long long>(1, std::min<long long>(b, 148LL * 8)));
 }
 
-// One axis basis: Q (n x n, row = mode), its transpose, and a_d (2 - sigma)
-// per mode.
-void axis_basis(int n, bool periodic, double a, std::vector<double>& Q, std::vector<double>& QT,
-                std::vector<double>& om);
-
-// The sine basis folded by its symmetry Q[m][n-1-i] = (-1)^m Q[m][i]: with
-// hs = ceil(n/2), h = floor(n/2), the even modes 2k come from the folded sums
-// x[i] + x[n-1-i] (i < h) and the middle x[h] through Qe (hs x hs), the odd
-// modes 2k+1 from the differences x[i] - x[n-1-i], held at position n-1-i,
-// through QoR[k][j] = Q[2k+1][h-1-j] (h x h).  Modes are kept in the order
-// [even | odd]; om follows that order.
-void folded_basis(int n, double a, std::vector<double>& Qe, std::vector<double>& QeT, std::vector<double>& QoR,
-                  std::vector<double>& QoRT, std::vector<double>& om) {
-  std::vector<double> Q, QT, om0;
-  axis_basis(n, false, a, Q, QT, om0);
-  const int h = n / 2, hs = n - h;
-  Qe.assign((size_t)hs * hs, 0.0);
-  QeT.assign((size_t)hs * hs, 0.0);
-  QoR.assign((size_t)std::max(h, 1) * std::max(h, 1), 0.0);
-  QoRT.assign(QoR.size(), 0.0);
-  om.assign(n, 0.0);
-  for (int k = 0; k < hs; ++k) {
-    for (int i = 0; i < hs; ++i) {
-      Qe[(size_t)k * hs + i] = Q[(size_t)(2 * k) * n + i];
-      QeT[(size_t)i * hs + k] = Q[(size_t)(2 * k) * n + i];
-    }
-    om[k] = om0[2 * k];
-  }
-  for (int k = 0; k < h; ++k) {
-    for (int j = 0; j < h; ++j) {
-      QoR[(size_t)k * h + j] = Q[(size_t)(2 * k + 1) * n + (h - 1 - j)];
-      QoRT[(size_t)j * h + k] = QoR[(size_t)k * h + j];
-    }
-    om[hs + k] = om0[2 * k + 1];
-  }
-}
-
-void axis_basis(int n, bool periodic, double a, std::vector<double>& Q, std::vector<double>& QT,
-                std::vector<double>& om) {
+// The basis of one axis, folded (spec_axis_kernel): Pe[m][i] (ne x ne, the
+// even functions on i < ne) and Po[m][i - s] (no x no, the odd ones on s <= i <
+// no + s), and om, a_d (2 - sigma) per mode, in the order [even | odd].
+//   open (s = 0): sqrt(2/(n+1)) sin(pi (f+1)(i+1)/(n+1)), even for even f;
+//   periodic (s = 1): 1/sqrt(n), sqrt(2/n) cos(2 pi f i/n) and, n even,
+//   (-1)^i/sqrt(n) even; sqrt(2/n) sin(2 pi f i/n) odd.
+void folded_basis(int n, bool periodic, double a, AxisBasis& A, std::vector<double>& Pe, std::vector<double>& Po,
+                  std::vector<double>& om) {
   const double pi = 3.14159265358979323846264338327950288;
-  Q.assign((size_t)n * n, 0.0);
-  QT.assign((size_t)n * n, 0.0);
+  A.s = periodic ? 1 : 0;
+  A.ne = periodic ? n / 2 + 1 : n - n / 2;
+  A.no = n - A.ne;
+  const int ne = A.ne, no = A.no;
+  Pe.assign((size_t)ne * ne, 0.0);
+  Po.assign((size_t)std::max(no, 1) * std::max(no, 1), 0.0);
   om.assign(n, 0.0);
   if (!periodic) {
-    const double s = std::sqrt(2.0 / (n + 1));
+    const double scale = std::sqrt(2.0 / (n + 1));
     const long long per = 2LL * (n + 1);
-    for (int m = 0; m < n; ++m) {
-      for (int i = 0; i < n; ++i) {
-        const long long p = ((long long)(m + 1) * (i + 1)) % per;  // sin(pi p/(n+1)) has period 2(n+1)
-        Q[(size_t)m * n + i] = s * std::sin(pi * (double)p / (double)(n + 1));
+    for (int f = 0; f < n; ++f) {
+      const int m = f / 2, cnt = f % 2 ? no : ne;
+      for (int i = 0; i < cnt; ++i) {
+        const long long p = ((long long)(f + 1) * (i + 1)) % per;  // sin(pi p/(n+1)) has period 2(n+1)
+        (f % 2 ? Po[(size_t)m * no + i] : Pe[(size_t)m * ne + i]) = scale * std::sin(pi * (double)p / (double)(n + 1));
       }
-      const double h = std::sin(pi * (m + 1) / (2.0 * (n + 1)));
-      om[m] = a * 4.0 * h * h;  // a (2 - 2 cos(theta)) = 4 a sin^2(theta/2)
+      const double h = std::sin(pi * (f + 1) / (2.0 * (n + 1)));
+      om[f % 2 ? ne + m : m] = a * 4.0 * h * h;  // a (2 - 2 cos(theta)) = 4 a sin^2(theta/2)
     }
-  } else {
-    int row = 0;
-    auto put = [&](int f, int kind) {  // kind 0: constant, 1: cos, 2: sin, 3: alternating
-      for (int i = 0; i < n; ++i) {
-        double v;
-        const long long p = ((long long)f * i) % n;
-        if (kind == 0) v = 1.0 / std::sqrt((double)n);
-        else if (kind == 3) v = (i % 2 ? -1.0 : 1.0) / std::sqrt((double)n);
-        else if (kind == 1) v = std::sqrt(2.0 / n) * std::cos(2.0 * pi * (double)p / n);
-        else v = std::sqrt(2.0 / n) * std::sin(2.0 * pi * (double)p / n);
-        Q[(size_t)row * n + i] = v;
-      }
-      const double h = std::sin(pi * f / (double)n);
-      om[row] = a * 4.0 * h * h;
-      ++row;
-    };
-    put(0, 0);
-    for (int f = 1; 2 * f < n; ++f) {
-      put(f, 1);
-      put(f, 2);
-    }
-    if (n % 2 == 0 && n >= 2) put(n / 2, 3);
+    return;
   }
-  for (int m = 0; m < n; ++m)
-    for (int i = 0; i < n; ++i) QT[(size_t)i * n + m] = Q[(size_t)m * n + i];
+  for (int f = 0; f < ne; ++f) {
+    const bool alone = f == 0 || 2 * f == n;
+    for (int i = 0; i < ne; ++i) {
+      const long long p = ((long long)f * i) % n;
+      Pe[(size_t)f * ne + i] = f == 0       ? 1.0 / std::sqrt((double)n)
+                               : 2 * f == n ? (i % 2 ? -1.0 : 1.0) / std::sqrt((double)n)
+                                            : std::sqrt(2.0 / n) * std::cos(2.0 * pi * (double)p / n);
+      if (!alone && i >= 1 && i <= no)
+        Po[(size_t)(f - 1) * no + (i - 1)] = std::sqrt(2.0 / n) * std::sin(2.0 * pi * (double)p / n);
+    }
+    const double h = std::sin(pi * f / (double)n);
+    om[f] = a * 4.0 * h * h;
+    if (!alone) om[ne + f - 1] = om[f];
+  }
 }
 
-template <bool KB>
-cudaError_t gemm(const double* A, int lda, long long sa, const double* B, int ldb, long long sb, double* C, int ldc,
-                 long long sc, int M, int N, int K, int batch, cudaStream_t st) {
-  dim3 grid((N + kGemmBN - 1) / kGemmBN, (M + kGemmBM - 1) / kGemmBM, batch);
-  note_launch();
-  spec_gemm_kernel<KB><<<grid, 256, 0, st>>>(A, lda, sa, B, ldb, sb, C, ldc, sc, M, N, K);
-  return cudaGetLastError();
+void transpose(int n, const std::vector<double>& M, std::vector<double>& T) {
+  T.assign(M.size(), 0.0);
+  for (int r = 0; r < n; ++r)
+    for (int c = 0; c < n; ++c) T[(size_t)c * n + r] = M[(size_t)r * n + c];
 }
 
-cudaError_t fold(picard_ctx* c, double* x, long long O, int n, long long I) {
-  if (n < 2) return cudaSuccess;
-  note_launch();
-  spec_fold_kernel<<<stream_blocks(O * (n / 2) * I), kSpecThreads, 0, c->st>>>(x, O, n, I);
-  return cudaGetLastError();
-}
-
-// One axis pass from `in` to `out`.  Axis d of length n has outer extent O
-// and inner extent I (x: O = ny nz, I = 1; y: O = nz, I = nx; z: O = 1, I =
-// nx ny).  Dense axes (periodic): out = Q in (forward) or Q^T in (inverse)
-// along the axis.  Folded axes (open): forward folds `in` in place and applies
-// Qe and QoR to its two halves; inverse applies Qe^T and QoR^T to the two
-// halves of `in` and unfolds `out` in place.
-cudaError_t axis_pass(picard_ctx* c, int d, bool forward, double* in, double* out) {
-  SpectralPlan& S = c->spec;
+// One axis pass from `in` to `out` (out null: x, inverse, added to U's
+// interior).  Axis d has outer extent O and inner extent I: x rows (I = 1), y
+// O = nz slabs of nx columns, z one slab of nx ny columns.
+cudaError_t axis_pass(picard_ctx* c, int d, bool forward, const double* in, double* out) {
+  const SpectralPlan& S = c->spec;
+  const AxisBasis& A = S.ax[d];
   const int nx = c->K.nx, ny = c->K.ny, nz = c->K.nz;
   const int n = d == 0 ? nx : d == 1 ? ny : nz;
-  const long long O = d == 0 ? (long long)ny * nz : d == 1 ? nz : 1;
   const long long I = d == 0 ? 1 : d == 1 ? nx : (long long)nx * ny;
-  const long long plane = (long long)nx * ny;
-  cudaError_t e;
-  if (!S.folded[d]) {
-    if (d == 0) {
-      // x: out[r][m] = sum_i in[r][i] Q[m][i] (B K-contiguous), or sum_m in[r][m] Q[m][i]
-      return forward ? gemm<true>(in, nx, 0, S.Q[0], nx, 0, out, nx, 0, ny * nz, nx, nx, 1, c->st)
-                     : gemm<false>(in, nx, 0, S.Q[0], nx, 0, out, nx, 0, ny * nz, nx, nx, 1, c->st);
-    }
-    const double* M = forward ? S.Q[d] : S.QT[d];
-    if (d == 1) return gemm<false>(M, ny, 0, in, nx, plane, out, nx, plane, ny, nx, ny, nz, c->st);
-    return gemm<false>(M, nz, 0, in, (int)plane, 0, out, (int)plane, 0, nz, (int)plane, nz, 1, c->st);
-  }
-  const int h = n / 2, hs = n - h;
-  if (forward && (e = fold(c, in, O, n, I))) return e;
-  const double* Me = forward ? S.Qe[d] : S.QeT[d];
-  const double* Mo = forward ? S.QoR[d] : S.QoRT[d];
-  if (d == 0) {
-    if (forward) {
-      if ((e = gemm<true>(in, nx, 0, Me, hs, 0, out, nx, 0, ny * nz, hs, hs, 1, c->st))) return e;
-      if (h > 0 && (e = gemm<true>(in + hs, nx, 0, Mo, h, 0, out + hs, nx, 0, ny * nz, h, h, 1, c->st))) return e;
-    } else {
-      if ((e = gemm<false>(in, nx, 0, S.Qe[0], hs, 0, out, nx, 0, ny * nz, hs, hs, 1, c->st))) return e;
-      if (h > 0 && (e = gemm<false>(in + hs, nx, 0, S.QoR[0], h, 0, out + hs, nx, 0, ny * nz, h, h, 1, c->st)))
-        return e;
-    }
-  } else if (d == 1) {
-    if ((e = gemm<false>(Me, hs, 0, in, nx, plane, out, nx, plane, hs, nx, hs, nz, c->st))) return e;
-    if (h > 0 && (e = gemm<false>(Mo, h, 0, in + (long long)hs * nx, nx, plane, out + (long long)hs * nx, nx, plane, h,
-                                  nx, h, nz, c->st)))
-      return e;
-  } else {
-    if ((e = gemm<false>(Me, hs, 0, in, (int)plane, 0, out, (int)plane, 0, hs, (int)plane, hs, 1, c->st))) return e;
-    if (h > 0 && (e = gemm<false>(Mo, h, 0, in + (long long)hs * plane, (int)plane, 0, out + (long long)hs * plane,
-                                  (int)plane, 0, h, (int)plane, h, 1, c->st)))
-      return e;
-  }
-  if (!forward) return fold(c, out, O, n, I);
-  return cudaSuccess;
+  const int rows = d == 0 ? ny * nz : 0;
+  auto tiles = [](long long v) { return (unsigned)((v + kAxTile - 1) / kAxTile); };
+  const dim3 grid = d == 0 ? dim3(tiles(A.ne), tiles(rows)) : dim3(tiles(I), tiles(A.ne), d == 1 ? nz : 1);
+  note_launch();
+  if (d == 0 && forward)
+    spec_axis_kernel<false, true, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
+                                                                  c->K, nullptr);
+  else if (d == 0)
+    spec_axis_kernel<true, true, true><<<grid, 256, 0, c->st>>>(in, nullptr, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
+                                                                c->K, c->U);
+  else if (forward)
+    spec_axis_kernel<false, false, false><<<grid, 256, 0, c->st>>>(in, out, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
+                                                                   c->K, nullptr);
+  else
+    spec_axis_kernel<true, false, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
+                                                                  c->K, nullptr);
+  return cudaGetLastError();
 }
 
 // Forward: Qz Qy Qx of T[0] into T[1] (x, y, z passes ping-ponging T[0] and
-// T[1]); inverse: Qx^T Qy^T Qz^T of T[1] into T[0].
+// T[1]); inverse: Qx^T Qy^T Qz^T of T[1], added to U's interior.
 cudaError_t transform(picard_ctx* c, bool forward) {
   SpectralPlan& S = c->spec;
   cudaError_t e;
@@ -446,15 +520,21 @@ cudaError_t transform(picard_ctx* c, bool forward) {
   }
   if ((e = axis_pass(c, 2, false, S.T[1], S.T[0]))) return e;
   if ((e = axis_pass(c, 1, false, S.T[0], S.T[1]))) return e;
-  return axis_pass(c, 0, false, S.T[1], S.T[0]);
+  return axis_pass(c, 0, false, S.T[1], nullptr);
 }
 
 // Queues the evaluation of f at count (<= kSpecPoints) sweep counts and the
 // copy of the sums to c->h_pinned[0..count); the caller waits on the stream.
 int issue_norms(picard_ctx* c, long long d0, long long step, int count, bool doubling, double g2_skip) {
   SpectralPlan& S = c->spec;
+  const long long n = (long long)c->K.nx * c->K.ny * c->K.nz;
   note_launch();
-  spec_norms_kernel<<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], c->K.nx, c->K.ny, c->K.nz, S.om[0], S.om[1],
+  if (fits32(n))
+    spec_norms_kernel<unsigned><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], c->K.nx, c->K.ny, c->K.nz, S.om[0], S.om[1],
+                                                                S.om[2], d0, step, count, doubling ? 1 : 0, g2_skip,
+                                                                S.partial, S.counter, S.sums);
+  else
+    spec_norms_kernel<long long><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], c->K.nx, c->K.ny, c->K.nz, S.om[0], S.om[1],
                                                                 S.om[2], d0, step, count, doubling ? 1 : 0, g2_skip,
                                                                 S.partial, S.counter, S.sums);
   PICARD_CUDA(cudaGetLastError());
@@ -475,45 +555,30 @@ int spectral_alloc(picard_ctx* c) {
   const int len[3] = {K.nx, K.ny, K.nz};
   const bool per[3] = {!K.xflow, !K.yflow, !K.zflow};
   for (int d = 0; d < 3; ++d) {
-    void* p = nullptr;
-    if (!per[d]) {
-      std::vector<double> Qe, QeT, QoR, QoRT, om;
-      folded_basis(len[d], a[d], Qe, QeT, QoR, QoRT, om);
-      double** dst[5] = {&S.Qe[d], &S.QeT[d], &S.QoR[d], &S.QoRT[d], &S.om[d]};
-      const std::vector<double>* srcv[5] = {&Qe, &QeT, &QoR, &QoRT, &om};
-      for (int t = 0; t < 5; ++t) {
-        PICARD_TRY(dev_alloc(c, &p, sizeof(double) * srcv[t]->size()));
-        *dst[t] = static_cast<double*>(p);
-        // no wait: an asynchronous copy from pageable memory returns once the
-        // host data is staged, so the vectors may go out of scope
-        PICARD_CUDA(cudaMemcpyAsync(*dst[t], srcv[t]->data(), sizeof(double) * srcv[t]->size(),
-                                    cudaMemcpyHostToDevice, c->st));
-        c->stats.h2d_bytes += (int64_t)(sizeof(double) * srcv[t]->size());
-      }
-      S.folded[d] = 1;
-      continue;
+    AxisBasis& A = S.ax[d];
+    std::vector<double> Pe, Po, PeT, PoT, om;
+    folded_basis(len[d], per[d], a[d], A, Pe, Po, om);
+    transpose(A.ne, Pe, PeT);
+    transpose(A.no, Po, PoT);
+    double** dst[5] = {&A.Pe, &A.PeT, &A.Po, &A.PoT, &S.om[d]};
+    const std::vector<double>* srcv[5] = {&Pe, &PeT, &Po, &PoT, &om};
+    for (int t = 0; t < 5; ++t) {
+      void* p = nullptr;
+      PICARD_TRY(dev_alloc(c, &p, sizeof(double) * srcv[t]->size()));
+      *dst[t] = static_cast<double*>(p);
+      // no wait: an asynchronous copy from pageable memory returns once the
+      // host data is staged, so the vectors may go out of scope
+      PICARD_CUDA(cudaMemcpyAsync(*dst[t], srcv[t]->data(), sizeof(double) * srcv[t]->size(), cudaMemcpyHostToDevice,
+                                  c->st));
+      c->stats.h2d_bytes += (int64_t)(sizeof(double) * srcv[t]->size());
     }
-    std::vector<double> Q, QT, om;
-    axis_basis(len[d], per[d], a[d], Q, QT, om);
-    PICARD_TRY(dev_alloc(c, &p, sizeof(double) * Q.size()));
-    S.Q[d] = static_cast<double*>(p);
-    PICARD_TRY(dev_alloc(c, &p, sizeof(double) * QT.size()));
-    S.QT[d] = static_cast<double*>(p);
-    PICARD_TRY(dev_alloc(c, &p, sizeof(double) * om.size()));
-    S.om[d] = static_cast<double*>(p);
-    PICARD_CUDA(cudaMemcpyAsync(S.Q[d], Q.data(), sizeof(double) * Q.size(), cudaMemcpyHostToDevice, c->st));
-    PICARD_CUDA(cudaMemcpyAsync(S.QT[d], QT.data(), sizeof(double) * QT.size(), cudaMemcpyHostToDevice, c->st));
-    PICARD_CUDA(cudaMemcpyAsync(S.om[d], om.data(), sizeof(double) * om.size(), cudaMemcpyHostToDevice, c->st));
-    // no wait: an asynchronous copy from pageable memory returns once the host
-    // data is staged, so the vectors may go out of scope
-    c->stats.h2d_bytes += (int64_t)sizeof(double) * (Q.size() + QT.size() + om.size());
   }
   void* p = nullptr;
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * n));
   S.T[0] = static_cast<double*>(p);
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * n));
   S.T[1] = static_cast<double*>(p);
-  S.norm_blocks = stream_blocks(n);
+  S.norm_blocks = std::min(stream_blocks(n), 148 * 4);
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * (size_t)S.norm_blocks * kSpecPoints));
   S.partial = static_cast<double*>(p);
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * kSpecPoints));
@@ -561,7 +626,11 @@ int spec_begin(SpecSolve& Q, picard_ctx* c, double tol, long long smax, int maxi
   Q.hi = Q.dmax + 1;
   PICARD_CUDA(cudaEventRecord(c->ev[0], c->st));
   note_launch();
-  spec_r0_kernel<<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, 1.0 / J.dx2, 1.0 / J.dy2, 1.0 / J.dz2, c->U, c->b,
+  if (fits32(n))
+    spec_r0_kernel<unsigned><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, 1.0 / J.dx2, 1.0 / J.dy2, 1.0 / J.dz2, c->U, c->b,
+                                                                S.T[0]);
+  else
+    spec_r0_kernel<long long><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, 1.0 / J.dx2, 1.0 / J.dy2, 1.0 / J.dz2, c->U, c->b,
                                                                 S.T[0]);
   PICARD_CUDA(cudaGetLastError());
   PICARD_CUDA(transform(c, true));
@@ -642,13 +711,14 @@ int spec_apply_issue(SpecSolve& Q) {
   const JacobiCoef J = jacobi_coef(K);
   PICARD_CUDA(cudaEventRecord(c->ev[2], c->st));
   note_launch();
-  spec_scale_kernel<<<stream_blocks(n), kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
+  if (fits32(n))
+    spec_scale_kernel<unsigned><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
+                                                                   S.om[2], Q.d, J.af);
+  else
+    spec_scale_kernel<long long><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
                                                                    S.om[2], Q.d, J.af);
   PICARD_CUDA(cudaGetLastError());
   PICARD_CUDA(transform(c, false));
-  note_launch();
-  spec_apply_kernel<<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, S.T[0], c->U);
-  PICARD_CUDA(cudaGetLastError());
   PICARD_CUDA(cudaEventRecord(c->ev[3], c->st));
   Q.done = true;
   return PICARD_OK;
