@@ -541,8 +541,7 @@ struct RunSolve {
   picard_ctx* c = nullptr;
   EpotSetup e;
   F32Solve S;
-  SpecSolve Q;           // SOLVER_SPECTRAL: the closed-form solve
-  bool spectral = false;
+  bool spectral = false; // SOLVER_SPECTRAL: queued whole, collected with the next count
   bool batched = false;  // the batched loop drives this run's solve
   bool active = false;   // in the set of runs that sweep together
   bool w32 = false;      // 32-wide tiles (tile32.cuh) instead of 64-wide x pairs
@@ -742,7 +741,7 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
   // PICARD_BATCH_LOG=1: host time per phase (waits for the device included)
   const char* logv = std::getenv("PICARD_BATCH_LOG");
   const bool log = logv && *logv && *logv != '0';
-  double ph[6] = {0, 0, 0, 0, 0, 0};
+  double ph[3] = {0, 0, 0};
   long long rounds = 0, launches = 0, ticks = 0;
   g_batch_ctas = 0;
   auto now = []() { return std::chrono::steady_clock::now(); };
@@ -752,10 +751,34 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
     ph[k] += std::chrono::duration<double, std::milli>(t - tick).count();
     tick = t;
   };
+  // CalcEfield + BCfields, AdvanceVelocity (CELL32, when another step follows:
+  // fused with that step's AdvancePosition, as the single-run loop)
+  auto push = [&](int r, int32_t step) -> int {
+    picard_ctx* c = ctxs[r];
+    PICARD_TRY(picard_gpu_calc_efield(c));
+    if (step < nsteps && c->layout == PICARD_LAYOUT_CELL32)
+      PICARD_CUDA(launch_push_advance_c32(c->K, c->c32, c->num_local, c->E32, c->prm.dt, c->st));
+    else
+      PICARD_TRY(picard_gpu_advance_velocity(c, c->prm.dt));
+    c->stats.steps += 1;
+    c->stats.particle_steps += c->num_local;
+    return PICARD_OK;
+  };
+  // the closed-form solve of a run's previous step, once its stream has been waited for
+  auto settle = [&](int r) -> int {
+    long long sw = 0;
+    const int q = spec_collect(ctxs[r], &sw);
+    if (sweeps_total) sweeps_total[r] += sw;
+    if (q == PICARD_ERR_NOT_CONVERGED) nc = true;
+    else if (q != PICARD_OK) return q;
+    return PICARD_OK;
+  };
+  for (int r = 0; r < n; ++r) ctxs[r]->spec.pending = false;
   auto body = [&]() -> int {
     for (int32_t step = 1; step <= nsteps; ++step) {
       tick = now();
-      // ---- AdvancePosition, ParticlesProduce (device count) for every run
+      // ---- AdvancePosition, ParticlesProduce (device count), BCoutflow +
+      // ParticlesTransfer (in place), BCinflow (fused), ParticlesGridify
       PICARD_TRY(pool.run(n, [&](int r) -> int {
         picard_ctx* c = ctxs[r];
         const KParams& K = c->K;
@@ -763,57 +786,52 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
         // CELL32 runs after their first step: the previous step's push advanced them
         if (step == 1 || c->layout != PICARD_LAYOUT_CELL32) PICARD_TRY(picard_gpu_advance_position(c, c->prm.dt));
         const int32_t it = it0[r] + step;
-        PICARD_CUDA(launch_produce_count(K, it, c->cell_counts, c->st));
-        PICARD_CUDA(launch_scan_int(c->cell_counts, c->cell_offsets, cells, c->cell_offsets + cells,
-                                    c->cell_offsets + cells + 2, c->st));
-        if (c->layout == PICARD_LAYOUT_F64)
-          PICARD_CUDA(launch_produce_emit_f64(K, it, c->cell_offsets, c->f64, c->d_count,
-                                              c->capacity, c->d_err, c->st));
-        else
-          PICARD_CUDA(launch_produce_emit_c32(K, it, c->cell_offsets, c->c32, c->d_count,
-                                              c->capacity, c->d_err, c->st));
-        PICARD_TRY(count_issue(c));
-        return count_collect(c);
-      }));
-      lap(0);
-      // ---- BCoutflow + ParticlesTransfer (in place), BCinflow (fused)
-      PICARD_TRY(pool.run(n, [&](int r) -> int {
-        picard_ctx* c = ctxs[r];
-        const int32_t it = it0[r] + step;
+        if (has_neutral_source(K)) {
+          PICARD_CUDA(launch_produce_count(K, it, c->cell_counts, c->st));
+          PICARD_CUDA(launch_scan_int(c->cell_counts, c->cell_offsets, cells, c->cell_offsets + cells,
+                                      c->cell_offsets + cells + 2, c->st));
+          if (c->layout == PICARD_LAYOUT_F64)
+            PICARD_CUDA(launch_produce_emit_f64(K, it, c->cell_offsets, c->f64, c->d_count,
+                                                c->capacity, c->d_err, c->st));
+          else
+            PICARD_CUDA(launch_produce_emit_c32(K, it, c->cell_offsets, c->c32, c->d_count,
+                                                c->capacity, c->d_err, c->st));
+          PICARD_TRY(count_issue(c));
+          PICARD_TRY(count_collect(c));
+        }
         PICARD_CUDA(launch_outflow(c, 1));
         PICARD_CUDA(launch_inflow_fused(c, it));
         PICARD_TRY(count_issue(c));
-        return count_collect(c);
+        PICARD_TRY(count_collect(c));
+        PICARD_TRY(settle(r));
+        return picard_gpu_particles_gridify(c);
       }));
-      lap(1);
-      // ---- ParticlesGridify, BCpotentials (FFT runs: one launch per stage
-      // for all of them), b and ||b||
-      PICARD_TRY(pool.run(n, [&](int r) -> int { return picard_gpu_particles_gridify(ctxs[r]); }));
+      lap(0);
+      // ---- BCpotentials (FFT runs: one launch per stage for all of them)
       PICARD_TRY(bc_potentials_batch(ctxs, n, bst, rev.data(), bev));
-      PICARD_TRY(pool.run(n, [&](int r) -> int {
-        PICARD_TRY(epot_rhs_issue(ctxs[r]));
-        PICARD_CUDA(cudaStreamSynchronize(ctxs[r]->st));
-        return PICARD_OK;
-      }));
-      lap(2);
-      // ---- CalcEpotential: closed-form solves and solves of their own
-      // issued per run in parallel; FP32 runs in lockstep ticks below
+      lap(1);
+      // ---- CalcEpotential: closed-form solves queued whole, with the rest of
+      // the step behind them; solves of their own issued per run in parallel;
+      // FP32 runs in lockstep ticks below
       PICARD_TRY(pool.run(n, [&](int r) -> int {
         picard_ctx* c = ctxs[r];
         RunSolve& rs = solves[r];
         rs = RunSolve();
         rs.c = c;
-        rs.e = epot_setup(c, c->prm.maxerr, c->prm.maxit);
-        rs.done = rs.e.trivial;
         rs.sweeps = 0;
         rs.converged = true;
-        if (rs.done) return PICARD_OK;
+        rs.done = true;
         if (c->solver == PICARD_SOLVER_SPECTRAL) {
-          // closed form: queued now, its Parseval evaluations collected for
-          // every such run together below
           rs.spectral = true;
-          PICARD_TRY(spec_begin(rs.Q, c, rs.e.tol, rs.e.smax, rs.e.maxit));
-        } else if (c->solver == PICARD_SOLVER_F32_REFINE && c->G.tma && c->G.zc <= 8) {
+          PICARD_TRY(spec_issue(c, c->prm.maxerr, c->prm.maxit));
+          return push(r, step);
+        }
+        PICARD_TRY(epot_rhs_issue(c));
+        PICARD_CUDA(cudaStreamSynchronize(c->st));
+        rs.e = epot_setup(c, c->prm.maxerr, c->prm.maxit);
+        rs.done = rs.e.trivial;
+        if (rs.done) return PICARD_OK;
+        if (c->solver == PICARD_SOLVER_F32_REFINE && c->G.tma && c->G.zc <= 8) {
           rs.batched = true;
           // 32-wide tiles when 64-wide ones would leave a 32-column half empty
           rs.w32 = tile_w32 && ((c->K.nx + 31) / 32) % 2 == 1;
@@ -924,66 +942,34 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
           if (sweeping == 0) break;  // one at a time while blocking: replan at once
         }
       }
-      // closed-form solves: each worker takes its runs' Parseval evaluations
-      // in turn, one host round trip per evaluation for all of them
-      PICARD_TRY(pool.run(threads, [&](int w) -> int {
-        for (bool pending = true; pending;) {
-          pending = false;
-          for (int r = w; r < n; r += threads) {
-            RunSolve& rs = solves[r];
-            if (!rs.spectral || rs.done) continue;
-            PICARD_CUDA(cudaStreamSynchronize(ctxs[r]->st));
-            if (rs.Q.done) {
-              spec_account(rs.Q);
-              rs.done = true;
-              rs.sweeps = rs.Q.d;
-              rs.converged = rs.Q.converged;
-              continue;
-            }
-            PICARD_TRY(spec_collect(rs.Q));
-            pending = true;
-          }
-        }
-        return PICARD_OK;
-      }));
+      // ---- the other runs' wrap-up, CalcEfield + BCfields, AdvanceVelocity
       PICARD_TRY(pool.run(n, [&](int r) -> int {
         RunSolve& rs = solves[r];
-        if (!rs.batched && !rs.spectral && !rs.e.trivial) return PICARD_OK;  // solved on its own above
-        int32_t sw = 0;
-        int q = epot_finish(ctxs[r], rs.e, rs.sweeps, rs.converged, &sw);
-        if (q == PICARD_ERR_NOT_CONVERGED) nc = true;
-        else if (q != PICARD_OK) return q;
-        if (sweeps_total) sweeps_total[r] += sw;
-        return PICARD_OK;
+        if (rs.spectral) return PICARD_OK;  // queued above
+        if (rs.batched || rs.e.trivial) {   // else solved on its own above
+          int32_t sw = 0;
+          int q = epot_finish(ctxs[r], rs.e, rs.sweeps, rs.converged, &sw);
+          if (q == PICARD_ERR_NOT_CONVERGED) nc = true;
+          else if (q != PICARD_OK) return q;
+          if (sweeps_total) sweeps_total[r] += sw;
+        }
+        return push(r, step);
       }));
-      lap(3);
-      // ---- CalcEfield + BCfields, AdvanceVelocity (CELL32, when another step
-      // follows: fused with that step's AdvancePosition, as the single-run loop)
-      PICARD_TRY(pool.run(n, [&](int r) -> int {
-        picard_ctx* c = ctxs[r];
-        PICARD_TRY(picard_gpu_calc_efield(c));
-        if (step < nsteps && c->layout == PICARD_LAYOUT_CELL32)
-          PICARD_CUDA(launch_push_advance_c32(c->K, c->c32, c->num_local, c->E32, c->prm.dt, c->st));
-        else
-          PICARD_TRY(picard_gpu_advance_velocity(c, c->prm.dt));
-        c->stats.steps += 1;
-        c->stats.particle_steps += c->num_local;
-        return PICARD_OK;
-      }));
-      lap(4);
+      lap(2);
     }
     for (int r = 0; r < n; ++r) {
       PICARD_TRY(count_issue(ctxs[r]));  // a wait that gave up in the last step
       PICARD_TRY(count_collect(ctxs[r]));
+      PICARD_TRY(settle(r));
     }
     return PICARD_OK;
   };
   rc = body();
   if (log)
     std::fprintf(stderr,
-                 "picard batch %d runs: particles %.1f ms, compaction+inflow %.1f ms, deposit+bcpot+rhs %.1f ms, "
-                 "jacobi %.1f ms (%lld rounds, %lld ticks, %lld launches, %lld CTAs), push %.1f ms\n",
-                 n, ph[0], ph[1], ph[2], ph[3], rounds, ticks, launches, g_batch_ctas, ph[4]);
+                 "picard batch %d runs: particles+deposit %.1f ms, bcpot %.1f ms, solve+push %.1f ms "
+                 "(%lld rounds, %lld ticks, %lld launches, %lld CTAs)\n",
+                 n, ph[0], ph[1], ph[2], rounds, ticks, launches, g_batch_ctas);
   if (rc == PICARD_OK) rc = check_cuda(cudaStreamSynchronize(bst), "batch stream");
   cleanup();
   if (rc != PICARD_OK) return rc;

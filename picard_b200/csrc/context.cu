@@ -225,19 +225,17 @@ int sync_count(picard_ctx* c) {
   return PICARD_OK;
 }
 
+// The host's count to the device, in stream order (the value travels with the
+// launch: nothing to wait for).
+__global__ void set_count_kernel(int* count, int value) { *count = value; }
+
 int push_count(picard_ctx* c) {
-  c->h_pinned_i[1] = int(c->num_local);
-  PICARD_CUDA(cudaMemcpyAsync(c->d_count, c->h_pinned_i + 1, sizeof(int), cudaMemcpyHostToDevice, c->st));
-  PICARD_CUDA(cudaStreamSynchronize(c->st));
-  c->stats.h2d_bytes += sizeof(int);
-  return PICARD_OK;
+  note_launch();
+  set_count_kernel<<<1, 1, 0, c->st>>>(c->d_count, int(c->num_local));
+  return check_cuda(cudaGetLastError(), "set_count_kernel");
 }
 
-int check_dev_err(picard_ctx* c) {
-  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i + 2, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  PICARD_CUDA(cudaStreamSynchronize(c->st));
-  c->stats.d2h_bytes += sizeof(int);
-  int e = c->h_pinned_i[2];
+int report_dev_err(picard_ctx* c, int e) {
   if (e == kDevCapacity) {
     cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st);
     return fail(PICARD_ERR_CAPACITY, "particle capacity max_per_proc exceeded on the device");
@@ -251,6 +249,13 @@ int check_dev_err(picard_ctx* c) {
     return fail(PICARD_ERR_STATE, "a particle move left its range on the device and was skipped");
   }
   return PICARD_OK;
+}
+
+int check_dev_err(picard_ctx* c) {
+  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i + 2, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  PICARD_CUDA(cudaStreamSynchronize(c->st));
+  c->stats.d2h_bytes += sizeof(int);
+  return report_dev_err(c, c->h_pinned_i[2]);
 }
 
 int check_dev_err_timeout(picard_ctx* c) {
@@ -274,9 +279,12 @@ int ensure_capacity(picard_ctx* c, long long add) {
 }  // namespace
 
 namespace picard {
-int sync_count_public(picard_ctx* c) {
-  PICARD_TRY(check_dev_err(c));
-  return sync_count(c);
+bool has_neutral_source(const KParams& K) {
+  // ParticlesProduce.f90:62-73: the number of ions is int(rate + u), u < 1, and
+  // the rate is 0 without an outflow speed, a production or an ionisation rate
+  for (int s = 0; s < K.species; ++s)
+    if (K.n2p[s] > 0.0 && K.vn[s] > 0.0 && !(K.Qn[s] == 0.0) && !(K.nu_i[s] == 0.0)) return true;
+  return false;
 }
 
 int check_dev_err_public(picard_ctx* c) { return check_dev_err(c); }
@@ -333,28 +341,17 @@ cudaError_t launch_inflow_fused(picard_ctx* c, int iteration) {
                                  c->inflow_offsets, c->d_err, c->inflow_stage, c->st);
 }
 
+// The count and the error word lie side by side: one copy.
 int count_issue(picard_ctx* c) {
-  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i + 2, c->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i, c->d_count, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i + 8, c->d_count, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->st));
   c->stats.d2h_bytes += 2 * sizeof(int);
   return PICARD_OK;
 }
 
 int count_collect(picard_ctx* c) {
   PICARD_CUDA(cudaStreamSynchronize(c->st));
-  if (c->h_pinned_i[2] == kDevCapacity) {
-    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st);
-    return fail(PICARD_ERR_CAPACITY, "particle capacity max_per_proc exceeded on the device");
-  }
-  if (c->h_pinned_i[2] == kDevTimeout) {
-    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st);
-    return fail(PICARD_ERR_TIMEOUT, "a bounded device wait gave up");
-  }
-  if (c->h_pinned_i[2] == kDevRange) {
-    cudaMemsetAsync(c->d_err, 0, sizeof(int), c->st);
-    return fail(PICARD_ERR_STATE, "a particle move left its range on the device and was skipped");
-  }
-  c->num_local = c->h_pinned_i[0];
+  PICARD_TRY(report_dev_err(c, c->h_pinned_i[9]));
+  c->num_local = c->h_pinned_i[8];
   return PICARD_OK;
 }
 }  // namespace picard
@@ -448,11 +445,12 @@ int picard_gpu_create(const picard_params* p, int32_t layout, int32_t solver, pi
       return bail(rc);
   }
   const long long nn = s.nodes;
-  if ((rc = dalloc(c, c->d_count, 1)) || (rc = dalloc(c, c->d_err, 1)) || (rc = dalloc(c, c->d_info, 4)) ||
+  if ((rc = dalloc(c, c->d_count, 2)) || (rc = dalloc(c, c->d_info, 4)) ||
       (rc = dalloc(c, c->Nacc, nn * s.species)) || (rc = dalloc(c, c->N, nn * s.species)) ||
       (rc = dalloc(c, c->C, nn)) || (rc = dalloc(c, c->U, nn)) || (rc = dalloc(c, c->E, 3 * nn)) ||
       (rc = dalloc(c, c->D, s.dsize)) || (rc = dalloc(c, c->b, nn)) || (rc = dalloc(c, c->U1, nn)))
     return bail(rc);
+  c->d_err = c->d_count + 1;  // read together with the count
   if (layout == PICARD_LAYOUT_CELL32 && (rc = dalloc(c, c->E32, nn))) return bail(rc);
   if (solver == PICARD_SOLVER_F64) {
     if ((rc = dalloc(c, c->Usnap, nn))) return bail(rc);
@@ -498,12 +496,12 @@ int picard_gpu_create(const picard_params* p, int32_t layout, int32_t solver, pi
     return bail(rc);
   c->red_blocks = std::max<int>(148 * 16, rhs_blocks(c->K));
   if ((rc = dalloc(c, c->red_partial, c->red_blocks)) || (rc = dalloc(c, c->red_result, 8))) return bail(rc);
-  if ((rc = check_cuda(cudaMallocHost((void**)&c->h_pinned, sizeof(double) * (c->m_max + 16)), "cudaMallocHost")))
+  if ((rc = check_cuda(cudaMallocHost((void**)&c->h_pinned, sizeof(double) * (c->m_max + 64)), "cudaMallocHost")))
     return bail(rc);
   if ((rc = check_cuda(cudaMallocHost((void**)&c->h_pinned_i, sizeof(int) * 16), "cudaMallocHost"))) return bail(rc);
   for (int e = 0; e < 4; ++e)
     if ((rc = check_cuda(cudaEventCreate(&c->ev[e]), "cudaEventCreate"))) return bail(rc);
-  for (int e = 0; e < 6; ++e)
+  for (int e = 0; e < 12; ++e)
     if ((rc = check_cuda(cudaEventCreate(&c->pev[e]), "cudaEventCreate"))) return bail(rc);
   if ((rc = tune_sweep(c, false))) return bail(rc);
   if ((rc = check_cuda(cudaStreamSynchronize(c->st), "create"))) return bail(rc);
@@ -523,7 +521,7 @@ int picard_gpu_destroy(picard_ctx* c) {
   if (c->h_pinned_i) cudaFreeHost(c->h_pinned_i);
   for (int e = 0; e < 4; ++e)
     if (c->ev[e]) cudaEventDestroy(c->ev[e]);
-  for (int e = 0; e < 6; ++e)
+  for (int e = 0; e < 12; ++e)
     if (c->pev[e]) cudaEventDestroy(c->pev[e]);
   if (c->st) cudaStreamDestroy(c->st);
   delete c;
@@ -769,6 +767,7 @@ int picard_gpu_advance_position(picard_ctx* c, double dt) {
 // ParticlesProduce.f90:1-113
 int picard_gpu_particles_produce(picard_ctx* c, int32_t iteration) {
   if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
+  if (!has_neutral_source(c->K)) return PICARD_OK;
   const int cells = c->prm.nx * c->prm.ny * c->prm.nz;
   PICARD_CUDA(launch_produce_count(c->K, iteration, c->cell_counts, c->st));
   int* total = c->cell_offsets + cells;
@@ -785,8 +784,8 @@ int picard_gpu_particles_produce(picard_ctx* c, int32_t iteration) {
   else
     PICARD_CUDA(launch_produce_emit_c32(c->K, iteration, c->cell_offsets, c->c32, c->d_count,
                                         c->capacity, c->d_err, c->st));
-  PICARD_TRY(check_dev_err(c));
-  return sync_count(c);
+  PICARD_TRY(count_issue(c));
+  return count_collect(c);
 }
 
 // BCoutflow.f90:5-87, in place and in the reference's order (outflow.cuh)

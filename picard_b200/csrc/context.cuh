@@ -41,6 +41,19 @@ struct AxisBasis {
   double* PoT = nullptr;
 };
 
+// The stopping-sweep search of the closed-form solve, kept on the device
+// (spectral.cu spec_advance).
+struct SpecState {
+  double bnorm, tol2, f1, r2_hit;  // ||b||; (maxerr ||b||)^2; ||r_1||^2; ||r_d||^2 of the accepted iterate
+  double g2_skip;
+  long long smax, dmax, lo, hi;
+  long long d0, step;              // the next evaluation's sweep counts
+  long long d;                     // the accepted sweep count
+  int count, phase, done, converged;
+  int trivial;                     // ||b|| meets the test at the top of sweep 1: zero sweeps
+  int pad;
+};
+
 // Closed-form Jacobi solve (spectral.cu): the axis bases and the compact FP64
 // interior arrays the transforms use.  Modes of an axis in the order [even |
 // odd].
@@ -49,10 +62,10 @@ struct SpectralPlan {
   double* om[3] = {nullptr, nullptr, nullptr};  // a_d (2 - sigma_d) per mode
   double* T[2] = {nullptr, nullptr};            // nx*ny*nz each
   double* partial = nullptr;                    // [norm_blocks][32]
-  double* sums = nullptr;                       // [32]
-  unsigned int* counter = nullptr;              // blocks done in an evaluation (re-armed by the last)
+  SpecState* state = nullptr;
+  unsigned int* counter = nullptr;              // blocks done in a reduction (re-armed by the last)
   int norm_blocks = 0;
-  long long evals = 0;                          // Parseval evaluations (launch pairs)
+  bool pending = false;                         // a queued solve whose result has not been collected
 };
 }  // namespace picard
 
@@ -68,7 +81,7 @@ struct picard_ctx {
   picard::PartF64 f64 = {};  // the particles (one layout allocated)
   picard::PartC32 c32 = {};
   int* d_count = nullptr;    // live particle count
-  int* d_err = nullptr;
+  int* d_err = nullptr;      // error word, right after the count
   int* d_info = nullptr;     // small device results read with a count (BCoutflow window)
   long long num_local = 0;   // host mirror of *d_count
 
@@ -115,7 +128,7 @@ struct picard_ctx {
   double* red_partial = nullptr;
   double* red_result = nullptr;  // [8]
   int red_blocks = 0;
-  double* h_pinned = nullptr;    // [m_max + 16] host staging
+  double* h_pinned = nullptr;    // [m_max + 64] host staging
   int* h_pinned_i = nullptr;     // [16]
 
   // register-resident sweeps (jacobi_resident.cu)
@@ -146,7 +159,7 @@ struct picard_ctx {
   picard_stats stats = {};
   long long launches_at_reset = 0;
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  cudaEvent_t pev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};  // phase boundaries
+  cudaEvent_t pev[12] = {};  // phase boundaries of two steps (the one running and the one before)
 };
 
 namespace picard {
@@ -154,11 +167,11 @@ int fail(int code, const std::string& msg);
 int check_cuda(cudaError_t e, const char* what);
 picard::KParams make_kparams(const picard_params& p);
 picard::InflowTable make_inflow_table(const picard_params& p);
+// Whether ParticlesProduce can create a particle with these parameters.
+bool has_neutral_source(const KParams& K);
 // Reads the device particle count into ctx->num_local after surfacing any
-// device-side capacity error.
-int sync_count_public(picard_ctx* c);
-// The same in two halves, so that many contexts' counts travel together:
-// count_issue queues the copies, count_collect waits for the context's stream.
+// device-side error, in two halves so that many contexts' counts travel
+// together: count_issue queues the copy, count_collect waits for the stream.
 int count_issue(picard_ctx* c);
 // BCpotentials without waiting for the device: a tensor-core timeout stays in
 // the context's error word, which the Jacobi solve that follows reads.
@@ -204,27 +217,12 @@ int bc_potentials_batch(picard_ctx** ctxs, int n, cudaStream_t bst, cudaEvent_t*
 void bcpot_fft_invalidate(picard_ctx* c);
 void bcpot_fft_free(picard_ctx* c);
 long long spectral_bytes(const KParams& K);
-int solve_spectral(picard_ctx* c, double tol, long long smax, int maxit, long long* sweeps, bool* converged);
-// The same solve as a resumable state machine, so that a batch of runs can
-// take its host round trips together: spec_begin queues the initial residual,
-// the forward transform and the first Parseval evaluation; after the run's
-// stream has been synchronised, spec_collect reads the evaluation and queues
-// the next one, or the scaling, inverse transform and update of U (then
-// done is set; spec_account books the device time once the stream has passed
-// that work).
-struct SpecSolve {
-  picard_ctx* c = nullptr;
-  double tol2 = 0.0, r2_hit = 0.0, f1 = 0.0;  // f1: ||r_1||^2 from the doubling pass
-  long long smax = 0, dmax = 0, lo = 0, hi = 0;
-  long long d0 = 0, step = 0, d = 0;  // pending evaluation; the accepted sweep count
-  int count = 0;
-  bool doubling = false, final_eval = false, done = false, converged = true;
-};
-int spec_begin(SpecSolve& Q, picard_ctx* c, double tol, long long smax, int maxit);
-int spec_collect(SpecSolve& Q);
-int spec_finish_issue(SpecSolve& Q);
-int spec_apply_issue(SpecSolve& Q);
-void spec_account(SpecSolve& Q);
+// Queues the whole closed-form solve on the context's stream (set-up, search,
+// iterate, periodic ghosts, copy of its SpecState to the host).
+int spec_issue(picard_ctx* c, double maxerr, int maxit);
+// After the stream has passed it: books the solve and reports its sweeps and
+// status (PICARD_ERR_NOT_CONVERGED included).  Zero sweeps when none is pending.
+int spec_collect(picard_ctx* c, long long* sweeps);
 }  // namespace picard
 
 #define PICARD_CUDA(expr)                                          \

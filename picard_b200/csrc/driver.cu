@@ -241,44 +241,78 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
   const picard_params& p = c->prm;
   const KParams& K = c->K;
   const int cells = p.nx * p.ny * p.nz;
+  const bool source = has_neutral_source(K);
   bool nc = false;
   bool advanced = false;  // the previous step's push already advanced the positions
-  for (int32_t it = iter_start + 1; it <= iter_end; ++it) {
-    PICARD_CUDA(cudaEventRecord(c->pev[0], c->st));
-    // AdvancePosition on the particles present before BCinflow
-    if (!advanced) PICARD_TRY(picard_gpu_advance_position(c, p.dt));
-    // ParticlesProduce, appended behind them (device-side count)
-    PICARD_CUDA(launch_produce_count(K, it, c->cell_counts, c->st));
-    PICARD_CUDA(launch_scan_int(c->cell_counts, c->cell_offsets, cells, c->cell_offsets + cells,
-                                c->cell_offsets + cells + 2, c->st));
-    if (c->layout == PICARD_LAYOUT_F64)
-      PICARD_CUDA(launch_produce_emit_f64(K, it, c->cell_offsets, c->f64, c->d_count, c->capacity,
-                                          c->d_err, c->st));
-    else
-      PICARD_CUDA(launch_produce_emit_c32(K, it, c->cell_offsets, c->c32, c->d_count, c->capacity,
-                                          c->d_err, c->st));
-    PICARD_TRY(sync_count_public(c));
-    // BCoutflow + ParticlesTransfer in place, in the reference's order
-    PICARD_CUDA(launch_outflow(c, 1));
-    // BCinflow + AdvancePosition + BCoutflow + ParticlesTransfer of the new particles
-    PICARD_CUDA(launch_inflow_fused(c, it));
-    PICARD_TRY(sync_count_public(c));
-    // ParticlesTransfer's slot: every sort_every iterations, the particles
-    // put back in cell order (a permutation; nothing downstream depends on it)
-    if (c->sort_every > 0 && it % c->sort_every == 0) PICARD_TRY(sort_particles(c));
-    PICARD_CUDA(cudaEventRecord(c->pev[1], c->st));
-    PICARD_TRY(picard_gpu_particles_gridify(c));
-    PICARD_CUDA(cudaEventRecord(c->pev[2], c->st));
-    PICARD_TRY(bc_potentials_async(c));  // a timeout surfaces through the solve's error check
-    PICARD_CUDA(cudaEventRecord(c->pev[3], c->st));
-    int32_t sw = 0;
-    int rc = picard_gpu_calc_epotential(c, p.maxerr, p.maxit, &sw);
+  bool open = false;      // the previous step's events and closed-form solve are still to be read
+  // A step is queued up to its velocity push without waiting for its solve; what
+  // the host has to know of it is read at the next step's particle count, so the
+  // device has work while the host goes from one step to the next.
+  auto settle = [&](const cudaEvent_t* ev) -> int {
+    if (!open) return PICARD_OK;
+    open = false;
+    for (int ph = 0; ph < 5; ++ph) {
+      float ms = 0.0f;
+      if (cudaEventElapsedTime(&ms, ev[ph], ev[ph + 1]) == cudaSuccess) c->stats.phase_ms[ph] += ms;
+    }
+    long long sw = 0;
+    const int rc = spec_collect(c, &sw);
+    if (sweeps_total) *sweeps_total += sw;
     if (rc == PICARD_ERR_NOT_CONVERGED)
       nc = true;
     else if (rc != PICARD_OK)
       return rc;
-    if (sweeps_total) *sweeps_total += sw;
-    PICARD_CUDA(cudaEventRecord(c->pev[4], c->st));
+    return PICARD_OK;
+  };
+  c->spec.pending = false;
+  for (int32_t it = iter_start + 1; it <= iter_end; ++it) {
+    const cudaEvent_t* ev = c->pev + 6 * (it & 1);
+    const cudaEvent_t* before = c->pev + 6 * (1 - (it & 1));
+    PICARD_CUDA(cudaEventRecord(ev[0], c->st));
+    // AdvancePosition on the particles present before BCinflow
+    if (!advanced) PICARD_TRY(picard_gpu_advance_position(c, p.dt));
+    // ParticlesProduce, appended behind them (device-side count)
+    if (source) {
+      PICARD_CUDA(launch_produce_count(K, it, c->cell_counts, c->st));
+      PICARD_CUDA(launch_scan_int(c->cell_counts, c->cell_offsets, cells, c->cell_offsets + cells,
+                                  c->cell_offsets + cells + 2, c->st));
+      if (c->layout == PICARD_LAYOUT_F64)
+        PICARD_CUDA(launch_produce_emit_f64(K, it, c->cell_offsets, c->f64, c->d_count, c->capacity,
+                                            c->d_err, c->st));
+      else
+        PICARD_CUDA(launch_produce_emit_c32(K, it, c->cell_offsets, c->c32, c->d_count, c->capacity,
+                                            c->d_err, c->st));
+      PICARD_TRY(count_issue(c));
+      PICARD_TRY(count_collect(c));
+      PICARD_TRY(settle(before));
+    }
+    // BCoutflow + ParticlesTransfer in place, in the reference's order
+    PICARD_CUDA(launch_outflow(c, 1));
+    // BCinflow + AdvancePosition + BCoutflow + ParticlesTransfer of the new particles
+    PICARD_CUDA(launch_inflow_fused(c, it));
+    PICARD_TRY(count_issue(c));
+    PICARD_TRY(count_collect(c));
+    PICARD_TRY(settle(before));
+    // ParticlesTransfer's slot: every sort_every iterations, the particles
+    // put back in cell order (a permutation; nothing downstream depends on it)
+    if (c->sort_every > 0 && it % c->sort_every == 0) PICARD_TRY(sort_particles(c));
+    PICARD_CUDA(cudaEventRecord(ev[1], c->st));
+    PICARD_TRY(picard_gpu_particles_gridify(c));
+    PICARD_CUDA(cudaEventRecord(ev[2], c->st));
+    PICARD_TRY(bc_potentials_async(c));  // a timeout surfaces through the solve's error check
+    PICARD_CUDA(cudaEventRecord(ev[3], c->st));
+    if (c->solver == PICARD_SOLVER_SPECTRAL) {
+      PICARD_TRY(spec_issue(c, p.maxerr, p.maxit));
+    } else {
+      int32_t sw = 0;
+      int rc = picard_gpu_calc_epotential(c, p.maxerr, p.maxit, &sw);
+      if (rc == PICARD_ERR_NOT_CONVERGED)
+        nc = true;
+      else if (rc != PICARD_OK)
+        return rc;
+      if (sweeps_total) *sweeps_total += sw;
+    }
+    PICARD_CUDA(cudaEventRecord(ev[4], c->st));
     PICARD_TRY(picard_gpu_calc_efield(c));
     // AdvanceVelocity; in the CELL32 layout, when another step follows, fused
     // with that step's AdvancePosition (one pass over the particles)
@@ -287,17 +321,13 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
       PICARD_CUDA(launch_push_advance_c32(K, c->c32, c->num_local, c->E32, p.dt, c->st));
     else
       PICARD_TRY(picard_gpu_advance_velocity(c, p.dt));
-    PICARD_CUDA(cudaEventRecord(c->pev[5], c->st));
-    PICARD_CUDA(cudaEventSynchronize(c->pev[5]));
-    for (int ph = 0; ph < 5; ++ph) {
-      float ms = 0.0f;
-      if (cudaEventElapsedTime(&ms, c->pev[ph], c->pev[ph + 1]) == cudaSuccess) c->stats.phase_ms[ph] += ms;
-    }
+    PICARD_CUDA(cudaEventRecord(ev[5], c->st));
+    open = true;
     c->stats.steps += 1;
     c->stats.particle_steps += c->num_local;
   }
-  PICARD_CUDA(cudaStreamSynchronize(c->st));
-  PICARD_TRY(check_dev_err_public(c));  // a wait that gave up in the last step
+  PICARD_TRY(check_dev_err_public(c));  // waits for the stream; a wait that gave up in the last step
+  PICARD_TRY(settle(c->pev + 6 * (iter_end & 1)));
   if (nc) return fail(PICARD_ERR_NOT_CONVERGED, "at least one Jacobi solve hit 2*maxit+1 sweeps");
   return PICARD_OK;
 }

@@ -41,6 +41,7 @@ struct F32Solve {
 
 // CalcEpotential's set-up and wrap-up around the solve loop.
 constexpr int kPinnedB2 = kMaxSweepsPerRound + 8;  // slot of ||b||^2 in ctx->h_pinned (past the r2 copies)
+constexpr int kPinnedSpec = kMaxSweepsPerRound + 16;  // slots of a queued closed-form solve's SpecState
 struct EpotSetup {
   double bnorm = 0.0, tol = 0.0, sigma = 1.0;
   long long smax = 0;
@@ -51,7 +52,9 @@ struct EpotSetup {
 int epot_rhs_issue(picard_ctx* c);
 // after the copy has landed
 EpotSetup epot_setup(picard_ctx* c, double maxerr, int32_t maxit);
-// periodic ghost refresh, statistics, status
+// statistics and status of a finished solve
+int epot_account(picard_ctx* c, double bnorm, double residual, long long smax, long long sweeps, bool converged);
+// the same after a periodic ghost refresh
 int epot_finish(picard_ctx* c, const EpotSetup& e, long long sweeps, bool converged, int32_t* sweeps_out);
 
 int f32_begin(F32Solve& S, picard_ctx* c, double tol, long long smax, int maxit, double sigma);

@@ -358,19 +358,24 @@ EpotSetup epot_setup(picard_ctx* c, double maxerr, int32_t maxit) {
   return e;
 }
 
-int epot_finish(picard_ctx* c, const EpotSetup& e, long long sweeps, bool converged, int32_t* sweeps_out) {
-  if (e.trivial) c->last_residual = e.bnorm;
-  PICARD_CUDA(launch_refresh_periodic(c->K, c->U, c->st));
+int epot_account(picard_ctx* c, double bnorm, double residual, long long smax, long long sweeps, bool converged) {
+  c->last_bnorm = bnorm;
+  c->last_residual = residual;
   c->last_sweeps = sweeps;
   c->stats.solves += 1;
   c->stats.sweeps += sweeps;
-  c->stats.last_residual = c->last_residual;
-  c->stats.last_bnorm = e.bnorm;
-  if (sweeps_out) *sweeps_out = int32_t(sweeps);
+  c->stats.last_residual = residual;
+  c->stats.last_bnorm = bnorm;
   if (!converged)
     return fail(PICARD_ERR_NOT_CONVERGED,
-                "Jacobi reached 2*maxit+1 = " + std::to_string(e.smax) + " sweeps without meeting maxerr");
+                "Jacobi reached 2*maxit+1 = " + std::to_string(smax) + " sweeps without meeting maxerr");
   return PICARD_OK;
+}
+
+int epot_finish(picard_ctx* c, const EpotSetup& e, long long sweeps, bool converged, int32_t* sweeps_out) {
+  PICARD_CUDA(launch_refresh_periodic(c->K, c->U, c->st));
+  if (sweeps_out) *sweeps_out = int32_t(sweeps);
+  return epot_account(c, e.bnorm, e.trivial ? e.bnorm : c->last_residual, e.smax, sweeps, converged);
 }
 
 }  // namespace picard
@@ -378,6 +383,14 @@ int epot_finish(picard_ctx* c, const EpotSetup& e, long long sweeps, bool conver
 extern "C" int picard_gpu_calc_epotential(picard_ctx* c, double maxerr, int32_t maxit, int32_t* sweeps_out) {
   if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
   if (maxit < 0) return fail(PICARD_ERR_BAD_ARG, "maxit must be >= 0");
+  if (c->solver == PICARD_SOLVER_SPECTRAL) {
+    long long done = 0;
+    PICARD_TRY(spec_issue(c, maxerr, maxit));
+    PICARD_CUDA(cudaStreamSynchronize(c->st));
+    const int rc = spec_collect(c, &done);
+    if (sweeps_out) *sweeps_out = int32_t(done);
+    return rc;
+  }
   PICARD_TRY(epot_rhs_issue(c));
   PICARD_CUDA(cudaStreamSynchronize(c->st));
   const EpotSetup e = epot_setup(c, maxerr, maxit);
@@ -387,8 +400,6 @@ extern "C" int picard_gpu_calc_epotential(picard_ctx* c, double maxerr, int32_t 
     sweeps = 0;
   } else if (c->solver == PICARD_SOLVER_F64) {
     PICARD_TRY(solve_f64(c, e.tol, e.smax, maxit, &sweeps, &converged));
-  } else if (c->solver == PICARD_SOLVER_SPECTRAL) {
-    PICARD_TRY(solve_spectral(c, e.tol, e.smax, maxit, &sweeps, &converged));
   } else {
     PICARD_TRY(solve_f32(c, e.tol, e.smax, maxit, e.sigma, &sweeps, &converged));
   }

@@ -22,7 +22,9 @@
 // ||r_d|| does not increase with d (|g| <= 1), and the stopping sweep of the
 // reference -- the first iterate d >= 1 with d + 1 <= maxit and
 // ||r_d|| <= maxerr ||b|| -- is found by a bracketing search: each launch
-// evaluates the Parseval sum at up to kSpecPoints sweep counts.
+// evaluates the Parseval sum at up to kSpecPoints sweep counts, and its last
+// block narrows the bracket and chooses the next ones (SpecState), so that the
+// whole solve is queued without a host round trip.
 //
 // The transforms are per-axis products, one launch each, on the FP64 tensor
 // cores (spec_axis_kernel).  Every axis basis is folded by its even / odd
@@ -35,10 +37,12 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "context.cuh"
 #include "picard_gpu.h"
+#include "solve_f32.cuh"
 
 namespace picard {
 
@@ -46,6 +50,7 @@ namespace {
 
 constexpr int kSpecPoints = 32;     // sweep counts per evaluation launch
 constexpr int kSpecThreads = 256;
+enum SpecPhase { kSpecDoubling = 0, kSpecUniform = 1, kSpecFinal = 2 };
 constexpr int kAxTile = 64, kAxK = 16;  // spec_axis_kernel: 64 x 64 outputs per parity, K chunks of 16
 
 // Element t of a compact nx x ny array of planes -> (i, j, k).  T is 32 bits
@@ -60,12 +65,31 @@ __device__ __forceinline__ void split3(T t, int nx, int ny, int& i, int& j, int&
 }
 inline bool fits32(long long n) { return n < (1LL << 31); }
 
-// r_0 = b - L U over the interior, compact x-fastest (CalcEpotential.f90:83-92;
-// periodic axes read the wrapped interior instead of the ghost).
+// The sum over the block of one value per thread, in thread 0 (fixed order).
+__device__ __forceinline__ double block_sum(double v, double* sh) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = 0.0;
+  if (threadIdx.x == 0)
+    for (int w = 0; w < int(blockDim.x >> 5); ++w) t += sh[w];
+  return t;
+}
+
+// b = -C/(dV eps0) and r_0 = b - L U over the interior, compact x-fastest
+// (CalcEpotential.f90:50-54, 83-92; periodic axes read the wrapped interior
+// instead of the ghost), ||b||^2, and from it, in the last block, the start of
+// the stopping-sweep search.  The test at the top of sweep 1 uses ||b|| itself
+// (CalcEpotential.f90:55-61).
 template <class T>
-__global__ void spec_r0_kernel(KParams P, double idx2, double idy2, double idz2, const double* __restrict__ U,
-                               const double* __restrict__ b, double* __restrict__ R) {
+__global__ void __launch_bounds__(kSpecThreads) spec_begin_kernel(KParams P, double idx2, double idy2, double idz2,
+                                                                  double binv, const double* __restrict__ C,
+                                                                  const double* __restrict__ U, double* __restrict__ R,
+                                                                  double maxerr, int maxit,
+                                                                  double* __restrict__ partial, unsigned int* counter,
+                                                                  SpecState* state) {
   const T n = T(P.nx) * T(P.ny) * T(P.nz);
+  double b2 = 0.0;
   for (T t = T(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += T(gridDim.x) * blockDim.x) {
     int i, j, k;
     split3(t, P.nx, P.ny, i, j, k);
@@ -73,12 +97,57 @@ __global__ void spec_r0_kernel(KParams P, double idx2, double idy2, double idz2,
     const int im = (i == 1 && !P.xflow) ? P.nx : i - 1, ip = (i == P.nx && !P.xflow) ? 1 : i + 1;
     const int jm = (j == 1 && !P.yflow) ? P.ny : j - 1, jp = (j == P.ny && !P.yflow) ? 1 : j + 1;
     const int km = (k == 1 && !P.zflow) ? P.nz : k - 1, kp = (k == P.nz && !P.zflow) ? 1 : k + 1;
-    const double u = U[node_index(P, i, j, k)];
+    const long long g = node_index(P, i, j, k);
+    const double u = U[g];
     const double lap = (U[node_index(P, ip, j, k)] + U[node_index(P, im, j, k)] - 2.0 * u) * idx2 +
                        (U[node_index(P, i, jp, k)] + U[node_index(P, i, jm, k)] - 2.0 * u) * idy2 +
                        (U[node_index(P, i, j, kp)] + U[node_index(P, i, j, km)] - 2.0 * u) * idz2;
-    R[t] = b[node_index(P, i, j, k)] - lap;
+    const double b = -C[g] * binv;
+    R[t] = b - lap;
+    b2 += b * b;
   }
+  __shared__ double sh[kSpecThreads / 32];
+  __shared__ bool last;
+  b2 = block_sum(b2, sh);
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = b2;
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) v += __ldcg(partial + b);
+  v = block_sum(v, sh);
+  if (threadIdx.x != 0) return;
+  *counter = 0u;
+  SpecState Q;
+  Q.bnorm = sqrt(v);
+  const double tol = maxerr * Q.bnorm;
+  Q.tol2 = tol * tol;
+  Q.f1 = Q.r2_hit = 0.0;
+  Q.smax = 2LL * maxit + 1;
+  Q.dmax = (long long)maxit - 1;
+  Q.lo = 0;
+  Q.hi = Q.dmax + 1;
+  Q.d = 0;
+  Q.d0 = 1;
+  Q.step = 0;
+  Q.g2_skip = -1.0;
+  Q.trivial = 1 <= maxit && Q.bnorm <= tol;
+  Q.done = Q.trivial;
+  Q.converged = 1;
+  if (Q.dmax >= 1) {
+    Q.phase = kSpecDoubling;
+    Q.count = 1;
+    while (Q.count < kSpecPoints && (1LL << (Q.count - 1)) < Q.dmax) ++Q.count;
+  } else {
+    Q.phase = kSpecFinal;
+    Q.d0 = Q.smax;
+    Q.count = 1;
+  }
+  *state = Q;
 }
 
 // D += A B for one 8 x 4 by 4 x 8 FP64 tile: lane l holds A[l / 4][l % 4],
@@ -120,7 +189,9 @@ template <bool INV, bool X, bool APPLY>
 __global__ void __launch_bounds__(256, 2) spec_axis_kernel(const double* __restrict__ in, double* __restrict__ out,
                                                            const double* __restrict__ Pe,
                                                            const double* __restrict__ Po, int n, int ne, int no, int s,
-                                                           long long I, int rows, KParams P, double* __restrict__ U) {
+                                                           long long I, int rows, KParams P, double* __restrict__ U,
+                                                           const SpecState* __restrict__ state) {
+  if (APPLY && state->trivial) return;  // zero sweeps: U stays
   // row strides 4 mod 16 doubles: the 16 lanes of a half-warp read 16 banks
   __shared__ double sh[2 * kAxTile * (kAxK + 4) + 2 * kAxK * (kAxTile + 4)];
   double(*As)[kAxTile][kAxK + 4] = reinterpret_cast<double(*)[kAxTile][kAxK + 4]>(sh);
@@ -299,24 +370,81 @@ __device__ inline double ipow(double x, long long e) {
   return r;
 }
 
+// The stopping-sweep search: the first d in [1, dmax] with f(d) <= tol^2
+// (checked at the top of sweep d + 1 <= maxit).  Invariant: f(lo) > tol^2
+// (lo = 0: no sweep yet), and f(hi) <= tol^2 when hi <= dmax (hi = dmax + 1:
+// no passing d known).  The first evaluation doubles d from 1 up to the first
+// power of two >= dmax; later ones take up to 32 candidates of (lo, hi) at
+// equal steps, which leaves a bracket of ceil((hi - lo) / 33).  Without a
+// passing d the iterate of sweep smax is kept, after f(smax) (its residual).
+//
+// Modes whose g^2 is at most g2_skip add at most 2^-60 tol^2 to any f(d) that
+// an evaluation at equal steps takes (d > lo): sum over those modes of w
+// g^(2d) <= g2_max^(d-1) f(1).  None is skipped while lo < 2 or f(1) is unknown.
+__device__ void spec_advance(SpecState& Q, const double* f) {
+  if (Q.phase == kSpecFinal) {
+    Q.d = Q.smax;
+    Q.converged = 0;
+    Q.r2_hit = f[0];
+    Q.done = 1;
+    return;
+  }
+  const bool doubling = Q.phase == kSpecDoubling;
+  if (doubling) Q.f1 = f[0];
+  for (int t = 0; t < Q.count; ++t) {
+    const long long d = doubling ? 1LL << t : Q.d0 + Q.step * t;
+    if (d > Q.dmax) break;
+    if (f[t] <= Q.tol2) {
+      Q.hi = d;
+      Q.r2_hit = f[t];
+      break;
+    }
+    Q.lo = d;
+  }
+  if (Q.hi - Q.lo > 1) {
+    Q.phase = kSpecUniform;
+    Q.step = (Q.hi - Q.lo + kSpecPoints) / (kSpecPoints + 1);
+    const long long cnt = (Q.hi - Q.lo - 1) / Q.step;
+    Q.count = int(cnt < kSpecPoints ? cnt : kSpecPoints);
+    Q.d0 = Q.lo + Q.step;
+    Q.g2_skip = -1.0;
+    if (Q.lo >= 2 && Q.f1 > 0.0 && Q.tol2 > 0.0) {
+      const double ratio = Q.tol2 * 0x1p-60 / Q.f1;
+      if (ratio < 1.0) Q.g2_skip = exp(log(ratio) / double(Q.lo - 1));
+    }
+  } else if (Q.hi <= Q.dmax) {
+    Q.d = Q.hi;
+    Q.done = 1;
+  } else {
+    Q.phase = kSpecFinal;
+    Q.d0 = Q.smax;
+    Q.step = 1;
+    Q.count = 1;
+    Q.g2_skip = -1.0;
+  }
+}
+
 // What bounds it: the FP64 powers at large sizes, the final sum at small ones.
 // 256 x 128 x 128 37 us (76 with 64-bit element indices, 160 shuffles a warp
 // and a last block that read the partials one point at a time), 77^3 14 us (42).
 //
-// Parseval sums f(d_t) = sum_m g_m^(2 d_t) rh_m^2 at the sweep counts
-// d_t = d0 + t*step (doubling == 0) or d_t = d0 * 2^t (doubling == 1), for
-// t < count.  Modes with g^2 <= g2_skip add nothing (the caller bounds what
-// they could add far below the stop test's resolution).  Per-block partials
-// in a fixed order; the last block to finish sums them (in block order) into
-// out[t] and re-arms the counter.
+// One step of the search: the Parseval sums f(d_t) = sum_m g_m^(2 d_t) rh_m^2
+// at the sweep counts d_t = d0 2^t (the first evaluation) or d0 + t step, t <
+// count.  Modes with g^2 <= g2_skip add nothing (spec_advance bounds what they
+// could add far below the stop test's resolution).  Per-block partials in a
+// fixed order; the last block to finish sums them, re-arms the counter and
+// moves the search on.  A finished search returns at once.
 template <class T>
 __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* __restrict__ Rh, int nx, int ny,
                                                                   int nz, const double* __restrict__ omx,
                                                                   const double* __restrict__ omy,
-                                                                  const double* __restrict__ omz, long long d0,
-                                                                  long long step, int count, int doubling,
-                                                                  double g2_skip, double* __restrict__ partial,
-                                                                  unsigned int* counter, double* __restrict__ out) {
+                                                                  const double* __restrict__ omz,
+                                                                  double* __restrict__ partial, unsigned int* counter,
+                                                                  SpecState* state) {
+  if (state->done) return;
+  const long long d0 = state->d0, step = state->step;
+  const int count = state->count, doubling = state->phase == kSpecDoubling;
+  const double g2_skip = state->g2_skip;
   double acc[kSpecPoints];
 #pragma unroll
   for (int t = 0; t < kSpecPoints; ++t) acc[t] = 0.0;
@@ -390,9 +518,15 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
   if (threadIdx.x < kSpecPoints) {
     double v = 0.0;
     for (int w2 = 0; w2 < kSpecThreads / 32; ++w2) v += sh[w2][threadIdx.x];
-    out[threadIdx.x] = v;
+    sh[0][threadIdx.x] = v;  // this thread's own column
   }
-  if (threadIdx.x == 0) *counter = 0u;
+  __syncwarp();
+  if (threadIdx.x == 0) {
+    *counter = 0u;
+    SpecState Q = *state;
+    spec_advance(Q, sh[0]);
+    *state = Q;
+  }
 }
 
 // rh -> -af (1 - g^d)/(1 - g) rh in place.  For g > 0 the factor is
@@ -400,8 +534,10 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
 // omg == 0 (every axis periodic, the constant mode) takes d.
 template <class T>
 __global__ void spec_scale_kernel(double* __restrict__ Rh, int nx, int ny, int nz, const double* __restrict__ omx,
-                                  const double* __restrict__ omy, const double* __restrict__ omz, long long d,
-                                  double af) {
+                                  const double* __restrict__ omy, const double* __restrict__ omz, double af,
+                                  const SpecState* __restrict__ state) {
+  const long long d = state->d;
+  if (state->trivial) return;
   const T n = T(nx) * T(ny) * T(nz);
   for (T q = T(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += T(gridDim.x) * blockDim.x) {
     int mx, my, mz;
@@ -495,16 +631,16 @@ cudaError_t axis_pass(picard_ctx* c, int d, bool forward, const double* in, doub
   note_launch();
   if (d == 0 && forward)
     spec_axis_kernel<false, true, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
-                                                                  c->K, nullptr);
+                                                                  c->K, nullptr, S.state);
   else if (d == 0)
     spec_axis_kernel<true, true, true><<<grid, 256, 0, c->st>>>(in, nullptr, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
-                                                                c->K, c->U);
+                                                                c->K, c->U, S.state);
   else if (forward)
     spec_axis_kernel<false, false, false><<<grid, 256, 0, c->st>>>(in, out, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
-                                                                   c->K, nullptr);
+                                                                   c->K, nullptr, S.state);
   else
     spec_axis_kernel<true, false, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
-                                                                  c->K, nullptr);
+                                                                  c->K, nullptr, S.state);
   return cudaGetLastError();
 }
 
@@ -523,25 +659,16 @@ cudaError_t transform(picard_ctx* c, bool forward) {
   return axis_pass(c, 0, false, S.T[1], nullptr);
 }
 
-// Queues the evaluation of f at count (<= kSpecPoints) sweep counts and the
-// copy of the sums to c->h_pinned[0..count); the caller waits on the stream.
-int issue_norms(picard_ctx* c, long long d0, long long step, int count, bool doubling, double g2_skip) {
-  SpectralPlan& S = c->spec;
-  const long long n = (long long)c->K.nx * c->K.ny * c->K.nz;
-  note_launch();
-  if (fits32(n))
-    spec_norms_kernel<unsigned><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], c->K.nx, c->K.ny, c->K.nz, S.om[0], S.om[1],
-                                                                S.om[2], d0, step, count, doubling ? 1 : 0, g2_skip,
-                                                                S.partial, S.counter, S.sums);
-  else
-    spec_norms_kernel<long long><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], c->K.nx, c->K.ny, c->K.nz, S.om[0], S.om[1],
-                                                                S.om[2], d0, step, count, doubling ? 1 : 0, g2_skip,
-                                                                S.partial, S.counter, S.sums);
-  PICARD_CUDA(cudaGetLastError());
-  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned, S.sums, sizeof(double) * count, cudaMemcpyDeviceToHost, c->st));
-  c->stats.d2h_bytes += (int64_t)sizeof(double) * count;
-  S.evals += 1;
-  return PICARD_OK;
+// Evaluations that the search of spec_advance can need with this maxit: the
+// doubling one, the ones at equal steps for the widest bracket it can leave,
+// and f(smax).
+int max_evaluations(int maxit) {
+  if (maxit < 2) return 1;
+  long long gap = 1;
+  while (gap < maxit) gap <<= 1;
+  int e = 2;
+  for (; gap > 1; gap = (gap + kSpecPoints) / (kSpecPoints + 1)) ++e;
+  return e;
 }
 
 }  // namespace
@@ -581,8 +708,8 @@ int spectral_alloc(picard_ctx* c) {
   S.norm_blocks = std::min(stream_blocks(n), 148 * 4);
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * (size_t)S.norm_blocks * kSpecPoints));
   S.partial = static_cast<double*>(p);
-  PICARD_TRY(dev_alloc(c, &p, sizeof(double) * kSpecPoints));
-  S.sums = static_cast<double*>(p);
+  PICARD_TRY(dev_alloc(c, &p, sizeof(SpecState)));
+  S.state = static_cast<SpecState*>(p);
   PICARD_TRY(dev_alloc(c, &p, sizeof(unsigned int)));  // zeroed
   S.counter = static_cast<unsigned int*>(p);
   return PICARD_OK;
@@ -594,158 +721,67 @@ long long spectral_bytes(const KParams& K) {
                 K.ny + K.nz + (long long)stream_blocks(n) * kSpecPoints + kSpecPoints);
 }
 
-// The stopping-sweep search: the first d in [1, dmax] with f(d) <= tol^2
-// (checked at the top of sweep d + 1 <= maxit).  Invariant: f(lo) > tol^2
-// (lo = 0: no sweep yet), and f(hi) <= tol^2 when hi <= dmax (hi = dmax + 1:
-// no passing d known).  The first evaluation doubles d from 1 up to the
-// first power of two >= dmax; later ones take evenly spaced candidates of
-// (lo, hi).
-
-// Modes whose g^2 is at most the returned value add at most 2^-60 tol^2 to
-// any f(d) the uniform passes evaluate (d > lo): sum over those modes of
-// w g^(2d) <= g2_max^(d-1) f(1).  None is skipped while lo < 2 or f(1) is
-// unknown.
-static double skip_threshold(const SpecSolve& Q) {
-  if (Q.lo < 2 || !(Q.f1 > 0.0) || !(Q.tol2 > 0.0)) return -1.0;
-  const double ratio = Q.tol2 * 0x1p-60 / Q.f1;
-  if (!(ratio < 1.0)) return -1.0;
-  return std::exp(std::log(ratio) / double(Q.lo - 1));
-}
-
-int spec_begin(SpecSolve& Q, picard_ctx* c, double tol, long long smax, int maxit) {
+int spec_issue(picard_ctx* c, double maxerr, int maxit) {
   SpectralPlan& S = c->spec;
   const KParams& K = c->K;
   const long long n = (long long)K.nx * K.ny * K.nz;
   const JacobiCoef J = jacobi_coef(K);
-  Q = SpecSolve();
-  Q.c = c;
-  Q.tol2 = tol * tol;
-  Q.smax = smax;
-  Q.dmax = (long long)maxit - 1;
-  Q.lo = 0;
-  Q.hi = Q.dmax + 1;
+  const double ix = 1.0 / J.dx2, iy = 1.0 / J.dy2, iz = 1.0 / J.dz2, binv = 1.0 / (K.dV * kEps0);
+  const int nb = stream_blocks(n);  // at most 32 norm_blocks partials
   PICARD_CUDA(cudaEventRecord(c->ev[0], c->st));
   note_launch();
   if (fits32(n))
-    spec_r0_kernel<unsigned><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, 1.0 / J.dx2, 1.0 / J.dy2, 1.0 / J.dz2, c->U, c->b,
-                                                                S.T[0]);
+    spec_begin_kernel<unsigned><<<nb, kSpecThreads, 0, c->st>>>(K, ix, iy, iz, binv, c->C, c->U, S.T[0], maxerr, maxit,
+                                                                 S.partial, S.counter, S.state);
   else
-    spec_r0_kernel<long long><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(K, 1.0 / J.dx2, 1.0 / J.dy2, 1.0 / J.dz2, c->U, c->b,
-                                                                S.T[0]);
+    spec_begin_kernel<long long><<<nb, kSpecThreads, 0, c->st>>>(K, ix, iy, iz, binv, c->C, c->U, S.T[0], maxerr, maxit,
+                                                                  S.partial, S.counter, S.state);
   PICARD_CUDA(cudaGetLastError());
   PICARD_CUDA(transform(c, true));
   PICARD_CUDA(cudaEventRecord(c->ev[1], c->st));
-  if (Q.dmax >= 1) {
-    int cnt = 1;
-    while (cnt < kSpecPoints && (1LL << (cnt - 1)) < Q.dmax) ++cnt;
-    Q.d0 = 1;
-    Q.step = 0;
-    Q.count = cnt;
-    Q.doubling = true;
-    return issue_norms(c, 1, 0, cnt, true, -1.0);
+  for (int e = max_evaluations(maxit); e > 0; --e) {
+    note_launch();
+    if (fits32(n))
+      spec_norms_kernel<unsigned><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
+                                                                              S.om[2], S.partial, S.counter, S.state);
+    else
+      spec_norms_kernel<long long><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
+                                                                               S.om[2], S.partial, S.counter, S.state);
+    PICARD_CUDA(cudaGetLastError());
   }
-  return spec_finish_issue(Q);
-}
-
-int spec_collect(SpecSolve& Q) {
-  picard_ctx* c = Q.c;
-  if (Q.final_eval) {  // f(smax) of a solve without a hit
-    c->last_residual = std::sqrt(c->h_pinned[0]);
-    Q.final_eval = false;
-    return spec_apply_issue(Q);
-  }
-  if (Q.doubling) {
-    Q.f1 = c->h_pinned[0];  // f(1)
-    for (int t = 0; t < Q.count; ++t) {
-      const long long d = 1LL << t;
-      if (d > Q.dmax) break;
-      if (c->h_pinned[t] <= Q.tol2) {
-        Q.hi = d;
-        Q.r2_hit = c->h_pinned[t];
-        break;
-      }
-      Q.lo = d;
-    }
-    Q.doubling = false;
-  } else {
-    long long nlo = Q.d0 + Q.step * (Q.count - 1);
-    for (int t = 0; t < Q.count; ++t) {
-      if (c->h_pinned[t] <= Q.tol2) {
-        Q.hi = Q.d0 + Q.step * t;
-        Q.r2_hit = c->h_pinned[t];
-        nlo = Q.hi - Q.step;
-        break;
-      }
-    }
-    Q.lo = nlo;
-  }
-  if (Q.hi - Q.lo > 1) {
-    const long long span = Q.hi - 1 - Q.lo;  // candidates lo + 1 .. hi - 1
-    Q.step = (span + kSpecPoints - 1) / kSpecPoints;
-    Q.count = int(span / Q.step);
-    Q.d0 = Q.lo + Q.step;
-    return issue_norms(c, Q.d0, Q.step, Q.count, false, skip_threshold(Q));
-  }
-  return spec_finish_issue(Q);
-}
-
-int spec_finish_issue(SpecSolve& Q) {
-  picard_ctx* c = Q.c;
-  if (Q.hi <= Q.dmax) {
-    Q.d = Q.hi;
-    Q.converged = true;
-    c->last_residual = std::sqrt(Q.r2_hit);
-    return spec_apply_issue(Q);
-  }
-  Q.d = Q.smax;
-  Q.converged = false;
-  Q.final_eval = true;
-  return issue_norms(c, Q.smax, 1, 1, false, -1.0);
-}
-
-int spec_apply_issue(SpecSolve& Q) {
-  picard_ctx* c = Q.c;
-  SpectralPlan& S = c->spec;
-  const KParams& K = c->K;
-  const long long n = (long long)K.nx * K.ny * K.nz;
-  const JacobiCoef J = jacobi_coef(K);
   PICARD_CUDA(cudaEventRecord(c->ev[2], c->st));
   note_launch();
   if (fits32(n))
-    spec_scale_kernel<unsigned><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
-                                                                   S.om[2], Q.d, J.af);
+    spec_scale_kernel<unsigned><<<nb, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1], S.om[2],
+                                                                 J.af, S.state);
   else
-    spec_scale_kernel<long long><<<stream_blocks(n), kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
-                                                                   S.om[2], Q.d, J.af);
+    spec_scale_kernel<long long><<<nb, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1], S.om[2],
+                                                                  J.af, S.state);
   PICARD_CUDA(cudaGetLastError());
   PICARD_CUDA(transform(c, false));
   PICARD_CUDA(cudaEventRecord(c->ev[3], c->st));
-  Q.done = true;
+  PICARD_CUDA(launch_refresh_periodic(c->K, c->U, c->st));
+  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned + kPinnedSpec, S.state, sizeof(SpecState), cudaMemcpyDeviceToHost, c->st));
+  c->stats.d2h_bytes += sizeof(SpecState);
+  S.pending = true;
   return PICARD_OK;
 }
 
-// Device time of a finished solve (after its stream has passed ev[3]).
-void spec_account(SpecSolve& Q) {
-  picard_ctx* c = Q.c;
+int spec_collect(picard_ctx* c, long long* sweeps) {
+  *sweeps = 0;
+  if (!c->spec.pending) return PICARD_OK;
+  c->spec.pending = false;
+  SpecState Q;
+  std::memcpy(&Q, c->h_pinned + kPinnedSpec, sizeof(Q));
   float f0 = 0.f, f1 = 0.f;
   cudaEventElapsedTime(&f0, c->ev[0], c->ev[1]);
   cudaEventElapsedTime(&f1, c->ev[2], c->ev[3]);
-  c->stats.spectral_transforms += 2;
-  c->stats.spectral_transform_ms += f0 + f1;
-}
-
-int solve_spectral(picard_ctx* c, double tol, long long smax, int maxit, long long* sweeps, bool* converged) {
-  SpecSolve Q;
-  PICARD_TRY(spec_begin(Q, c, tol, smax, maxit));
-  for (;;) {
-    PICARD_CUDA(cudaStreamSynchronize(c->st));
-    if (Q.done) break;
-    PICARD_TRY(spec_collect(Q));
+  if (!Q.trivial) {
+    c->stats.spectral_transforms += 2;
+    c->stats.spectral_transform_ms += f0 + f1;
   }
-  spec_account(Q);
   *sweeps = Q.d;
-  *converged = Q.converged;
-  return PICARD_OK;
+  return epot_account(c, Q.bnorm, Q.trivial ? Q.bnorm : std::sqrt(Q.r2_hit), Q.smax, Q.d, Q.converged != 0);
 }
 
 }  // namespace picard

@@ -50,3 +50,23 @@ def test_axis_passes_at_tile_edges(dims, flows):
     assert err < 1e-11
     for s in sims:
         s.close()
+
+
+@pytest.mark.parametrize("maxerr", [0.9, 1e-2, 1e-6])
+@pytest.mark.parametrize("maxit", [0, 1, 2, 3, 34, 67, 100, 1100])
+def test_search_stops_where_the_sweeps_stop(maxit, maxerr):
+    # the on-device search at every cap that changes its evaluations: no test
+    # at all (0, 1), one candidate, one and two brackets of 33, and caps above
+    # and below the sweep that passes; a charge of zero takes no sweep
+    p = boxed(12, 10, 9)
+    o = O.OracleState(p)
+    for C in (blobs(o, p, seed=4), np.zeros_like(o.C)):
+        out = []
+        for kw in (SPEC64, F64):
+            with Simulation(p, derive=False, **kw) as s:
+                s.set_field(capi.FIELD_C, C)
+                s.set_field(capi.FIELD_U, np.zeros_like(C))
+                n = s.calc_epotential(maxerr=maxerr, maxit=maxit)
+                out.append((n, s.field(capi.FIELD_U)))
+        assert out[0][0] == out[1][0]
+        assert rel_l2(out[0][1], out[1][1]) < 1e-11
