@@ -17,13 +17,15 @@
 // plane (rows along P keep LP/2+1 outputs, then columns along Q), the
 // contraction over planes against the precomputed slice transforms (the
 // constant (2 tau eps0)^-1 / (LP LQ) folded in), and one inverse FFT per face.
-// FP64 throughout: radix-4 Stockham FFTs (one radix-2 stage for odd powers
-// of two) in shared memory with twiddles computed on the host.  The slice transforms depend only on D and are
-// computed on the first call after D changes.
+// FP64 throughout: FFTs of radix 8 and 4 in registers (fft_block), the
+// twiddles computed on the host.  The slice transforms depend only on D and
+// are computed on the first call after D changes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "context.cuh"
@@ -33,71 +35,171 @@ namespace picard {
 namespace {
 
 constexpr int kFftThreads = 256;
-constexpr int kColElems = 1024;   // B2 * LQ per column CTA (4 elements per thread)
-constexpr int kRowElems = 2048;   // B1 * LP per row CTA
+constexpr int kFftPer = 8;                           // elements per thread
+constexpr int kFftElems = kFftThreads * kFftPer;     // elements per block: 2048 / L transforms of length L
+constexpr int kMinLog = 3, kMaxLog = 11;             // transform lengths 8 .. 2048
+constexpr int kMaxQ = 1024, kMaxP = 2048;            // accepted circular lengths along Q and P
 
-__device__ inline double2 cmul(double2 a, double2 b) {
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+// a times -i (forward) or +i (inverse)
+template <bool INV>
+__device__ __forceinline__ double2 crot(double2 a) {
+  return INV ? make_double2(-a.y, a.x) : make_double2(a.y, -a.x);
+}
 
-// B sequences of length L (a power of two) in x (x[b*L + i]); Stockham
-// stages ping-pong between x and y: one radix-2 stage when log2 L is odd, then
-// radix-4 stages.  Returns the buffer holding the transform (natural order).
-// tw[t] = exp(-2 pi i t / L), t < L; inv uses the conjugates (no scaling).
-__device__ double2* fft_batch(double2* x, double2* y, int L, int logL, int B, const double2* __restrict__ tw,
-                              bool inv) {
-  int s = 0;  // log2 of the sub-transform length Ns done so far
-  if (logL & 1) {
-    const int half = L >> 1;
-    for (int e = threadIdx.x; e < B * half; e += blockDim.x) {
-      const int b = e >> (logL - 1), j = e & (half - 1);
-      const double2* xb = x + (b << logL);
-      double2* yb = y + (b << logL);
-      const double2 v0 = xb[j], v1 = xb[j + half];
-      yb[2 * j] = make_double2(v0.x + v1.x, v0.y + v1.y);
-      yb[2 * j + 1] = make_double2(v0.x - v1.x, v0.y - v1.y);
-    }
-    __syncthreads();
-    double2* t = x;
-    x = y;
-    y = t;
-    s = 1;
+// Transforms of length 4 and 8 in registers, natural order in and out.
+template <bool INV>
+__device__ __forceinline__ void fft4(double2& v0, double2& v1, double2& v2, double2& v3) {
+  const double2 a = cadd(v0, v2), b = csub(v0, v2), c = cadd(v1, v3), d = crot<INV>(csub(v1, v3));
+  v0 = cadd(a, c);
+  v1 = cadd(b, d);
+  v2 = csub(a, c);
+  v3 = csub(b, d);
+}
+template <bool INV>
+__device__ __forceinline__ void fft8(double2 v[8]) {
+  const double h = 0.70710678118654752440;  // sqrt(1/2)
+  fft4<INV>(v[0], v[2], v[4], v[6]);
+  fft4<INV>(v[1], v[3], v[5], v[7]);
+  const double2 o1 = v[3], o2 = v[5], o3 = v[7];  // the odd half, in its order 0, 1, 2, 3
+  const double2 r1 = crot<INV>(o1), r3 = crot<INV>(o3);
+  const double2 w1 = make_double2(h * (o1.x + r1.x), h * (o1.y + r1.y));
+  const double2 w2 = crot<INV>(o2);
+  const double2 w3 = make_double2(h * (r3.x - o3.x), h * (r3.y - o3.y));
+  const double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1];
+  v[0] = cadd(e0, o0), v[4] = csub(e0, o0);
+  v[1] = cadd(e1, w1), v[5] = csub(e1, w1);
+  v[2] = cadd(e2, w2), v[6] = csub(e2, w2);
+  v[3] = cadd(e3, w3), v[7] = csub(e3, w3);
+}
+
+// log2 of the radix of the pass that has `done` of `LOG` bits behind it: 8
+// where three bits are left for it and the rest is not one bit, else 4 or 2.
+__host__ __device__ constexpr int pass_bits(int left) {
+  return left == 1 ? 1 : left == 2 || left == 4 ? 2 : 3;
+}
+constexpr int last_bits(int log) { return log <= 3 ? pass_bits(log) : last_bits(log - pass_bits(log)) ; }
+
+// Shared index of element i of a transform: one 16-byte slot of padding for
+// every eight, so that a pass's writes 8 apart fall into different banks.
+__device__ __forceinline__ int fpad(int i) { return i + (i >> 3); }
+// Slots per transform: odd, or for fewer than eight transforms per block 8 over
+// their number mod 8, so that the transforms which a quarter-warp touches
+// together lie in different banks.
+template <int LOG>
+__host__ __device__ constexpr int fstride() {
+  constexpr int L = 1 << LOG, B = kFftElems / L, base = L + L / 8;
+  if (B >= 8) return base | 1;
+  constexpr int want = B == 4 ? 2 : B == 2 ? 4 : 0;
+  return base + (want - base % 8 + 8) % 8;
+}
+template <int LOG>
+constexpr size_t fsmem() {
+  static_assert(sizeof(double2) * fstride<LOG>() * (kFftElems >> LOG) <= 48 * 1024, "default shared memory");
+  return sizeof(double2) * (size_t)fstride<LOG>() * (kFftElems >> LOG);
+}
+
+// One Stockham pass of radix 2^BITS with 2^S of the length done, and the ones
+// after it.  FIRST reads its inputs with load(b, i), the last one hands its
+// outputs to store(u, b, i, value) (u: the element's number in the thread, the
+// same for every call); between passes the block's transforms live in `x`.
+// Butterflies are dealt with consecutive positions on consecutive threads, or,
+// in the first pass with BLOAD and the last with BSTORE, with consecutive
+// transforms.
+template <int LOG, int S, bool INV, bool BLOAD, bool BSTORE, class Load, class Store>
+__device__ __forceinline__ void fft_pass(double2* x, const double2* __restrict__ tw, Load&& load, Store&& store) {
+  constexpr int BITS = pass_bits(LOG - S), R = 1 << BITS, NB = kFftPer / R, L = 1 << LOG, Ns = 1 << S;
+  constexpr bool first = S == 0, last = S + BITS == LOG;
+  constexpr int per = L >> BITS, B = kFftElems >> LOG;  // butterflies per transform, transforms per block
+  constexpr bool bfast = (first && BLOAD) || (last && BSTORE && !first);
+  double2 v[kFftPer];
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const int id = threadIdx.x + kFftThreads * u;
+    const int b = bfast ? id % B : id / per, j = bfast ? id / B : id % per;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      v[u * R + r] = first ? load(b, j + r * per) : x[b * fstride<LOG>() + fpad(j + r * per)];
   }
-  const int quarter = L >> 2;
-  for (; s < logL; s += 2) {
-    const int Ns = 1 << s;
-    const int tws = logL - 2 - s;  // twiddle index of factor r = r (j mod Ns) L / (4 Ns)
-    for (int e = threadIdx.x; e < B * quarter; e += blockDim.x) {
-      const int b = e >> (logL - 2), j = e & (quarter - 1);
-      const double2* xb = x + (b << logL);
-      double2* yb = y + (b << logL);
-      const int k = j & (Ns - 1);
-      double2 w1 = tw[k << tws], w2 = tw[(2 * k) << tws], w3 = tw[(3 * k) << tws];
-      if (inv) {
-        w1.y = -w1.y;
-        w2.y = -w2.y;
-        w3.y = -w3.y;
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    double2* w = v + u * R;
+    if constexpr (!first) {
+      const int id = threadIdx.x + kFftThreads * u;
+      const int j = bfast ? id / B : id % per;
+      const int k = (j & (Ns - 1)) << (LOG - S - BITS);
+      auto twiddle = [&](int m) {
+        double2 t = __ldg(tw + m * k);
+        if (INV) t.y = -t.y;
+        return t;
+      };
+      const double2 w1 = twiddle(1);
+      w[1] = cmul(w[1], w1);
+      if constexpr (R >= 4) {
+        const double2 w2 = twiddle(2);
+        const double2 w3 = cmul(w1, w2);
+        w[2] = cmul(w[2], w2);
+        w[3] = cmul(w[3], w3);
+        if constexpr (R == 8) {
+          const double2 w4 = twiddle(4);
+          w[4] = cmul(w[4], w4);
+          w[5] = cmul(w[5], cmul(w1, w4));
+          w[6] = cmul(w[6], cmul(w2, w4));
+          w[7] = cmul(w[7], cmul(w3, w4));
+        }
       }
-      const double2 v0 = xb[j];
-      const double2 v1 = cmul(xb[j + quarter], w1);
-      const double2 v2 = cmul(xb[j + 2 * quarter], w2);
-      const double2 v3 = cmul(xb[j + 3 * quarter], w3);
-      const double2 a0 = make_double2(v0.x + v2.x, v0.y + v2.y), a1 = make_double2(v0.x - v2.x, v0.y - v2.y);
-      const double2 a2 = make_double2(v1.x + v3.x, v1.y + v3.y);
-      const double2 d = make_double2(v1.x - v3.x, v1.y - v3.y);
-      const double2 a3 = inv ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);  // (v1 - v3) * (+-i)
-      const int idx = ((j & ~(Ns - 1)) << 2) + k;
-      yb[idx] = make_double2(a0.x + a2.x, a0.y + a2.y);
-      yb[idx + Ns] = make_double2(a1.x + a3.x, a1.y + a3.y);
-      yb[idx + 2 * Ns] = make_double2(a0.x - a2.x, a0.y - a2.y);
-      yb[idx + 3 * Ns] = make_double2(a1.x - a3.x, a1.y - a3.y);
     }
-    __syncthreads();
-    double2* t = x;
-    x = y;
-    y = t;
+    if constexpr (R == 8) {
+      fft8<INV>(w);
+    } else if constexpr (R == 4) {
+      fft4<INV>(w[0], w[1], w[2], w[3]);
+    } else {
+      const double2 a = w[0];
+      w[0] = cadd(a, w[1]);
+      w[1] = csub(a, w[1]);
+    }
   }
-  return x;
+  if constexpr (!first) {
+    if constexpr (!last) __syncthreads();  // every input of the pass is in registers
+  }
+#pragma unroll
+  for (int u = 0; u < NB; ++u) {
+    const int id = threadIdx.x + kFftThreads * u;
+    const int b = bfast ? id % B : id / per, j = bfast ? id / B : id % per;
+    const int idx = ((j & ~(Ns - 1)) << BITS) + (j & (Ns - 1));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if constexpr (last)
+        store(u * R + r, b, idx + r * Ns, v[u * R + r]);
+      else
+        x[b * fstride<LOG>() + fpad(idx + r * Ns)] = v[u * R + r];
+    }
+  }
+  if constexpr (!last) {
+    __syncthreads();
+    fft_pass<LOG, S + BITS, INV, BLOAD, BSTORE>(x, tw, load, store);
+  }
+}
+
+// What bounds the stages: latency at small sizes, the 128-register blocks' two
+// per SM at large ones (DRAM at an eighth of its rate).  Before, a stage was a
+// generic radix-4 Stockham transform that crossed shared memory at every
+// radix, in natural element order (30-44 % of its wavefronts were bank
+// conflicts), with one real row per complex transform and a launch per face
+// pair.  BCpotentials in us, before and now: 24^3 117 and 30, 77^3 378 and 99,
+// 128^3 654 and 206, 256 x 128 x 128 1159 and 350, 200 x 140 x 140 2258 and 622.
+//
+// B = 2048 / L transforms of length L = 2^LOG (8 .. 2048) by the block: inputs
+// load(b, i), outputs store(u, b, i, value), natural order, no scaling.  A
+// length of up to 512 crosses shared memory at most twice.  The caller puts a
+// block barrier between two calls on the same `x`.
+template <int LOG, bool INV, bool BLOAD, bool BSTORE, class Load, class Store>
+__device__ __forceinline__ void fft_block(double2* x, const double2* __restrict__ tw, Load&& load, Store&& store) {
+  fft_pass<LOG, 0, INV, BLOAD, BSTORE>(x, tw, load, store);
 }
 
 // Geometry of one face pair: A the normal axis, P and Q the tangential axes.
@@ -110,7 +212,6 @@ struct FaceGeom {
   long long base;            // node index of interior cell (0, 0, 0)
   long long face0, face1;    // node index of face node (p, q) = (0, 0) on the two faces
   int G;                     // plane groups of the contraction
-  int B1, B2;                // rows per row CTA, columns per column CTA
 };
 
 // Distance along a circular axis of length L to offset index t (the kernel
@@ -121,222 +222,201 @@ __device__ inline int circ_off(int t, int L, int n, bool& ok) {
   return d;
 }
 
-// Stage 1: FFT along P of rows.  mode 0: the charge rows (a, q), a in
-// [a0, a0+B1), q = blockIdx.y < nQ, from C; mode 1: the kernel rows (s, tQ)
-// of slices s0 + a (a < count), tQ = blockIdx.y < LQ, from D.  Output
-// W[(a * rowsQ + q) * HP + kP], kP < HP.
-__device__ __forceinline__ void bcfft_rows_body(const FaceGeom& F, int mode, const double* __restrict__ src, int s0,
-                                                int count, const double2* __restrict__ tw, double2* __restrict__ W,
-                                                int bx, int by) {
+// Stage 1: FFT along P of rows, two real rows in one complex transform: the
+// block takes the row pairs (2 m, 2 m + 1) of plane index a for m in [bx B, bx B
+// + B).  mode 0: the charge rows (a, q), q = by < nQ, from C; mode 1: the
+// kernel rows (s, tQ) of slices s0 + a (a < count), tQ = by < LQ, from D.
+// Output W[(a * rowsQ + q) * HP + kP], kP < HP.
+template <int LOG>
+__device__ void bcfft_rows_body(const FaceGeom& F, int mode, const double* __restrict__ src, int s0, int count,
+                                const double2* __restrict__ tw, double2* __restrict__ W, int bx, int by) {
   extern __shared__ double2 smem[];
-  const int B = F.B1;
-  double2* x = smem;
-  double2* y = smem + B * F.LP;
-  const int a0 = bx * B;
+  constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int q = by;
   const int rowsQ = mode == 0 ? F.nQ : F.LQ;
   const int na = mode == 0 ? F.nA : count;
-  const bool afast = F.sA == 1 && mode == 0;
+  const int a0 = 2 * bx * B;
   bool okq = true;
   int dq = 0;
   if (mode == 1) dq = circ_off(q, F.LQ, F.nQ, okq);
-  for (int e = threadIdx.x; e < B * F.LP; e += blockDim.x) {
-    int b, p;
-    if (afast) {
-      b = e % B;
-      p = e / B;
+  auto load = [&](int b, int p) {
+    const int a = a0 + 2 * b;
+    double2 v = make_double2(0.0, 0.0);
+    if (mode == 0) {
+      if (p < F.nP && a < na) {
+        const double* c = src + (F.base + (long long)a * F.sA + (long long)p * F.sP + (long long)q * F.sQ);
+        v.x = c[0];
+        if (a + 1 < na) v.y = c[F.sA];
+      }
     } else {
-      b = e >> F.logP;
-      p = e & (F.LP - 1);
-    }
-    const int a = a0 + b;
-    double v = 0.0;
-    if (a < na) {
-      if (mode == 0) {
-        if (p < F.nP) v = src[F.base + (long long)a * F.sA + (long long)p * F.sP + (long long)q * F.sQ];
-      } else {
-        bool okp;
-        const int dp = circ_off(p, F.LP, F.nP, okp);
-        if (okp && okq) v = src[F.d0 + (long long)(s0 + a) * F.dA + (long long)dp * F.dP + (long long)dq * F.dQ];
+      bool okp;
+      const int dp = circ_off(p, L, F.nP, okp);
+      if (okp && okq && a < na) {
+        const double* d = src + (F.d0 + (long long)(s0 + a) * F.dA + (long long)dp * F.dP + (long long)dq * F.dQ);
+        v.x = d[0];
+        if (a + 1 < na) v.y = d[F.dA];
       }
     }
-    x[(b << F.logP) + p] = make_double2(v, 0.0);
-  }
+    return v;
+  };
+  // the spectrum of the pair back to shared memory: both rows need Z[k] and Z[L - k]
+  double2 z[kFftPer];
+  int zb[kFftPer], zi[kFftPer];
+  auto keep = [&](int u, int b, int i, double2 v) {
+    z[u] = v;
+    zb[u] = b;
+    zi[u] = i;
+  };
+  if (F.sA == 1 && mode == 0)
+    fft_block<LOG, false, true, false>(smem, tw, load, keep);
+  else
+    fft_block<LOG, false, false, false>(smem, tw, load, keep);
   __syncthreads();
-  const double2* X = fft_batch(x, y, F.LP, F.logP, B, tw, false);
-  for (int e = threadIdx.x; e < B * F.HP; e += blockDim.x) {
-    const int b = e / F.HP, k = e - b * F.HP;
-    const int a = a0 + b;
-    if (a < na) W[((long long)a * rowsQ + q) * F.HP + k] = X[(b << F.logP) + k];
+#pragma unroll
+  for (int u = 0; u < kFftPer; ++u) smem[zb[u] * fstride<LOG>() + fpad(zi[u])] = z[u];
+  __syncthreads();
+  constexpr int HP = L / 2 + 1;
+  for (int e = threadIdx.x; e < B * HP; e += kFftThreads) {
+    const int b = e / HP, k = e - b * HP, a = a0 + 2 * b;
+    if (a >= na) break;
+    const double2 p = smem[b * fstride<LOG>() + fpad(k)], m = smem[b * fstride<LOG>() + fpad((L - k) & (L - 1))];
+    double2* w = W + ((long long)a * rowsQ + q) * HP + k;
+    w[0] = make_double2(0.5 * (p.x + m.x), 0.5 * (p.y - m.y));
+    if (a + 1 < na) w[(long long)rowsQ * HP] = make_double2(0.5 * (p.y + m.y), 0.5 * (m.x - p.x));
   }
 }
 
-// Stage 2: FFT along Q of the columns kP in [k0, k0+B2).
-// mode 0 (contraction): planes a of group blockIdx.y; each thread keeps the
-// sums of its (kP, kQ) elements against Dh[s0(a)] and Dh[s1(a)] and writes the
-// group's partial to S[(g * 2 + f) * HP * LQ + kP * LQ + kQ].
-// mode 1 (kernel transforms): slices a < count of W, real part times scale
-// to Dh[(s0 + a) * HP * LQ + kP * LQ + kQ].
-__device__ __forceinline__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* __restrict__ W, int s0,
-                                                int count, double scale, const double2* __restrict__ tw,
-                                                double* __restrict__ Dh, double2* __restrict__ S, int bx, int by) {
+// Plane t of the contraction's order: 0, nA - 1, 1, nA - 2, ... so that the
+// slices of D that a plane reads for its two faces serve the next one too.
+__device__ __forceinline__ int plane_at(int t, int nA) { return t & 1 ? nA - 1 - (t >> 1) : t >> 1; }
+
+// Stage 2: FFT along Q of the columns kP in [bx B, bx B + B).
+// mode 0 (contraction): the planes of group by; each thread keeps the sums of
+// its (kP, kQ) elements against Dh[s0(a)] and Dh[s1(a)] and writes the group's
+// partial to S[(g * 2 + f) * HP * LQ + kP * LQ + kQ].
+// mode 1 (kernel transforms): slice by < count of W, real part times scale to
+// Dh[(s0 + by) * HP * LQ + kP * LQ + kQ].
+template <int LOG>
+__device__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* __restrict__ W, int s0, int count,
+                                double scale, const double2* __restrict__ tw, double* __restrict__ Dh,
+                                double2* __restrict__ S, int bx, int by) {
   extern __shared__ double2 smem[];
-  const int B = F.B2;
-  double2* x = smem;
-  double2* y = smem + B * F.LQ;
+  constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int k0 = bx * B;
-  const int rowsQ = mode == 0 ? F.nQ : F.LQ;
-  const long long plane = (long long)F.HP * F.LQ;
-  int a_lo, a_hi;
-  if (mode == 0) {
-    const int per = (F.nA + F.G - 1) / F.G;
-    a_lo = by * per;
-    a_hi = min(F.nA, a_lo + per);
-  } else {
-    a_lo = by;
-    a_hi = min(count, a_lo + 1);
-  }
-  double2 acc0[kColElems / kFftThreads], acc1[kColElems / kFftThreads];
+  const int rowsQ = mode == 0 ? F.nQ : L;
+  const long long plane = (long long)F.HP * L;
+  const int per = (F.nA + F.G - 1) / F.G;
+  const int t_lo = mode == 0 ? by * per : by, t_hi = mode == 0 ? min(F.nA, t_lo + per) : min(count, t_lo + 1);
+  double2 acc0[kFftPer], acc1[kFftPer];
 #pragma unroll
-  for (int u = 0; u < kColElems / kFftThreads; ++u) acc0[u] = acc1[u] = make_double2(0.0, 0.0);
-  for (int a = a_lo; a < a_hi; ++a) {
-    for (int e = threadIdx.x; e < B * F.LQ; e += blockDim.x) {
-      const int q = e / B, b = e - q * B;  // kP fastest: contiguous in W
-      const int k = k0 + b;
-      double2 v = make_double2(0.0, 0.0);
-      if (k < F.HP && q < rowsQ) v = W[((long long)a * rowsQ + q) * F.HP + k];
-      x[(b << F.logQ) + q] = v;
+  for (int u = 0; u < kFftPer; ++u) acc0[u] = acc1[u] = make_double2(0.0, 0.0);
+  for (int t = t_lo; t < t_hi; ++t) {
+    const int a = mode == 0 ? plane_at(t, F.nA) : t;
+    const double2* w = W + (long long)a * rowsQ * F.HP + k0;
+    auto load = [&](int b, int q) {
+      return k0 + b < F.HP && q < rowsQ ? __ldg(w + (long long)q * F.HP + b) : make_double2(0.0, 0.0);
+    };
+    if (t > t_lo) __syncthreads();  // the plane before has read its last shared element
+    if (mode == 0) {
+      const double* d0 = Dh + (long long)a * plane + (long long)k0 * L;                // s = a + 1
+      const double* d1 = Dh + (long long)(F.nA - 1 - a) * plane + (long long)k0 * L;   // s = nA - a
+      fft_block<LOG, false, true, false>(smem, tw, load, [&](int u, int b, int kq, double2 v) {
+        if (k0 + b < F.HP) {
+          const double e0 = __ldg(d0 + b * L + kq), e1 = __ldg(d1 + b * L + kq);
+          acc0[u].x = fma(v.x, e0, acc0[u].x);
+          acc0[u].y = fma(v.y, e0, acc0[u].y);
+          acc1[u].x = fma(v.x, e1, acc1[u].x);
+          acc1[u].y = fma(v.y, e1, acc1[u].y);
+        }
+      });
+    } else {
+      double* d = Dh + (long long)(s0 + a) * plane + (long long)k0 * L;
+      fft_block<LOG, false, true, false>(smem, tw, load, [&](int, int b, int kq, double2 v) {
+        if (k0 + b < F.HP) d[b * L + kq] = v.x * scale;
+      });
     }
-    __syncthreads();
-    const double2* X = fft_batch(x, y, F.LQ, F.logQ, B, tw, false);
-#pragma unroll
-    for (int u = 0; u < kColElems / kFftThreads; ++u) {
-      const int e = threadIdx.x + u * kFftThreads;  // B * LQ == kColElems
-      const int b = e >> F.logQ, kq = e & (F.LQ - 1);
-      const int k = k0 + b;
-      if (k >= F.HP) continue;
-      const double2 v = X[e];
-      if (mode == 0) {
-        const double d0 = Dh[(long long)a * plane + (long long)k * F.LQ + kq];                   // s = a + 1
-        const double d1 = Dh[(long long)(F.nA - 1 - a) * plane + (long long)k * F.LQ + kq];      // s = nA - a
-        acc0[u].x = fma(v.x, d0, acc0[u].x);
-        acc0[u].y = fma(v.y, d0, acc0[u].y);
-        acc1[u].x = fma(v.x, d1, acc1[u].x);
-        acc1[u].y = fma(v.y, d1, acc1[u].y);
-      } else {
-        Dh[(long long)(s0 + a) * plane + (long long)k * F.LQ + kq] = v.x * scale;
-      }
-    }
-    __syncthreads();
   }
   if (mode != 0) return;
+  // the elements of the last pass, in its order
+  constexpr int BITS = last_bits(LOG), R = 1 << BITS, lastper = L >> BITS;
 #pragma unroll
-  for (int u = 0; u < kColElems / kFftThreads; ++u) {
-    const int e = threadIdx.x + u * kFftThreads;
-    const int b = e >> F.logQ, kq = e & (F.LQ - 1);
-    const int k = k0 + b;
-    if (k >= F.HP) continue;
-    S[((long long)by * 2 + 0) * plane + (long long)k * F.LQ + kq] = acc0[u];
-    S[((long long)by * 2 + 1) * plane + (long long)k * F.LQ + kq] = acc1[u];
+  for (int u = 0; u < kFftPer; ++u) {
+    const int id = threadIdx.x + kFftThreads * (u / R), b = id / lastper, kq = id % lastper + (u % R) * lastper;
+    if (k0 + b < F.HP) {
+      const long long e = (long long)(k0 + b) * L + kq;
+      S[((long long)by * 2 + 0) * plane + e] = acc0[u];
+      S[((long long)by * 2 + 1) * plane + e] = acc1[u];
+    }
   }
 }
 
 // Stage 3a: sum of the group partials (fixed order) and the inverse FFT along
-// Q of columns kP in [k0, k0+B2) of face f = blockIdx.y; V[(f*nQ + q)*HP + kP]
-// for q < nQ.
-__device__ __forceinline__ void bcfft_invq_body(const FaceGeom& F, const double2* __restrict__ S,
-                                                const double2* __restrict__ tw, double2* __restrict__ V, int bx,
-                                                int by) {
+// Q of columns kP in [bx B, bx B + B) of face f = by; V[(f*nQ + q)*HP + kP] for
+// q < nQ.
+template <int LOG>
+__device__ void bcfft_invq_body(const FaceGeom& F, const double2* __restrict__ S, const double2* __restrict__ tw,
+                                double2* __restrict__ V, int bx, int by) {
   extern __shared__ double2 smem[];
-  const int B = F.B2;
-  double2* x = smem;
-  double2* y = smem + B * F.LQ;
+  constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int k0 = bx * B, f = by;
-  const long long plane = (long long)F.HP * F.LQ;
-  for (int e = threadIdx.x; e < B * F.LQ; e += blockDim.x) {
-    const int b = e >> F.logQ, kq = e & (F.LQ - 1);
-    const int k = k0 + b;
-    double2 v = make_double2(0.0, 0.0);
-    if (k < F.HP)
-      for (int g = 0; g < F.G; ++g) {
-        const double2 s = S[((long long)g * 2 + f) * plane + (long long)k * F.LQ + kq];
-        v.x += s.x;
-        v.y += s.y;
-      }
-    x[e] = v;
-  }
-  __syncthreads();
-  const double2* X = fft_batch(x, y, F.LQ, F.logQ, B, tw, true);
-  for (int e = threadIdx.x; e < B * F.nQ; e += blockDim.x) {
-    const int q = e / B, b = e - q * B;
-    const int k = k0 + b;
-    if (k < F.HP) V[((long long)f * F.nQ + q) * F.HP + k] = X[(b << F.logQ) + q];
-  }
+  const long long plane = (long long)F.HP * L;
+  fft_block<LOG, true, false, true>(
+      smem, tw,
+      [&](int b, int kq) {
+        double2 v = make_double2(0.0, 0.0);
+        if (k0 + b < F.HP) {
+          const double2* s = S + (long long)f * plane + (long long)(k0 + b) * L + kq;
+#pragma unroll 4
+          for (int g = 0; g < F.G; ++g) {
+            const double2 e = __ldg(s + (long long)g * 2 * plane);
+            v.x += e.x;
+            v.y += e.y;
+          }
+        }
+        return v;
+      },
+      [&](int, int b, int q, double2 v) {
+        if (k0 + b < F.HP && q < F.nQ) V[((long long)f * F.nQ + q) * F.HP + k0 + b] = v;
+      });
 }
 
-// Stage 3b: inverse real FFT along P of rows q in [q0, q0+B1) of face f =
-// blockIdx.y (the spectrum's upper half from Hermitian symmetry); the real
-// parts p < nP are the face potential.
-__device__ __forceinline__ void bcfft_invp_body(const FaceGeom& F, const double2* __restrict__ V,
-                                                const double2* __restrict__ tw, double* __restrict__ U, int bx,
-                                                int by) {
+// Stage 3b: inverse real FFT along P of the row pairs (2 m, 2 m + 1) of face f =
+// by, m in [bx B, bx B + B) (the spectrum's upper half from Hermitian
+// symmetry): two real rows as the real and imaginary part of one transform.
+template <int LOG>
+__device__ void bcfft_invp_body(const FaceGeom& F, const double2* __restrict__ V, const double2* __restrict__ tw,
+                                double* __restrict__ U, int bx, int by) {
   extern __shared__ double2 smem[];
-  const int B = F.B1;
-  double2* x = smem;
-  double2* y = smem + B * F.LP;
-  const int q0 = bx * B, f = by;
-  for (int e = threadIdx.x; e < B * F.LP; e += blockDim.x) {
-    const int b = e >> F.logP, k = e & (F.LP - 1);
-    const int q = q0 + b;
-    double2 v = make_double2(0.0, 0.0);
-    if (q < F.nQ) {
-      if (k < F.HP) {
-        v = V[((long long)f * F.nQ + q) * F.HP + k];
-      } else {
-        v = V[((long long)f * F.nQ + q) * F.HP + (F.LP - k)];
-        v.y = -v.y;
-      }
-    }
-    x[e] = v;
-  }
-  __syncthreads();
-  const double2* X = fft_batch(x, y, F.LP, F.logP, B, tw, true);
+  constexpr int L = 1 << LOG, B = kFftElems >> LOG, HP = L / 2 + 1;
+  const int q0 = 2 * bx * B, f = by;
   const long long face = f == 0 ? F.face0 : F.face1;
-  for (int e = threadIdx.x; e < B * F.nP; e += blockDim.x) {
-    const int b = e / F.nP, p = e - b * F.nP;
-    const int q = q0 + b;
-    if (q < F.nQ) U[face + (long long)p * F.sP + (long long)q * F.sQ] = X[(b << F.logP) + p].x;
-  }
+  fft_block<LOG, true, false, false>(
+      smem, tw,
+      [&](int b, int k) {
+        const int q = q0 + 2 * b;
+        double2 z = make_double2(0.0, 0.0);
+        if (q < F.nQ) {
+          const bool up = k >= HP;
+          const double2* r = V + ((long long)f * F.nQ + q) * HP + (up ? L - k : k);
+          double2 v = __ldg(r), w = q + 1 < F.nQ ? __ldg(r + HP) : make_double2(0.0, 0.0);
+          if (up) v.y = -v.y, w.y = -w.y;
+          z = make_double2(v.x - w.y, v.y + w.x);  // v + i w
+        }
+        return z;
+      },
+      [&](int, int b, int p, double2 v) {
+        const int q = q0 + 2 * b;
+        if (p < F.nP && q < F.nQ) {
+          double* u = U + (face + (long long)p * F.sP + (long long)q * F.sQ);
+          u[0] = v.x;
+          if (q + 1 < F.nQ) u[F.sQ] = v.y;
+        }
+      });
 }
 
-__global__ void __launch_bounds__(kFftThreads) bcfft_rows_kernel(FaceGeom F, int mode, const double* __restrict__ src,
-                                                                 int s0, int count, const double2* __restrict__ tw,
-                                                                 double2* __restrict__ W) {
-  bcfft_rows_body(F, mode, src, s0, count, tw, W, blockIdx.x, blockIdx.y);
-}
-
-__global__ void __launch_bounds__(kFftThreads) bcfft_cols_kernel(FaceGeom F, int mode, const double2* __restrict__ W,
-                                                                 int s0, int count, double scale,
-                                                                 const double2* __restrict__ tw,
-                                                                 double* __restrict__ Dh, double2* __restrict__ S) {
-  bcfft_cols_body(F, mode, W, s0, count, scale, tw, Dh, S, blockIdx.x, blockIdx.y);
-}
-
-__global__ void __launch_bounds__(kFftThreads) bcfft_invq_kernel(FaceGeom F, const double2* __restrict__ S,
-                                                                 const double2* __restrict__ tw,
-                                                                 double2* __restrict__ V) {
-  bcfft_invq_body(F, S, tw, V, blockIdx.x, blockIdx.y);
-}
-
-__global__ void __launch_bounds__(kFftThreads) bcfft_invp_kernel(FaceGeom F, const double2* __restrict__ V,
-                                                                 const double2* __restrict__ tw,
-                                                                 double* __restrict__ U) {
-  bcfft_invp_body(F, V, tw, U, blockIdx.x, blockIdx.y);
-}
-
-// One face pair of one run in a batched launch: its geometry and buffers,
-// and per stage (rows, columns + contraction, inverse along Q, inverse along
-// P) the first block of its blocks in the launch and its blocks along x.
+// One face pair in a launch: its geometry and buffers, and per stage (rows,
+// columns + contraction, inverse along Q, inverse along P) the first block of
+// its blocks in the launch and its blocks along x.
 struct FftJob {
   FaceGeom F;
   const double* C;
@@ -351,26 +431,79 @@ struct FftJob {
   int bx[4];
 };
 
-// One stage for every face pair of every run of a batch in one launch: block
-// b belongs to the job with the largest start <= b (binary search), and runs
-// that job's block (local % bx, local / bx) of the stage.
-__global__ void __launch_bounds__(kFftThreads) bcfft_batch_kernel(const FftJob* __restrict__ jobs, int njobs,
-                                                                  int stage) {
+template <int STAGE, int LOG>
+__device__ __forceinline__ void bcfft_stage(const FftJob& J, int bx, int by) {
+  const FaceGeom F = J.F;
+  if constexpr (STAGE == 0) bcfft_rows_body<LOG>(F, 0, J.C, 0, F.nA, J.twP, J.W, bx, by);
+  else if constexpr (STAGE == 1) bcfft_cols_body<LOG>(F, 0, J.W, 0, 0, 0.0, J.twQ, J.Dh, J.S, bx, by);
+  else if constexpr (STAGE == 2) bcfft_invq_body<LOG>(F, J.S, J.twQ, J.V, bx, by);
+  else bcfft_invp_body<LOG>(F, J.V, J.twP, J.U, bx, by);
+}
+
+// The blocks of one face pair in a stage of a batched launch.
+struct FftSeg {
+  long long start;  // its first block
+  int job, bx;
+};
+
+// One stage of length 2^LOG for a table of face pairs in one launch: block b
+// belongs to the segment with the largest start <= b (binary search), and runs
+// block (local % bx, local / bx) of that job's stage.
+template <int STAGE, int LOG>
+__global__ void __launch_bounds__(kFftThreads, 2) bcfft_table_kernel(const FftJob* __restrict__ jobs,
+                                                                     const FftSeg* __restrict__ segs, int n) {
   const long long b = blockIdx.x;
-  int lo = 0, hi = njobs - 1;
+  int lo = 0, hi = n - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (jobs[mid].start[stage] <= b) lo = mid;
+    if (segs[mid].start <= b) lo = mid;
     else hi = mid - 1;
   }
-  const FftJob& J = jobs[lo];
-  const FaceGeom F = J.F;
-  const long long local = b - J.start[stage];
-  const int bx = int(local % J.bx[stage]), by = int(local / J.bx[stage]);
-  if (stage == 0) bcfft_rows_body(F, 0, J.C, 0, F.nA, J.twP, J.W, bx, by);
-  else if (stage == 1) bcfft_cols_body(F, 0, J.W, 0, 0, 0.0, J.twQ, J.Dh, J.S, bx, by);
-  else if (stage == 2) bcfft_invq_body(F, J.S, J.twQ, J.V, bx, by);
-  else bcfft_invp_body(F, J.V, J.twP, J.U, bx, by);
+  const FftSeg g = segs[lo];
+  const long long local = b - g.start;
+  bcfft_stage<STAGE, LOG>(jobs[g.job], int(local % g.bx), int(local / g.bx));
+}
+
+// The same for up to three face pairs of one run, the table in the parameters.
+struct FftJobs3 {
+  FftJob j[3];
+  int n;
+};
+template <int STAGE, int LOG>
+__global__ void __launch_bounds__(kFftThreads, 2) bcfft_run_kernel(const __grid_constant__ FftJobs3 T) {
+  const long long b = blockIdx.x;
+  int q = 0;
+  while (q + 1 < T.n && T.j[q + 1].start[STAGE] <= b) ++q;
+  const FftJob& J = T.j[q];
+  const long long local = b - J.start[STAGE];
+  bcfft_stage<STAGE, LOG>(J, int(local % J.bx[STAGE]), int(local / J.bx[STAGE]));
+}
+
+// Slice transforms (mode 1 of the row and column stages).
+template <int LOG>
+__global__ void __launch_bounds__(kFftThreads, 2) bcfft_slice_rows_kernel(FaceGeom F, const double* __restrict__ D,
+                                                                          int s0, int count,
+                                                                          const double2* __restrict__ tw,
+                                                                          double2* __restrict__ W) {
+  bcfft_rows_body<LOG>(F, 1, D, s0, count, tw, W, blockIdx.x, blockIdx.y);
+}
+template <int LOG>
+__global__ void __launch_bounds__(kFftThreads, 2) bcfft_slice_cols_kernel(FaceGeom F, const double2* __restrict__ W,
+                                                                          int s0, int count, double scale,
+                                                                          const double2* __restrict__ tw,
+                                                                          double* __restrict__ Dh) {
+  bcfft_cols_body<LOG>(F, 1, W, s0, count, scale, tw, Dh, nullptr, blockIdx.x, blockIdx.y);
+}
+
+// f(std::integral_constant<int, log>) for the run-time length 2^log.
+template <int LOG = kMinLog, class Fn>
+int with_log(int log, Fn&& f) {
+  if constexpr (LOG <= kMaxLog) {
+    if (log == LOG) return f(std::integral_constant<int, LOG>());
+    return with_log<LOG + 1>(log, f);
+  } else {
+    return fail(PICARD_ERR_BAD_ARG, "FFT BCpotentials: unsupported transform length");
+  }
 }
 
 int pow2_at_least(int v) {
@@ -384,6 +517,20 @@ int ilog2(int L) {
   return l;
 }
 
+int col_blocks(const FaceGeom& F) { return (F.HP + (kFftElems >> F.logQ) - 1) / (kFftElems >> F.logQ); }
+// blocks of row pairs
+int pair_blocks(const FaceGeom& F, int rows) { return (rows + 2 * (kFftElems >> F.logP) - 1) / (2 * (kFftElems >> F.logP)); }
+
+// Whether the face pairs go through the row and contraction stages together:
+// while their row transforms fit the L2 cache with room to spare.  Else one
+// after another, so that each contraction finds its own row transforms in L2.
+bool faces_together(const KParams& K) {
+  auto half = [](int n) { return pow2_at_least(2 * n - 1) / 2 + 1LL; };
+  const long long elems = (long long)K.nx * K.nz * half(K.ny) + (long long)K.ny * K.nz * half(K.nx) +
+                          (long long)K.nz * K.ny * half(K.nx);
+  return 16 * elems <= (64LL << 20);
+}
+
 FaceGeom face_geom(const KParams& K, int axis) {
   const int n[3] = {K.nx, K.ny, K.nz};
   const long long s[3] = {1, K.nxp, (long long)K.nxp * K.nyp};
@@ -394,8 +541,8 @@ FaceGeom face_geom(const KParams& K, int axis) {
   F.nA = n[axis];
   F.nP = n[P];
   F.nQ = n[Q];
-  F.LP = pow2_at_least(2 * F.nP - 1);
-  F.LQ = pow2_at_least(2 * F.nQ - 1);
+  F.LP = std::max(1 << kMinLog, pow2_at_least(2 * F.nP - 1));
+  F.LQ = std::max(1 << kMinLog, pow2_at_least(2 * F.nQ - 1));
   F.logP = ilog2(F.LP);
   F.logQ = ilog2(F.LQ);
   F.HP = F.LP / 2 + 1;
@@ -409,14 +556,15 @@ FaceGeom face_geom(const KParams& K, int axis) {
   F.base = 1 + K.nxp * (1 + (long long)K.nyp * 1);
   F.face0 = F.base - F.sA;                       // plane 0 along A, tangential (1, 1)
   F.face1 = F.base + (long long)F.nA * F.sA;     // plane nA + 1
-  F.B1 = std::max(1, std::min(16, kRowElems / F.LP));
-  F.B2 = std::max(1, kColElems / F.LQ);  // B2 * LQ == kColElems (LQ a power of two <= kColElems)
-  const int colblocks = (F.HP + F.B2 - 1) / F.B2;
-  F.G = std::max(1, std::min(F.nA, (4 * 148 + colblocks - 1) / colblocks));
+  // plane groups of the contraction: two blocks per SM, counting the other face
+  // pairs of a launch; on small grids no more than eight partials, which the
+  // inverse along Q sums before it starts
+  const int share = col_blocks(F) * (faces_together(K) ? 3 : 1);
+  F.G = std::max(1, std::min(std::min(F.nA, F.nA <= 64 ? 8 : 32), 2 * 148 / share));
   return F;
 }
 
-bool fits(const FaceGeom& F) { return F.LP <= kRowElems && F.LQ <= kColElems; }
+bool fits(const FaceGeom& F) { return F.LP <= kMaxP && F.LQ <= kMaxQ; }
 
 }  // namespace
 
@@ -469,9 +617,6 @@ void twiddles(int L, std::vector<double2>& t) {
   }
 }
 
-size_t smem_rows(const FaceGeom& F) { return sizeof(double2) * 2 * (size_t)F.B1 * F.LP; }
-size_t smem_cols(const FaceGeom& F) { return sizeof(double2) * 2 * (size_t)F.B2 * F.LQ; }
-
 }  // namespace
 
 struct BcFft {
@@ -479,23 +624,9 @@ struct BcFft {
   bool ready = false;  // slice transforms of the current D
 };
 
-static int set_smem_limits() {
-  static bool done = false;
-  if (done) return PICARD_OK;
-  const int big = 2 * 16 * kRowElems;  // 64 KB
-  PICARD_CUDA(cudaFuncSetAttribute(bcfft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  PICARD_CUDA(cudaFuncSetAttribute(bcfft_cols_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  PICARD_CUDA(cudaFuncSetAttribute(bcfft_invq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  PICARD_CUDA(cudaFuncSetAttribute(bcfft_invp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  PICARD_CUDA(cudaFuncSetAttribute(bcfft_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-  done = true;
-  return PICARD_OK;
-}
-
 int bcpot_fft_alloc(picard_ctx* c) {
   if (c->bcfft) return PICARD_OK;
   if (!bcpot_fft_supported(c->K)) return fail(PICARD_ERR_BAD_ARG, "FFT BCpotentials: a face is longer than 1024 cells");
-  PICARD_TRY(set_smem_limits());
   BcFft* B = new BcFft();
   c->bcfft = B;
   const KParams& K = c->K;
@@ -556,59 +687,135 @@ static int prepare(picard_ctx* c) {
     const int chunk = int(std::max<long long>(1, A.w_elems / ((long long)F.LQ * F.HP)));
     for (int s0 = 0; s0 < F.nA; s0 += chunk) {
       const int cnt = std::min(chunk, F.nA - s0);
-      dim3 g1((cnt + F.B1 - 1) / F.B1, F.LQ);
       note_launch();
       // slice index a <-> normal offset s0 + a + 1 (the D table at offset a + 1 along A)
-      bcfft_rows_kernel<<<g1, kFftThreads, smem_rows(F), c->st>>>(F, 1, c->D + F.dA, s0, cnt, A.twP, A.W);
-      PICARD_CUDA(cudaGetLastError());
-      dim3 g2((F.HP + F.B2 - 1) / F.B2, cnt);
+      PICARD_TRY(with_log(F.logP, [&](auto lg) {
+        constexpr int LOG = decltype(lg)::value;
+        bcfft_slice_rows_kernel<LOG><<<dim3(pair_blocks(F, cnt), F.LQ), kFftThreads, fsmem<LOG>(), c->st>>>(
+            F, c->D + F.dA, s0, cnt, A.twP, A.W);
+        return check_cuda(cudaGetLastError(), "bcfft_slice_rows_kernel");
+      }));
       note_launch();
-      bcfft_cols_kernel<<<g2, kFftThreads, smem_cols(F), c->st>>>(F, 1, A.W, s0, cnt, scale, A.twQ, A.Dh, nullptr);
-      PICARD_CUDA(cudaGetLastError());
+      PICARD_TRY(with_log(F.logQ, [&](auto lg) {
+        constexpr int LOG = decltype(lg)::value;
+        bcfft_slice_cols_kernel<LOG><<<dim3(col_blocks(F), cnt), kFftThreads, fsmem<LOG>(), c->st>>>(
+            F, A.W, s0, cnt, scale, A.twQ, A.Dh);
+        return check_cuda(cudaGetLastError(), "bcfft_slice_cols_kernel");
+      }));
     }
   }
   B->ready = true;
   return PICARD_OK;
 }
 
+namespace {
+
+FftJob make_job(picard_ctx* c, const AxisPlan& A) {
+  FftJob J;
+  J.F = A.F;
+  J.C = c->C;
+  J.W = A.W;
+  J.twP = A.twP;
+  J.twQ = A.twQ;
+  J.Dh = A.Dh;
+  J.S = A.S;
+  J.V = A.V;
+  J.U = c->U;
+  const FaceGeom& F = A.F;
+  J.bx[0] = pair_blocks(F, F.nA);
+  J.bx[1] = J.bx[2] = col_blocks(F);
+  J.bx[3] = pair_blocks(F, F.nQ);
+  return J;
+}
+int stage_rows(const FaceGeom& F, int stage) { return stage == 0 ? F.nQ : stage == 1 ? F.G : 2; }
+int stage_log(const FaceGeom& F, int stage) { return stage == 0 || stage == 3 ? F.logP : F.logQ; }
+
+template <int STAGE>
+int launch_run_stage(FftJobs3& T, int log, long long blocks, cudaStream_t st) {
+  note_launch();
+  return with_log(log, [&](auto lg) {
+    constexpr int LOG = decltype(lg)::value;
+    bcfft_run_kernel<STAGE, LOG><<<(unsigned)blocks, kFftThreads, fsmem<LOG>(), st>>>(T);
+    return check_cuda(cudaGetLastError(), "bcfft_run_kernel");
+  });
+}
+// Stages [STAGE, END) of jobs [first, last) of `J`, one launch per stage and
+// transform length.
+template <int STAGE, int END>
+int run_stages(const std::vector<FftJob>& J, size_t first, size_t last, cudaStream_t st) {
+  if constexpr (STAGE < END) {
+    for (int log = kMinLog; log <= kMaxLog; ++log) {
+      FftJobs3 T;
+      T.n = 0;
+      long long blocks = 0;
+      for (size_t q = first; q < last; ++q) {
+        const FftJob& j = J[q];
+        if (stage_log(j.F, STAGE) != log) continue;
+        T.j[T.n] = j;
+        T.j[T.n].start[STAGE] = blocks;
+        blocks += (long long)j.bx[STAGE] * stage_rows(j.F, STAGE);
+        ++T.n;
+      }
+      if (T.n) PICARD_TRY(launch_run_stage<STAGE>(T, log, blocks, st));
+    }
+    return run_stages<STAGE + 1, END>(J, first, last, st);
+  }
+  return PICARD_OK;
+}
+
+}  // namespace
+
 int bc_potentials_fft(picard_ctx* c) {
   PICARD_TRY(bcpot_fft_alloc(c));
   BcFft* B = c->bcfft;
   if (!B->ready) PICARD_TRY(prepare(c));
   PICARD_CUDA(cudaMemsetAsync(c->U, 0, sizeof(double) * c->K.nodes, c->st));  // BCpotentials.f90:36
-  for (int a = 0; a < 3; ++a) {
-    AxisPlan& A = B->ax[a];
-    if (!A.Dh) continue;
-    const FaceGeom& F = A.F;
-    dim3 g1((F.nA + F.B1 - 1) / F.B1, F.nQ);
-    note_launch();
-    bcfft_rows_kernel<<<g1, kFftThreads, smem_rows(F), c->st>>>(F, 0, c->C, 0, F.nA, A.twP, A.W);
-    PICARD_CUDA(cudaGetLastError());
-    dim3 g2((F.HP + F.B2 - 1) / F.B2, F.G);
-    note_launch();
-    bcfft_cols_kernel<<<g2, kFftThreads, smem_cols(F), c->st>>>(F, 0, A.W, 0, 0, 0.0, A.twQ, A.Dh, A.S);
-    PICARD_CUDA(cudaGetLastError());
-    dim3 g3((F.HP + F.B2 - 1) / F.B2, 2);
-    note_launch();
-    bcfft_invq_kernel<<<g3, kFftThreads, smem_cols(F), c->st>>>(F, A.S, A.twQ, A.V);
-    PICARD_CUDA(cudaGetLastError());
-    dim3 g4((F.nQ + F.B1 - 1) / F.B1, 2);
-    note_launch();
-    bcfft_invp_kernel<<<g4, kFftThreads, smem_rows(F), c->st>>>(F, A.V, A.twP, c->U);
-    PICARD_CUDA(cudaGetLastError());
+  std::vector<FftJob> jobs;
+  for (int a = 0; a < 3; ++a)
+    if (B->ax[a].Dh) jobs.push_back(make_job(c, B->ax[a]));
+  const size_t n = jobs.size(), step = faces_together(c->K) ? 3 : 1;
+  for (size_t q = 0; q < n; q += step) PICARD_TRY((run_stages<0, 2>(jobs, q, std::min(n, q + step), c->st)));
+  PICARD_TRY((run_stages<2, 4>(jobs, 0, n, c->st)));
+  return PICARD_OK;
+}
+
+namespace {
+
+// The stages of a whole batch, one launch per stage and transform length that
+// occurs; segs[stage][log]: [first, last) of its segments in the table.
+struct SegRange {
+  int first = 0, count = 0;
+  long long blocks = 0;
+};
+template <int STAGE = 0>
+int table_stages(const FftJob* jobs, const FftSeg* segs, const SegRange (*range)[kMaxLog + 1], cudaStream_t st) {
+  if constexpr (STAGE < 4) {
+    for (int log = kMinLog; log <= kMaxLog; ++log) {
+      const SegRange& r = range[STAGE][log];
+      if (!r.count) continue;
+      note_launch();
+      PICARD_TRY(with_log(log, [&](auto lg) {
+        constexpr int LOG = decltype(lg)::value;
+        bcfft_table_kernel<STAGE, LOG><<<(unsigned)r.blocks, kFftThreads, fsmem<LOG>(), st>>>(jobs, segs + r.first,
+                                                                                              r.count);
+        return check_cuda(cudaGetLastError(), "bcfft_table_kernel");
+      }));
+    }
+    return table_stages<STAGE + 1>(jobs, segs, range, st);
   }
   return PICARD_OK;
 }
 
+}  // namespace
+
 // BCpotentials of many runs: the FFT runs' face pairs advance stage by stage,
-// each stage one launch over all of them on the batch stream (after every
-// such run's U is zeroed and its slice transforms exist, on its own stream);
-// the other runs take their own method on their own streams.
+// each stage one launch per transform length over all of them on the batch
+// stream (after every such run's U is zeroed and its slice transforms exist,
+// on its own stream); the other runs take their own method on their own
+// streams.
 int bc_potentials_batch(picard_ctx** ctxs, int n, cudaStream_t bst, cudaEvent_t* rev, cudaEvent_t bev) {
   std::vector<FftJob> jobs;
   std::vector<int> fft_runs;
-  long long total[4] = {0, 0, 0, 0};
-  size_t smem[4] = {0, 0, 0, 0};
   for (int r = 0; r < n; ++r) {
     picard_ctx* c = ctxs[r];
     if (c->bcpot_tensor != PICARD_BCPOT_FFT) {
@@ -622,44 +829,33 @@ int bc_potentials_batch(picard_ctx** ctxs, int n, cudaStream_t bst, cudaEvent_t*
     PICARD_CUDA(cudaEventRecord(rev[r], c->st));
     PICARD_CUDA(cudaStreamWaitEvent(bst, rev[r], 0));
     fft_runs.push_back(r);
-    for (int a = 0; a < 3; ++a) {
-      AxisPlan& A = B->ax[a];
-      if (!A.Dh) continue;
-      FftJob J;
-      J.F = A.F;
-      J.C = c->C;
-      J.W = A.W;
-      J.twP = A.twP;
-      J.twQ = A.twQ;
-      J.Dh = A.Dh;
-      J.S = A.S;
-      J.V = A.V;
-      J.U = c->U;
-      const FaceGeom& F = A.F;
-      const int bxs[4] = {(F.nA + F.B1 - 1) / F.B1, (F.HP + F.B2 - 1) / F.B2, (F.HP + F.B2 - 1) / F.B2,
-                          (F.nQ + F.B1 - 1) / F.B1};
-      const int bys[4] = {F.nQ, F.G, 2, 2};
-      const size_t sm[4] = {smem_rows(F), smem_cols(F), smem_cols(F), smem_rows(F)};
-      for (int t = 0; t < 4; ++t) {
-        J.start[t] = total[t];
-        J.bx[t] = bxs[t];
-        total[t] += (long long)bxs[t] * bys[t];
-        smem[t] = std::max(smem[t], sm[t]);
-      }
-      jobs.push_back(J);
-    }
+    for (int a = 0; a < 3; ++a)
+      if (B->ax[a].Dh) jobs.push_back(make_job(c, B->ax[a]));
   }
   if (jobs.empty()) return PICARD_OK;
-  // the job table lives on the batch stream until its last launch
+  std::vector<FftSeg> segs;
+  SegRange range[4][kMaxLog + 1];
+  for (int stage = 0; stage < 4; ++stage)
+    for (int log = kMinLog; log <= kMaxLog; ++log) {
+      SegRange& r = range[stage][log];
+      r.first = (int)segs.size();
+      for (size_t q = 0; q < jobs.size(); ++q) {
+        if (stage_log(jobs[q].F, stage) != log) continue;
+        segs.push_back(FftSeg{r.blocks, (int)q, jobs[q].bx[stage]});
+        r.blocks += (long long)jobs[q].bx[stage] * stage_rows(jobs[q].F, stage);
+      }
+      r.count = (int)segs.size() - r.first;
+    }
+  // the table lives on the batch stream until its last launch
+  const size_t jb = sizeof(FftJob) * jobs.size(), sb = sizeof(FftSeg) * segs.size();
+  std::vector<unsigned char> table(jb + sb);
+  std::memcpy(table.data(), jobs.data(), jb);
+  std::memcpy(table.data() + jb, segs.data(), sb);
   void* dj = nullptr;
-  PICARD_CUDA(cudaMallocAsync(&dj, sizeof(FftJob) * jobs.size(), bst));
-  PICARD_CUDA(cudaMemcpyAsync(dj, jobs.data(), sizeof(FftJob) * jobs.size(), cudaMemcpyHostToDevice, bst));
-  for (int t = 0; t < 4; ++t) {
-    note_launch();
-    bcfft_batch_kernel<<<(unsigned)total[t], kFftThreads, smem[t], bst>>>(static_cast<const FftJob*>(dj),
-                                                                            (int)jobs.size(), t);
-    PICARD_CUDA(cudaGetLastError());
-  }
+  PICARD_CUDA(cudaMallocAsync(&dj, table.size(), bst));
+  PICARD_CUDA(cudaMemcpyAsync(dj, table.data(), table.size(), cudaMemcpyHostToDevice, bst));
+  const FftJob* dev = static_cast<const FftJob*>(dj);
+  PICARD_TRY(table_stages(dev, reinterpret_cast<const FftSeg*>(static_cast<unsigned char*>(dj) + jb), range, bst));
   PICARD_CUDA(cudaFreeAsync(dj, bst));
   PICARD_CUDA(cudaEventRecord(bev, bst));
   for (int r : fft_runs) PICARD_CUDA(cudaStreamWaitEvent(ctxs[r]->st, bev, 0));
