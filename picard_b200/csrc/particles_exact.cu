@@ -8,6 +8,7 @@
 // converted to the CELL32 layout only when stored.
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cmath>
 
 #include "common.cuh"
@@ -581,14 +582,40 @@ struct Cic64 {
   double F[8];
 };
 
+// One axis: base node int((x - lo)/d + 1/2) and fmod(x - lo + d/2, d), both
+// exactly as the reference's arithmetic gives them.  The quotient by the
+// reciprocal decides unless it lies within 1e-6 of an integer (its error is a
+// few ulp of at most 2^31), where the division does; the remainder is one FMA
+// (exact when it lies in [0, d)), else fmod's.  Three library fmod calls and
+// divisions a particle were most of the deposit's and the push's instructions.
+__device__ __forceinline__ void cic_axis(double x, double lo, double d, double inv, int& i, double& rest) {
+  const double a = x - lo, t2 = a * inv + 0.5;
+  i = int(t2);
+  if (!(fabs(t2 - rint(t2)) >= 1e-6)) i = int(a / d + 0.5);
+  const double t = a + 0.5 * d;
+  rest = fma(-double(i), d, t);
+  if (!(rest >= 0.0 && rest < d)) rest = fmod(t, d);
+}
+
+// Base node and the distances `r` from it on each axis.
+struct Cic64Axes {
+  int i, j, k;
+  double r[3];
+};
+__device__ __forceinline__ void cic_axes(const KParams& P, double x, double y, double z, Cic64Axes& c) {
+  cic_axis(x, P.Lx_min, P.dx, 1.0 / P.dx, c.i, c.r[0]);
+  cic_axis(y, P.Ly_min, P.dy, 1.0 / P.dy, c.j, c.r[1]);
+  cic_axis(z, P.Lz_min, P.dz, 1.0 / P.dz, c.k, c.r[2]);
+}
+
 __device__ inline void cic64(const KParams& P, double x, double y, double z, Cic64& w) {
-  double rest0 = fmod(x - P.Lx_min + 0.5 * P.dx, P.dx);
-  double rest1 = fmod(y - P.Ly_min + 0.5 * P.dy, P.dy);
-  double rest2 = fmod(z - P.Lz_min + 0.5 * P.dz, P.dz);
-  double d0 = P.dx - rest0, d1 = P.dy - rest1, d2 = P.dz - rest2;
-  w.i = int((x - P.Lx_min) / P.dx + 0.5);
-  w.j = int((y - P.Ly_min) / P.dy + 0.5);
-  w.k = int((z - P.Lz_min) / P.dz + 0.5);
+  Cic64Axes c;
+  cic_axes(P, x, y, z, c);
+  const double rest0 = c.r[0], rest1 = c.r[1], rest2 = c.r[2];
+  const double d0 = P.dx - rest0, d1 = P.dy - rest1, d2 = P.dz - rest2;
+  w.i = c.i;
+  w.j = c.j;
+  w.k = c.k;
   w.F[0] = d0 * d1 * d2;
   w.F[1] = rest0 * d1 * d2;
   w.F[2] = d0 * rest1 * d2;
@@ -735,6 +762,234 @@ __device__ inline unsigned long long stencil_key(int i, int j, int k, int s) {
   return (c(i) | (c(j) << 20) | (c(k) << 40)) << 4 | (unsigned long long)s;
 }
 
+// True when x lies within half a cell of [L_min, L_max] (NaN: false).  There
+// the CIC base node is 0 .. n and both stencil nodes lie inside the
+// ghost-padded box, with non-negative weights.  The reference deposits after
+// BCoutflow and ParticlesTransfer, which leave every particle inside
+// [min, max], so its particles always pass.
+__device__ inline bool within_half_cell(double x, double lo, double hi, double d) {
+  return x >= lo - 0.5 * d && x < hi + 0.5 * d;
+}
+
+// F (a product of three distances) -> round(F/dV 2^40), scale = 2^40/dV: one
+// FMA against 1.5 2^52 leaves the integer in the low mantissa bits (|result| <
+// 2^51).  Every FP64 deposit takes its weights from here, so their sums agree
+// bit for bit.
+__device__ __forceinline__ long long fixed_bits_f64(double F, double scale) {
+  return __double_as_longlong(fma(F, scale, 6755399441055744.0));
+}
+__device__ __forceinline__ long long fixed_f64(double F, double scale) {
+  return fixed_bits_f64(F, scale) - 0x4338000000000000LL;
+}
+
+// The deposit of FP64 positions (ParticlesGridify.f90:65-123), shared-memory
+// tiled as the CELL32 one (deposit_tile_c32_kernel): a warp takes 64
+// consecutive particles, two to a lane in 16-byte loads, finds the box of their
+// CIC stencils, adds the weights in 20-bit halves to its own tile, lane
+// l visiting the corners in the order q ^ (l & 7), and flushes each touched
+// node to global memory once.  A box that does not fit keeps the particles
+// around the warp's middle cell and adds the others' corners directly.
+//
+// CALLER: positions and 1-based species of another owner (gridify_noalloc):
+// species outside 1 .. species, and positions farther than half a cell outside
+// the domain, are skipped.  VEC: the arrays allow 16-byte loads.
+//
+// What bounds it: instruction issue (65 % of the slots; FP64 arithmetic, then
+// 16 shared atomics a particle).  8 M particles on 64^3: 198 us, against 1687
+// for one particle per lane with warp aggregation by match_any and two
+// partial-mask reductions per corner, three fmod calls and eleven divisions; 1
+// M on 32^3 47 and 218, 2 M on 90^3 (under three per cell) 129 and 648, 4 M in
+// no order 234 and 1424.  Two particles per lane at 64 registers beat four (80
+// registers 248 us, 106 registers 261) and eight (128 registers, 521).
+constexpr int kTileF64 = 768;   // entries per warp (two u32 halves)
+constexpr int kTileWarps = 8;
+constexpr int kTilePer = 2;     // particles per lane
+constexpr int kTileCtas = 4;    // CTAs per SM (64 registers, 48 KB)
+
+template <bool CALLER, bool VEC, class Sp>
+__global__ void __launch_bounds__(256, kTileCtas) deposit_tile_f64_kernel(KParams P, const double* __restrict__ x,
+                                                                  const double* __restrict__ y,
+                                                                  const double* __restrict__ z,
+                                                                  const Sp* __restrict__ sp, long long n,
+                                                                  unsigned long long* Nacc, int reach) {
+  extern __shared__ unsigned int f64_tile[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned int* lo = f64_tile + warp * 2 * kTileF64;
+  constexpr int kHi = kTileF64;
+  const bool sx = lane & 1, sy = lane & 2, sz = lane & 4;
+  const double scale = kDepositScale / P.dV;
+  int zeroed = 0;  // entries below this are zero between chunks: the flush clears what it reads
+  const long long warps = (long long)gridDim.x * kTileWarps;
+  for (long long base = ((long long)blockIdx.x * kTileWarps + warp) * (32 * kTilePer); base < n;
+       base += warps * (32 * kTilePer)) {
+    // pairs of consecutive particles: base + 2 lane
+    double px[kTilePer], py[kTilePer], pz[kTilePer];
+    int s[kTilePer];
+    Cic64Axes c[kTilePer];
+    unsigned live = 0;
+    const bool full = base + 32 * kTilePer <= n;
+#pragma unroll
+    for (int h = 0; h < kTilePer / 2; ++h) {
+      const long long p = base + 64 * h + 2 * lane;
+      if (VEC && full) {
+        const double2 vx = __ldcs(reinterpret_cast<const double2*>(x + p)), vy = __ldcs(reinterpret_cast<const double2*>(y + p)),
+                      vz = __ldcs(reinterpret_cast<const double2*>(z + p));
+        px[2 * h] = vx.x, px[2 * h + 1] = vx.y;
+        py[2 * h] = vy.x, py[2 * h + 1] = vy.y;
+        pz[2 * h] = vz.x, pz[2 * h + 1] = vz.y;
+        s[2 * h] = int(sp[p]), s[2 * h + 1] = int(sp[p + 1]);
+        live |= 3u << (2 * h);
+      } else {
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          const bool in = p + t < n;
+          px[2 * h + t] = in ? x[p + t] : 0.0;
+          py[2 * h + t] = in ? y[p + t] : 0.0;
+          pz[2 * h + t] = in ? z[p + t] : 0.0;
+          s[2 * h + t] = in ? int(sp[p + t]) : 0;
+          if (in) live |= 1u << (2 * h + t);
+        }
+      }
+    }
+    int imin = INT_MAX, imax = INT_MIN, jmin = INT_MAX, jmax = INT_MIN, kmin = INT_MAX, kmax = INT_MIN;
+    int smin = INT_MAX, smax = INT_MIN;
+    unsigned near = 0;
+    auto widen = [&](int m) {
+      near |= 1u << m;
+      imin = min(imin, c[m].i), imax = max(imax, c[m].i);
+      jmin = min(jmin, c[m].j), jmax = max(jmax, c[m].j);
+      kmin = min(kmin, c[m].k), kmax = max(kmax, c[m].k);
+      smin = min(smin, s[m]), smax = max(smax, s[m]);
+    };
+#pragma unroll
+    for (int m = 0; m < kTilePer; ++m) {
+      if (CALLER) {
+        s[m] -= 1;
+        if (!(s[m] >= 0 && s[m] < P.species && within_half_cell(px[m], P.Lx_min, P.Lx_max, P.dx) &&
+              within_half_cell(py[m], P.Ly_min, P.Ly_max, P.dy) && within_half_cell(pz[m], P.Lz_min, P.Lz_max, P.dz)))
+          live &= ~(1u << m);
+      }
+      cic_axes(P, px[m], py[m], pz[m], c[m]);
+      // only non-negative weights go to the tile
+      const bool in = c[m].r[0] >= 0.0 && c[m].r[0] <= P.dx && c[m].r[1] >= 0.0 && c[m].r[1] <= P.dy &&
+                      c[m].r[2] >= 0.0 && c[m].r[2] <= P.dz;
+      if ((live >> m & 1u) && in) widen(m);
+    }
+    auto reduce_box = [&]() -> int {
+      imin = __reduce_min_sync(0xffffffffu, imin), imax = __reduce_max_sync(0xffffffffu, imax);
+      jmin = __reduce_min_sync(0xffffffffu, jmin), jmax = __reduce_max_sync(0xffffffffu, jmax);
+      kmin = __reduce_min_sync(0xffffffffu, kmin), kmax = __reduce_max_sync(0xffffffffu, kmax);
+      smin = __reduce_min_sync(0xffffffffu, smin), smax = __reduce_max_sync(0xffffffffu, smax);
+      if (imax < imin) return 0;  // nothing near
+      const long long bi = (long long)imax - imin + 2, bj = (long long)jmax - jmin + 2, bk = (long long)kmax - kmin + 2;
+      if (bi > 64 || bj > 64 || bk > 64) return 0;
+      const int v = int(bi * bj * bk) * (smax - smin + 1);
+      return v <= kTileF64 ? v : 0;
+    };
+    int vol = reduce_box();
+    if (vol == 0) {
+      // the particles around the first near one of the middle lane that has one
+      const unsigned have = __ballot_sync(0xffffffffu, near != 0u);
+      if (have) {
+        const unsigned upper = have & 0xffff0000u;
+        const int src = upper ? __ffs(upper) - 1 : 31 - __clz(have);
+        int mi = 0, mj = 0, mk = 0;
+#pragma unroll
+        for (int m = kTilePer - 1; m >= 0; --m)
+          if (near >> m & 1u) mi = c[m].i, mj = c[m].j, mk = c[m].k;
+        mi = __shfl_sync(0xffffffffu, mi, src), mj = __shfl_sync(0xffffffffu, mj, src), mk = __shfl_sync(0xffffffffu, mk, src);
+        const unsigned was = near;
+        near = 0;
+        imin = jmin = kmin = smin = INT_MAX;
+        imax = jmax = kmax = smax = INT_MIN;
+#pragma unroll
+        for (int m = 0; m < kTilePer; ++m)
+          if ((was >> m & 1u) && abs(c[m].i - mi) <= reach && abs(c[m].j - mj) <= 2 && abs(c[m].k - mk) <= 2) widen(m);
+        vol = reduce_box();
+      }
+      if (vol == 0) near = 0;
+    }
+    if (vol > 0) {
+      const int bi = imax - imin + 2, bj = jmax - jmin + 2, bk = kmax - kmin + 2;
+      const int sj = bi, sk = bi * bj, ss = sk * bk;
+      if (vol > zeroed) {
+        for (int e = zeroed + lane; e < vol; e += 32) lo[e] = 0u, lo[e + kHi] = 0u;
+        zeroed = vol;
+        __syncwarp();
+      }
+      const int first = (sx ? 1 : 0) + (sy ? sj : 0) + (sz ? sk : 0) - (imin + jmin * sj + kmin * sk + smin * ss);
+      const int ex = sx ? -1 : 1, ey = sy ? -sj : sj, ez = sz ? -sk : sk;
+#pragma unroll
+      for (int m = 0; m < kTilePer; ++m) {
+        if (!(near >> m & 1u)) continue;
+        const double r0 = c[m].r[0], r1 = c[m].r[1], r2 = c[m].r[2];
+        const double d0 = P.dx - r0, d1 = P.dy - r1, d2 = P.dz - r2;
+        const double ax[2] = {sx ? r0 : d0, sx ? d0 : r0}, ay[2] = {sy ? r1 : d1, sy ? d1 : r1},
+                     az[2] = {sz ? r2 : d2, sz ? d2 : r2};
+        unsigned int* e0 = lo + (first + c[m].i + c[m].j * sj + c[m].k * sk + s[m] * ss);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const long long u = fixed_bits_f64((ax[q & 1] * ay[q >> 1 & 1]) * az[q >> 2], scale);
+          unsigned int* e = e0 + ((q & 1) ? ex : 0) + ((q & 2) ? ey : 0) + ((q & 4) ? ez : 0);
+          // low 20 bits; the high ones under a constant top bit that the sum masks off
+          atomicAdd(e, unsigned(u) & 0xFFFFFu);
+          atomicAdd(e + kHi, unsigned(u >> 20));
+        }
+      }
+      __syncwarp();
+      // v / d = (v inv) >> 16 for v < 1024, d <= 64
+      const uint32_t ri = (65535u + bi) / uint32_t(bi), rj = (65535u + bj) / uint32_t(bj), rk = (65535u + bk) / uint32_t(bk);
+      for (int e = lane; e < vol; e += 32) {
+        const unsigned l = lo[e], h = lo[e + kHi];
+        if ((l | h) == 0u) continue;
+        lo[e] = 0u, lo[e + kHi] = 0u;
+        const int r1 = int((uint32_t(e) * ri) >> 16), r2 = int((uint32_t(r1) * rj) >> 16),
+                  r3 = int((uint32_t(r2) * rk) >> 16);
+        const int i = fold_index(e - r1 * bi + imin, P.nx, P.xflow), j = fold_index(r1 - r2 * bj + jmin, P.ny, P.yflow),
+                  k = fold_index(r2 - r3 * bk + kmin, P.nz, P.zflow);
+        const unsigned long long v = ((unsigned long long)(h & 0x7FFFFFFFu) << 20) + (unsigned long long)l;
+        atomicAdd(Nacc + (long long)(r3 + smin) * P.nodes + node_index(P, i, j, k), v);
+      }
+      __syncwarp();
+    }
+    unsigned far = live & ~near;
+    if (__any_sync(0xffffffffu, far != 0u)) {
+#pragma unroll
+      for (int m = 0; m < kTilePer; ++m) {
+        if (!(far >> m & 1u)) continue;
+        unsigned long long* plane = Nacc + (long long)s[m] * P.nodes;
+#pragma unroll 1
+        for (int q = 0; q < 8; ++q) {
+          const double F = (((q & 1) ? c[m].r[0] : P.dx - c[m].r[0]) * ((q & 2) ? c[m].r[1] : P.dy - c[m].r[1])) *
+                           ((q & 4) ? c[m].r[2] : P.dz - c[m].r[2]);
+          const int i = fold_index(c[m].i + (q & 1), P.nx, P.xflow), j = fold_index(c[m].j + (q >> 1 & 1), P.ny, P.yflow),
+                    k = fold_index(c[m].k + (q >> 2), P.nz, P.zflow);
+          atomicAdd(plane + node_index(P, i, j, k), (unsigned long long)fixed_f64(F, scale));
+        }
+      }
+    }
+  }
+}
+
+template <bool CALLER, class Sp>
+cudaError_t launch_deposit_tile_f64(const KParams& P, const double* x, const double* y, const double* z, const Sp* sp,
+                                    long long n, unsigned long long* acc, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const size_t smem = size_t(kTileWarps) * 2 * sizeof(unsigned int) * kTileF64;  // within the default 48 KB
+  const long long chunk = (long long)kTileWarps * 32 * kTilePer, chunks = (n + chunk - 1) / chunk;
+  const int grid = int(chunks < 148LL * kTileCtas ? chunks : 148LL * kTileCtas);
+  // the window reaches as far along x as one warp's particles do at this density, and two cells
+  const long long span = 32LL * kTilePer * P.nx * P.ny * P.nz / n + 2;
+  const int reach = int(span < 15 ? span : 15);
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(z);
+  note_launch();
+  if (bits % 16 == 0)
+    deposit_tile_f64_kernel<CALLER, true, Sp><<<grid, 256, smem, st>>>(P, x, y, z, sp, n, acc, reach);
+  else
+    deposit_tile_f64_kernel<CALLER, false, Sp><<<grid, 256, smem, st>>>(P, x, y, z, sp, n, acc, reach);
+  return cudaGetLastError();
+}
+
 __global__ void deposit_f64_kernel(KParams P, PartF64 a, long long n, unsigned long long* Nacc,
                                    unsigned long long* Facc) {
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -751,7 +1006,7 @@ __global__ void deposit_f64_kernel(KParams P, PartF64 a, long long n, unsigned l
       s = a.sp[p];
       for (int q = 0; q < 8; ++q) {
         Fw[q] = c.F[q] / P.dV;
-        w[q] = __double2ll_rn(Fw[q] * kDepositScale);
+        w[q] = fixed_f64(c.F[q], kDepositScale / P.dV);
         int i = fold_index(c.i + kOff[q][0], P.nx, P.xflow), j = fold_index(c.j + kOff[q][1], P.ny, P.yflow),
             k = fold_index(c.k + kOff[q][2], P.nz, P.zflow);
         nodes[q] = node_index(P, i, j, k);
@@ -1055,6 +1310,7 @@ cudaError_t launch_advance_velocity_f64(const KParams& P, PartF64 a, long long n
 cudaError_t launch_deposit_f64(const KParams& P, PartF64 a, long long n, unsigned long long* Nacc,
                                unsigned long long* Facc, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
+  if (!Facc) return launch_deposit_tile_f64<false>(P, a.x, a.y, a.z, a.sp, n, Nacc, st);
   note_launch();
   deposit_f64_kernel<<<persistent_grid(n), kThreads, 0, st>>>(P, a, n, Nacc, Facc);
   return cudaGetLastError();
@@ -1118,54 +1374,6 @@ namespace {
 // process exits.  All calls share it, so calls that overlap on the GPU race.
 static __device__ __align__(256) unsigned long long g_noalloc_acc[PICARD_NOALLOC_MAX_WORDS];
 
-// True when x lies within half a cell of [L_min, L_max] (NaN: false).  There
-// the CIC base node is 0 .. n and both stencil nodes lie inside the
-// ghost-padded box, with non-negative weights.  The reference deposits after
-// BCoutflow and ParticlesTransfer, which leave every particle inside
-// [min, max], so its particles always pass.
-__device__ inline bool within_half_cell(double x, double lo, double hi, double d) {
-  return x >= lo - 0.5 * d && x < hi + 0.5 * d;
-}
-
-// ParticlesGridify.f90:65-123 for caller-owned FP64 arrays; int_particles
-// holds the reference's 1-based species numbers.  Particles of another
-// species number, or farther than half a cell outside the domain on some
-// axis, are not deposited.
-__global__ void deposit_noalloc_kernel(KParams P, const double* __restrict__ x, const double* __restrict__ y,
-                                       const double* __restrict__ z, const int32_t* __restrict__ sp1, long long n,
-                                       unsigned long long* acc) {
-  long long stride = (long long)gridDim.x * blockDim.x;
-  long long n_round = ((n + 31) / 32) * 32;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n_round; p += stride) {
-    int s = (p < n) ? sp1[p] - 1 : -1;
-    bool active = s >= 0 && s < P.species;
-    double xp = 0.0, yp = 0.0, zp = 0.0;
-    if (active) {
-      xp = x[p];
-      yp = y[p];
-      zp = z[p];
-      active = within_half_cell(xp, P.Lx_min, P.Lx_max, P.dx) && within_half_cell(yp, P.Ly_min, P.Ly_max, P.dy) &&
-               within_half_cell(zp, P.Lz_min, P.Lz_max, P.dz);
-    }
-    long long w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, nodes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    unsigned long long key = ~0ull;
-    if (active) {
-      Cic64 c;
-      cic64(P, xp, yp, zp, c);
-      for (int q = 0; q < 8; ++q) {
-        w[q] = __double2ll_rn(c.F[q] / P.dV * kDepositScale);
-        int i = fold_index(c.i + kOff[q][0], P.nx, P.xflow), j = fold_index(c.j + kOff[q][1], P.ny, P.yflow),
-            k = fold_index(c.k + kOff[q][2], P.nz, P.zflow);
-        nodes[q] = node_index(P, i, j, k);
-      }
-      key = stencil_key(c.i, c.j, c.k, s);
-    } else {
-      s = 0;
-    }
-    deposit8(key, active, w, nodes, acc + (long long)s * P.nodes);
-  }
-}
-
 // N(s, node) = n2p_s * acc * 2^-40 in the reference layout (species fastest),
 // with the ghost folds of ParticlesGridify.f90:149-278; C = sum_s q_s N_s.
 __global__ void finish_noalloc_kernel(KParams P, const unsigned long long* acc, double* N, double* C) {
@@ -1222,11 +1430,8 @@ extern "C" int picard_gpu_particles_gridify_noalloc(const picard_params* p, cons
   // the array keeps the previous call's sums: clear the part this call uses
   e = cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * (size_t)words, st);
   if (e != cudaSuccess) return fail(PICARD_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-  if (num_local > 0) {
-    note_launch();
-    deposit_noalloc_kernel<<<persistent_grid(num_local), kThreads, 0, st>>>(K, x, y, z, int_particles, num_local,
-                                                                             acc);
-  }
+  e = launch_deposit_tile_f64<true>(K, x, y, z, int_particles, num_local, acc, st);
+  if (e != cudaSuccess) return fail(PICARD_ERR_CUDA, std::string("deposit launch: ") + cudaGetErrorString(e));
   note_launch();
   finish_noalloc_kernel<<<grid_for(nodes), kThreads, 0, st>>>(K, acc, N, C);
   e = cudaGetLastError();
