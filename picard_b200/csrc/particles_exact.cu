@@ -70,23 +70,35 @@ __device__ void half_rotate(double v[3], const double ve[3], const double tB[3])
 // Member `m` of the group (ss, pp) at cell `a`: m = 0 is the ion,
 // 1..epp its electrons, epp+1.. its protons.  ParticlesInitialize.f90:65-113,
 // BCinflow.f90:66-114.
-__device__ void gen_member(const KParams& P, uint32_t tag, uint32_t it, uint32_t a, int ss, int pp, int m, double x0,
-                           double y0, double z0, double x[3], double v[3], int& sp) {
-  int s0 = ss - 1;
-  Site ion(P.seed, a, (uint32_t(ss) << 24) | (uint32_t(pp) << 8), it, tag);
+// In two parts: the position, which all members of a group share, and the
+// velocity of member m.
+__device__ __forceinline__ void gen_position(const KParams& P, Site& ion, double x0, double y0, double z0, double x[3]) {
   x[0] = x0 + P.dx * ion.u(0);
   x[1] = y0 + P.dy * ion.u(1);
   x[2] = z0 + P.dz * ion.u(2);
+}
+__device__ inline int member_species(const KParams& P, int ss, int m) {
+  return m == 0 ? ss - 1 : (m <= P.epp[ss - 1] ? 0 : 1);  // the ion; 0 = electron, 1 = proton
+}
+__device__ void gen_velocity(const KParams& P, uint32_t tag, uint32_t it, uint32_t a, int ss, int pp, int m,
+                             const Site& ion, double v[3], int& sp) {
+  int s0 = ss - 1;
   // The ion draws its velocity from its own site after the position (from
   // u(3)); an electron or proton from a site of its own (from u(0)).  One
   // code path for both, so that a warp holding ions and their members runs
   // the Gaussian draws and the rotation once, not once per kind.
   const bool is_ion = m == 0;
-  const int t = is_ion ? s0 : (m <= P.epp[s0] ? 0 : 1);  // member: 0 = electron, 1 = proton
+  const int t = member_species(P, ss, m);
   Site src = is_ion ? ion : Site(P.seed, a, (uint32_t(ss) << 24) | (uint32_t(pp) << 8) | uint32_t(m), it, tag);
   gaussian_from(src, is_ion ? 3u : 0u, v, P.v0[s0], P.kelvin[t], P.mass[t]);
   half_rotate(v, P.ve, P.tB[t]);
   sp = t;
+}
+__device__ void gen_member(const KParams& P, uint32_t tag, uint32_t it, uint32_t a, int ss, int pp, int m, double x0,
+                           double y0, double z0, double x[3], double v[3], int& sp) {
+  Site ion(P.seed, a, (uint32_t(ss) << 24) | (uint32_t(pp) << 8), it, tag);
+  gen_position(P, ion, x0, y0, z0, x);
+  gen_velocity(P, tag, it, a, ss, pp, m, ion, v, sp);
 }
 
 // Slot of (ss, pp, member) inside one cell's block of created particles.
@@ -208,10 +220,10 @@ struct StoreC32 {
 // Candidate indices of one BCinflow call are decoded in 32-bit arithmetic.
 constexpr long long kMaxInflowCandidates = 0xFFFFFFFFLL;
 
-// Guard cell g of the inflow enumeration; the launchers keep every candidate
+// Guard cell g of the inflow enumeration, and the axis of its face; the launchers keep every candidate
 // index (and so g) below 2^32, so the decode divides in 32 bits.
-__device__ inline void inflow_cell(const KParams& P, const InflowTable& T, uint32_t g, int& ii, int& jj, int& kk,
-                                   double& x0, double& y0, double& z0) {
+__device__ inline int inflow_cell(const KParams& P, const InflowTable& T, uint32_t g, int& ii, int& jj, int& kk,
+                                  double& x0, double& y0, double& z0) {
   int f = 0;
   while (f < T.nfaces - 1 && (long long)g >= T.f[f + 1].first) ++f;
   const InflowFace& F = T.f[f];
@@ -241,6 +253,7 @@ __device__ inline void inflow_cell(const KParams& P, const InflowTable& T, uint3
     y0 = P.Ly_min + P.dy * (jj - 2);
     z0 = F.edge;
   }
+  return F.axis;
 }
 
 // BCinflow.f90:23-476 (append every candidate, reference order).
@@ -284,20 +297,68 @@ __device__ inline void transfer_wrap(const KParams& P, double& x, double& y, dou
   if (x > P.xmax) x = x - Lx;
 }
 
-// Fast-path inflow: BCinflow + AdvancePosition + BCoutflow + ParticlesTransfer
-// for the new candidates only.  Candidate t is generated, advanced by dt,
-// tested and wrapped; true = it survives.
-__device__ inline bool inflow_candidate(const KParams& P, const InflowTable& T, int iteration, long long t,
-                                        double x[3], double v[3], int& sp) {
-  const uint32_t tu = uint32_t(t), pc = uint32_t(T.per_cell), g = tu / pc;
-  const int local = int(tu - g * pc);
-  int ii, jj, kk;
+// How far a created particle can move in one step along each axis, by its
+// species.  A Gaussian draw is at most sqrt(-2 ln 2^-53) < 8.58 standard
+// deviations (the uniform it comes from is at least 2^-53), and the half
+// rotation keeps |v - ve|, so |v_c| <= |ve_c| + |v0 - ve| + sqrt(3) 8.58 sigma;
+// a millionth more covers the rounding.
+struct InflowReach {
+  double r[8][3];
+};
+
+InflowReach inflow_reach(const KParams& P) {
+  InflowReach R;
+  for (int t = 0; t < 8; ++t) {
+    double drift = 0.0;  // over the ion species that create members of species t
+    for (int s = 0; s < P.species; ++s) {
+      double d2 = 0.0;
+      for (int c = 0; c < 3; ++c) d2 += (P.v0[s][c] - P.ve[c]) * (P.v0[s][c] - P.ve[c]);
+      drift = std::fmax(drift, std::sqrt(d2));
+    }
+    const double sigma = P.kelvin[t] > 0.0 && P.mass[t] > 0.0 ? std::sqrt(kKb * P.kelvin[t] / P.mass[t]) : 0.0;
+    for (int c = 0; c < 3; ++c)
+      R.r[t][c] = std::fabs(P.dt) * (std::fabs(P.ve[c]) + drift + 14.9 * sigma) * (1.0 + 1e-6);
+  }
+  return R;
+}
+
+// Candidate t of the fast-path inflow: its group member and the draw site of
+// its position.
+struct InflowSite {
+  int ss, pp, m, axis;
+  uint32_t a;
   double x0, y0, z0;
-  inflow_cell(P, T, g, ii, jj, kk, x0, y0, z0);
-  uint32_t a = uint32_t(node_index(P, ii - 1, jj - 1, kk - 1));
-  int ss, pp, m;
-  decode_group(P, T.group_prefix, local, ss, pp, m);
-  gen_member(P, kTagInflow, uint32_t(iteration), a, ss, pp, m, x0, y0, z0, x, v, sp);
+};
+__device__ __forceinline__ InflowSite inflow_site(const KParams& P, const InflowTable& T, uint32_t t) {
+  const uint32_t pc = uint32_t(T.per_cell), g = t / pc;
+  InflowSite S;
+  int ii, jj, kk;
+  S.axis = inflow_cell(P, T, g, ii, jj, kk, S.x0, S.y0, S.z0);
+  S.a = uint32_t(node_index(P, ii - 1, jj - 1, kk - 1));
+  decode_group(P, T.group_prefix, int(t - g * pc), S.ss, S.pp, S.m);
+  return S;
+}
+
+// Whether the candidate starts near enough to its face to cross it in one step
+// with some velocity (a comparison that is never true for a NaN bound gives
+// nothing up then).  One Philox block decides.
+__device__ __forceinline__ bool inflow_near(const KParams& P, const InflowTable& T, const InflowReach& R,
+                                            int iteration, uint32_t t) {
+  const InflowSite S = inflow_site(P, T, t);
+  Site ion(P.seed, S.a, (uint32_t(S.ss) << 24) | (uint32_t(S.pp) << 8), uint32_t(iteration), kTagInflow);
+  const int ax = S.axis;
+  const double q = (ax == 0 ? S.x0 : ax == 1 ? S.y0 : S.z0) + (ax == 0 ? P.dx : ax == 1 ? P.dy : P.dz) * ion.u(uint32_t(ax));
+  const double lo = ax == 0 ? P.xmin : ax == 1 ? P.ymin : P.zmin, hi = ax == 0 ? P.xmax : ax == 1 ? P.ymax : P.zmax;
+  const double r = R.r[member_species(P, S.ss, S.m)][ax];
+  return !(q < lo - r || q > hi + r);
+}
+
+// BCinflow + AdvancePosition + BCoutflow + ParticlesTransfer of candidate t:
+// generated, advanced by dt, tested and wrapped; true = it survives.
+__device__ inline bool inflow_candidate(const KParams& P, const InflowTable& T, int iteration, uint32_t t, double x[3],
+                                        double v[3], int& sp) {
+  const InflowSite S = inflow_site(P, T, t);
+  gen_member(P, kTagInflow, uint32_t(iteration), S.a, S.ss, S.pp, S.m, S.x0, S.y0, S.z0, x, v, sp);
   x[0] = x[0] + v[0] * P.dt;
   x[1] = x[1] + v[1] * P.dt;
   x[2] = x[2] + v[2] * P.dt;
@@ -334,9 +395,10 @@ __device__ int produce_number(const KParams& P, int iteration, uint32_t a, int s
   double nden = 0.0;
   if (P.vn[s0] > 0.0) nden = P.Qn[s0] / (2.0 * kTau * r2 * P.vn[s0]) * exp(-P.nu_d[s0] * r1 / P.vn[s0]);
   if (!(P.n2p[s0] > 0.0)) return 0;
-  Site r(P.seed, a, uint32_t(ss), uint32_t(iteration), kTagProduceCount);
   double rate = P.nu_i[s0] * nden * P.dV / P.n2p[s0];
   if (P.produce_dt_scaled) rate = rate * P.dt;
+  if (rate == 0.0) return 0;  // int(u) with u < 1
+  Site r(P.seed, a, uint32_t(ss), uint32_t(iteration), kTagProduceCount);
   return int(rate + r.u(0));
 }
 
@@ -495,85 +557,103 @@ struct OutflowF64 {
   }
 };
 
-// The fused inflow in two passes, so that survivors land in candidate order
-// (deterministic): per-block survivor counts, an exclusive scan, then every
-// block regenerates its candidates and stores the survivors at *count + its
-// offset + their rank in the block.
-__global__ void __launch_bounds__(kThreads) inflow_count_kernel(KParams P, InflowTable T, int iteration,
-                                                                long long total, int* block_counts) {
+// The fused inflow in one generation: every block takes up to 2,048 candidates, lists
+// in order those that start near enough to the domain to reach it in one step
+// (inflow_near: most do not, whatever velocity they would draw), generates the
+// listed ones in full, and writes the survivors, in candidate order, to its own
+// stretch of a staging area (FP64 position and velocity, species); after the
+// scan of the block counts, the place pass stores them at *count + the block's
+// offset + their rank.
+//
+// What bounds it: the integer decode of the candidates.  Listing first matters
+// as much as the early test itself: with a test ahead of the draws but 256
+// candidates a block, nearly every block still waited for one lane's logarithm
+// and sine.  256 x 128 x 128, 10.7 M candidates: 164 us, 267 with the test
+// alone, 612 when every candidate drew its velocity.
+// A block takes `items` candidates per thread: 1 on small grids, so that the
+// device fills, up to 8.
+constexpr int kInflowItems = 8;
+inline int inflow_items(long long candidates) {
+  const long long q = candidates / (148LL * 4 * kThreads);
+  return q < 1 ? 1 : q > kInflowItems ? kInflowItems : int(q);
+}
+__global__ void __launch_bounds__(kThreads) inflow_stage_kernel(KParams P, InflowTable T, InflowReach R, int iteration,
+                                                                long long total, int items, int* block_counts,
+                                                                double* stage, int8_t* stage_sp, long long stride) {
+  constexpr int kWords = kInflowItems * kThreads / 32;
+  static_assert(kWords == 64, "two words per lane of the scanning warp");
   __shared__ int warp_sums[32];
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double x[3], v[3];
-  int sp = 0;
-  const bool keep = t < total && inflow_candidate(P, T, iteration, t, x, v, sp);
-  int sum;
-  block_exclusive_scan(keep ? 1 : 0, warp_sums, sum);
-  if (threadIdx.x == 0) block_counts[blockIdx.x] = sum;
+  __shared__ uint16_t list[kInflowItems * kThreads];
+  __shared__ unsigned near[kWords];   // bit l of word w: candidate 32 w + l starts near enough
+  __shared__ int before[kWords + 1];  // listed candidates before each word's
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long base = (long long)blockIdx.x * items * kThreads;
+  for (int q = 0; q < kInflowItems; ++q) {
+    unsigned m = 0;
+    if (q < items) {
+      const long long t = base + q * kThreads + threadIdx.x;
+      m = __ballot_sync(0xffffffffu, t < total && inflow_near(P, T, R, iteration, uint32_t(t)));
+    }
+    if (lane == 0) near[q * (kThreads / 32) + warp] = m;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const int c0 = __popc(near[2 * lane]), v = c0 + __popc(near[2 * lane + 1]);
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    before[2 * lane] = x - v;
+    before[2 * lane + 1] = x - v + c0;
+    if (lane == 31) before[kWords] = x;
+  }
+  __syncthreads();
+  for (int q = 0; q < items; ++q) {
+    const int w = q * (kThreads / 32) + warp;
+    if (near[w] >> lane & 1u) list[before[w] + __popc(near[w] & ((1u << lane) - 1u))] = uint16_t(32 * w + lane);
+  }
+  const int listed = before[kWords];
+  __syncthreads();
+  int done = 0;
+  for (int first = 0; first < listed; first += kThreads) {
+    const int e = first + threadIdx.x;
+    double x[3], v[3];
+    int sp = 0;
+    const bool keep = e < listed && inflow_candidate(P, T, iteration, uint32_t(base) + list[e], x, v, sp);
+    int sum;
+    const int rank = block_exclusive_scan(keep ? 1 : 0, warp_sums, sum);
+    if (keep) {
+      const long long q = base + done + rank;
+      stage[q] = x[0];
+      stage[q + stride] = x[1];
+      stage[q + 2 * stride] = x[2];
+      stage[q + 3 * stride] = v[0];
+      stage[q + 4 * stride] = v[1];
+      stage[q + 5 * stride] = v[2];
+      stage_sp[q] = int8_t(sp);
+    }
+    done += sum;
+  }
+  if (threadIdx.x == 0) block_counts[blockIdx.x] = done;
 }
 
 template <class Store>
-__global__ void __launch_bounds__(kThreads) inflow_emit_kernel(KParams P, InflowTable T, int iteration,
-                                                               long long total, const int* offsets, const int* count,
-                                                               long long capacity, int* err, Store store) {
-  __shared__ int warp_sums[32];
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double x[3], v[3];
-  int sp = 0;
-  const bool keep = t < total && inflow_candidate(P, T, iteration, t, x, v, sp);
-  int sum;
-  const int rank = block_exclusive_scan(keep ? 1 : 0, warp_sums, sum);
-  if (keep) {
-    const long long slot = (long long)*count + offsets[blockIdx.x] + rank;
-    if (slot < capacity)
-      store(slot, x, v, sp);
-    else
-      atomicCAS(err, 0, int(kDevCapacity));
-  }
-}
-
-// The fused inflow in one generation: every block generates its candidates
-// once and writes its survivors, in candidate order, to its own stretch of a
-// staging area (FP64 position and velocity, species); after the scan of the
-// block counts, the place pass stores them at *count + the block's offset +
-// their rank -- the same slots and values as count + emit.
-__global__ void __launch_bounds__(kThreads) inflow_stage_kernel(KParams P, InflowTable T, int iteration,
-                                                                long long total, int* block_counts, double* stage,
-                                                                int8_t* stage_sp, long long stride) {
-  __shared__ int warp_sums[32];
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double x[3], v[3];
-  int sp = 0;
-  const bool keep = t < total && inflow_candidate(P, T, iteration, t, x, v, sp);
-  int sum;
-  const int rank = block_exclusive_scan(keep ? 1 : 0, warp_sums, sum);
-  if (keep) {
-    const long long q = (long long)blockIdx.x * blockDim.x + rank;
-    stage[q] = x[0];
-    stage[q + stride] = x[1];
-    stage[q + 2 * stride] = x[2];
-    stage[q + 3 * stride] = v[0];
-    stage[q + 4 * stride] = v[1];
-    stage[q + 5 * stride] = v[2];
-    stage_sp[q] = int8_t(sp);
-  }
-  if (threadIdx.x == 0) block_counts[blockIdx.x] = sum;
-}
-
-template <class Store>
-__global__ void __launch_bounds__(kThreads) inflow_place_kernel(const int* block_counts, const int* offsets,
+__global__ void __launch_bounds__(kThreads) inflow_place_kernel(int tile, const int* block_counts, const int* offsets,
                                                                 const int* count, long long capacity, int* err,
                                                                 const double* stage, const int8_t* stage_sp,
                                                                 long long stride, Store store) {
-  const int r = threadIdx.x;
-  if (r >= block_counts[blockIdx.x]) return;
-  const long long q = (long long)blockIdx.x * blockDim.x + r;
-  const double x[3] = {stage[q], stage[q + stride], stage[q + 2 * stride]};
-  const double v[3] = {stage[q + 3 * stride], stage[q + 4 * stride], stage[q + 5 * stride]};
-  const long long slot = (long long)*count + offsets[blockIdx.x] + r;
-  if (slot < capacity)
-    store(slot, x, v, int(stage_sp[q]));
-  else
-    atomicCAS(err, 0, int(kDevCapacity));
+  for (int r = threadIdx.x; r < block_counts[blockIdx.x]; r += blockDim.x) {
+    const long long q = (long long)blockIdx.x * tile + r;
+    const double x[3] = {stage[q], stage[q + stride], stage[q + 2 * stride]};
+    const double v[3] = {stage[q + 3 * stride], stage[q + 4 * stride], stage[q + 5 * stride]};
+    const long long slot = (long long)*count + offsets[blockIdx.x] + r;
+    if (slot < capacity)
+      store(slot, x, v, int(stage_sp[q]));
+    else
+      atomicCAS(err, 0, int(kDevCapacity));
+  }
 }
 
 // CIC weights of ParticlesGridify.f90:70-88 (F1..F8 before the 1/dV).
@@ -1043,12 +1123,19 @@ __global__ void energy_particles_f64_kernel(KParams P, PartF64 a, long long n, d
   }
 }
 
+// One block of 256 threads (a single thread walking the 2,368 partials took 61
+// us): strided sums, then a tree, in an order that depends on nb alone.
 __global__ void finish_sum_kernel(const double* partial, int nb, double scale, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double t = 0.0;
-    for (int b = 0; b < nb; ++b) t += partial[b];
-    *out = t * scale;
+  __shared__ double sh[256];
+  double t = 0.0;
+  for (int b = threadIdx.x; b < nb; b += 256) t += partial[b];
+  sh[threadIdx.x] = t;
+  __syncthreads();
+  for (int o = 128; o > 0; o >>= 1) {
+    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
   }
+  if (threadIdx.x == 0) *out = sh[0] * scale;
 }
 
 __global__ void cell_indices_f64_kernel(KParams P, PartF64 a, long long n, int* ijk) {
@@ -1144,7 +1231,7 @@ __global__ void f64_to_c32_kernel(KParams P, PartF64 a, long long n, PartC32 o) 
 
 int compact_blocks(long long n) { return int((n + kOutflowTile - 1) / kOutflowTile); }
 
-int inflow_blocks(long long candidates) { return grid_for(candidates); }
+int inflow_blocks(long long candidates) { return grid_for(candidates, inflow_items(candidates) * kThreads); }
 
 cudaError_t launch_calc_distance(const KParams& P, double* D, cudaStream_t st) {
   long long total = (long long)(P.nx + 1) * (P.ny + 1) * (P.nz + 1);
@@ -1211,26 +1298,17 @@ static cudaError_t inflow_fused(const KParams& P, const InflowTable& T, int iter
   if (total == 0) return cudaSuccess;
   if (total > kMaxInflowCandidates) return cudaErrorInvalidValue;
   const int nb = inflow_blocks(total);
+  const InflowReach R = inflow_reach(P);
   cudaError_t e;
-  if (S.x) {
-    const long long stride = (long long)nb * kThreads;
-    note_launch();
-    inflow_stage_kernel<<<nb, kThreads, 0, st>>>(P, T, iteration, total, block_counts, S.x, S.sp, stride);
-    e = launch_scan_int(block_counts, block_offsets, nb, block_offsets + nb, block_offsets + nb + 1, st);
-    if (e != cudaSuccess) return e;
-    note_launch();
-    inflow_place_kernel<<<nb, kThreads, 0, st>>>(block_counts, block_offsets, count, capacity, err, S.x, S.sp, stride,
-                                                 store);
-    note_launch();
-    add_count_kernel<<<1, 1, 0, st>>>(count, block_offsets + nb, capacity);
-    return cudaGetLastError();
-  }
+  const int items = inflow_items(total), tile = items * kThreads;
+  const long long stride = (long long)nb * tile;
   note_launch();
-  inflow_count_kernel<<<nb, kThreads, 0, st>>>(P, T, iteration, total, block_counts);
+  inflow_stage_kernel<<<nb, kThreads, 0, st>>>(P, T, R, iteration, total, items, block_counts, S.x, S.sp, stride);
   e = launch_scan_int(block_counts, block_offsets, nb, block_offsets + nb, block_offsets + nb + 1, st);
   if (e != cudaSuccess) return e;
   note_launch();
-  inflow_emit_kernel<<<nb, kThreads, 0, st>>>(P, T, iteration, total, block_offsets, count, capacity, err, store);
+  inflow_place_kernel<<<nb, kThreads, 0, st>>>(tile, block_counts, block_offsets, count, capacity, err, S.x, S.sp, stride,
+                                               store);
   note_launch();
   add_count_kernel<<<1, 1, 0, st>>>(count, block_offsets + nb, capacity);
   return cudaGetLastError();
@@ -1249,7 +1327,7 @@ cudaError_t launch_inflow_fused_f64(const KParams& P, const InflowTable& T, int 
   return inflow_fused(P, T, iteration, StoreF64{out}, count, capacity, block_counts, block_offsets, err, stage, st);
 }
 
-long long inflow_stage_slots(long long candidates) { return (long long)inflow_blocks(candidates) * kThreads; }
+long long inflow_stage_slots(long long candidates) { return (long long)inflow_blocks(candidates) * inflow_items(candidates) * kThreads; }
 
 cudaError_t launch_produce_emit_f64(const KParams& P, int iteration, const int* offsets, PartF64 out, int* count,
                                     long long capacity, int* err, cudaStream_t st) {
@@ -1322,7 +1400,7 @@ cudaError_t launch_energy_particles_f64(const KParams& P, PartF64 a, long long n
   note_launch();
   energy_particles_f64_kernel<<<nb, kThreads, 0, st>>>(P, a, n, rb.partial);
   note_launch();
-  finish_sum_kernel<<<1, 32, 0, st>>>(rb.partial, nb, 0.5, rb.result);
+  finish_sum_kernel<<<1, 256, 0, st>>>(rb.partial, nb, 0.5, rb.result);
   return cudaGetLastError();
 }
 
