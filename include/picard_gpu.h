@@ -147,9 +147,10 @@ PICARD_API const char* picard_gpu_last_error(void);
  * by memory budget); nothing is allocated.  Not counted: buffers a context
  * allocates on first use -- the flux accumulators of GridifyAll (48 B per
  * node and species), the second particle buffer and scratch of
- * picard_gpu_sort_particles, and the pointer-jumping scratch of
- * picard_gpu_bc_outflow (8 B per removed particle, up to 8 B per particle of
- * capacity). */
+ * picard_gpu_sort_particles, the pointer-jumping scratch of
+ * picard_gpu_bc_outflow (4 B per removed particle, up to 4 B per particle of
+ * capacity), the partial sums of the direct BCpotentials (a few MB), and those
+ * of the FP64 sweeps that run in one cluster (up to 17 MB). */
 PICARD_API int picard_gpu_footprint(const picard_params* p, int32_t layout, int32_t solver, uint64_t* bytes);
 /* Context memory comes from the device's stream-ordered pool.  By default the
  * pool hands freed memory back to the driver at the next synchronisation, so

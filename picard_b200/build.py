@@ -28,6 +28,7 @@ UNITS = {
     "bcpot_tc.cu": [],
     "solver.cu": [],
     "jacobi_resident.cu": [],
+    "jacobi_cluster.cu": [],
     "context.cu": [],
     "driver.cu": [],
     "server.cu": [],

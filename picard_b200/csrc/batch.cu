@@ -803,8 +803,8 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
         PICARD_CUDA(launch_inflow_fused(c, it));
         PICARD_TRY(count_issue(c));
         PICARD_TRY(count_collect(c));
-        PICARD_TRY(settle(r));
-        return picard_gpu_particles_gridify(c);
+        PICARD_TRY(picard_gpu_particles_gridify(c));
+        return settle(r);  // while the device has the deposit to do
       }));
       lap(0);
       // ---- BCpotentials (FFT runs: one launch per stage for all of them)

@@ -303,7 +303,8 @@ int bc_potentials_async(picard_ctx* c) {
     PICARD_CUDA(launch_bc_potentials_tc(c->K, c->C, c->D, c->U, c->tc_cs, c->tc_partial, c->d_err, c->st));
     return PICARD_OK;
   }
-  PICARD_CUDA(launch_bc_potentials(c->K, c->C, c->D, c->U, c->st));
+  if (!c->bc_scratch) PICARD_TRY(dalloc(c, c->bc_scratch, (size_t)bc_direct_scratch(c->K)));
+  PICARD_CUDA(launch_bc_potentials(c->K, c->C, c->D, c->U, c->bc_scratch, c->st));
   return PICARD_OK;
 }
 
@@ -445,7 +446,7 @@ int picard_gpu_create(const picard_params* p, int32_t layout, int32_t solver, pi
       return bail(rc);
   }
   const long long nn = s.nodes;
-  if ((rc = dalloc(c, c->d_count, 2)) || (rc = dalloc(c, c->d_info, 4)) ||
+  if ((rc = dalloc(c, c->d_count, 2)) || (rc = dalloc(c, c->d_info, 32)) ||
       (rc = dalloc(c, c->Nacc, nn * s.species)) || (rc = dalloc(c, c->N, nn * s.species)) ||
       (rc = dalloc(c, c->C, nn)) || (rc = dalloc(c, c->U, nn)) || (rc = dalloc(c, c->E, 3 * nn)) ||
       (rc = dalloc(c, c->D, s.dsize)) || (rc = dalloc(c, c->b, nn)) || (rc = dalloc(c, c->U1, nn)))
@@ -791,14 +792,17 @@ int picard_gpu_particles_produce(picard_ctx* c, int32_t iteration) {
 // BCoutflow.f90:5-87, in place and in the reference's order (outflow.cuh)
 //
 // In two stages around a read of the survivor count n': when the window
-// [n', n) is wide (2^16 positions or more) and at least 64 times its
-// survivors -- right after BCinflow has appended every candidate -- its chains
-// are resolved by pointer jumping (outflow.cuh), with scratch of two ints per
-// window position allocated on first use.
+// [n', n) holds 2^14 positions or more and at least four times its survivors --
+// right after BCinflow has appended every candidate -- its chains are resolved
+// by pointer jumping (outflow.cuh), with scratch of one int per window
+// position allocated on first use.  A chain takes about window/survivors
+// dependent loads (the longest several times that), the jumping a few rounds
+// over the window: with the reference's default parameters (30^3, a window of
+// 738,000) the walk took 312 us, the jumping takes 160.
 int picard_gpu_bc_outflow(picard_ctx* c) {
   if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
   const long long n = c->num_local;
-  OutflowSplit sp{1, 0, c->d_info, {nullptr, nullptr}};
+  OutflowSplit sp{1, 0, c->d_info, nullptr};
   PICARD_CUDA(launch_outflow_split(c, n, &sp));
   PICARD_CUDA(cudaMemcpyAsync(c->h_pinned_i + 6, c->d_info, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   PICARD_TRY(sync_count(c));
@@ -806,20 +810,18 @@ int picard_gpu_bc_outflow(picard_ctx* c) {
   const long long np = c->num_local, window = n - np, m = c->h_pinned_i[6];
   sp.stage = 2;
   sp.np = np;
-  if (window >= (1LL << 16) && window >= 64 * m) {
+  if (window >= (1LL << 14) && window >= 4 * m) {
     if (c->jump_cap < window) {
       const long long cap = std::min<long long>(c->capacity, std::max<long long>(window, 2 * c->jump_cap));
-      for (int q = 0; q < 2; ++q) {
-        if (c->jump[q]) {
-          release(c, c->jump[q]);
-          c->jump[q] = nullptr;
-        }
-        PICARD_TRY(dalloc(c, c->jump[q], (size_t)cap));
+      if (c->jump) {
+        release(c, c->jump);
+        c->jump = nullptr;
+        c->jump_cap = 0;
       }
+      PICARD_TRY(dalloc(c, c->jump, (size_t)cap));
       c->jump_cap = cap;
     }
-    sp.nxt[0] = c->jump[0];
-    sp.nxt[1] = c->jump[1];
+    sp.nxt = c->jump;
   }
   PICARD_CUDA(launch_outflow_split(c, n, &sp));
   return check_dev_err(c);

@@ -82,7 +82,7 @@ struct picard_ctx {
   picard::PartC32 c32 = {};
   int* d_count = nullptr;    // live particle count
   int* d_err = nullptr;      // error word, right after the count
-  int* d_info = nullptr;     // small device results read with a count (BCoutflow window)
+  int* d_info = nullptr;     // [32] small device results (BCoutflow: window survivors, jump rounds)
   long long num_local = 0;   // host mirror of *d_count
 
   // node arrays (plane-major, see common.cuh)
@@ -118,7 +118,7 @@ struct picard_ctx {
   int* blk_counts = nullptr;     // BCoutflow block counts and offsets
   int* blk_offsets = nullptr;
   uint2* out_words = nullptr;    // BCoutflow keep words (outflow.cuh)
-  int* jump[2] = {nullptr, nullptr};  // BCoutflow pointer jumping (allocated on first use)
+  int* jump = nullptr;           // BCoutflow pointer jumping (allocated on first use)
   long long jump_cap = 0;
   int* inflow_counts = nullptr;  // fused BCinflow block counts and offsets
   int* inflow_offsets = nullptr;
@@ -135,6 +135,13 @@ struct picard_ctx {
   float* res_faces = nullptr;
   unsigned int* res_bar = nullptr;
   long long res_faces_cap = 0;  // floats
+
+  // FP64 sweeps in one cluster (jacobi_cluster.cu): planned and allocated on
+  // the first solve
+  picard::ClusterPlan cluster;
+  bool cluster_planned = false;
+  double* cluster_partials = nullptr;  // [m_max][cluster_partials(plan)]
+  double* bc_scratch = nullptr;        // direct BCpotentials, allocated on first use
 
   int wait_test = 0;  // PICARD_OPT_WAIT_TEST
   // counting sort by cell (sort.cu): the second particle buffer and the

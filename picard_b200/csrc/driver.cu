@@ -284,7 +284,6 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
                                             c->d_err, c->st));
       PICARD_TRY(count_issue(c));
       PICARD_TRY(count_collect(c));
-      PICARD_TRY(settle(before));
     }
     // BCoutflow + ParticlesTransfer in place, in the reference's order
     PICARD_CUDA(launch_outflow(c, 1));
@@ -292,7 +291,6 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
     PICARD_CUDA(launch_inflow_fused(c, it));
     PICARD_TRY(count_issue(c));
     PICARD_TRY(count_collect(c));
-    PICARD_TRY(settle(before));
     // ParticlesTransfer's slot: every sort_every iterations, the particles
     // put back in cell order (a permutation; nothing downstream depends on it)
     if (c->sort_every > 0 && it % c->sort_every == 0) PICARD_TRY(sort_particles(c));
@@ -301,6 +299,9 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
     PICARD_CUDA(cudaEventRecord(ev[2], c->st));
     PICARD_TRY(bc_potentials_async(c));  // a timeout surfaces through the solve's error check
     PICARD_CUDA(cudaEventRecord(ev[3], c->st));
+    // the step before has passed the count above; read it while the device has
+    // the deposit and the boundary potential to do
+    PICARD_TRY(settle(before));
     if (c->solver == PICARD_SOLVER_SPECTRAL) {
       PICARD_TRY(spec_issue(c, p.maxerr, p.maxit));
     } else {

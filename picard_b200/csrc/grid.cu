@@ -106,8 +106,12 @@ __device__ inline long long dindex(const KParams& P, int a, int b, int c) {
   return (long long)(a - 1) + DX * ((long long)(b - 1) + DY * (long long)(c - 1));
 }
 
-__global__ void bc_potentials_kernel(KParams P, int axis, const double* __restrict__ C, const double* __restrict__ D,
-                                     double* U) {
+// blockIdx.z takes the planes [z per, z per + per): on small faces the planes
+// are split over blocks, or a 32 x 32 face would keep 4 of the 148 SMs busy
+// (2.7 ms a call at 32^3).  The blocks' sums go to partial[z][face][p2][p1] and
+// are added in plane order by bc_direct_sum_kernel.
+__global__ void bc_potentials_kernel(KParams P, int axis, int per, const double* __restrict__ C,
+                                     const double* __restrict__ D, double* __restrict__ partial) {
   __shared__ double cs[kBT][kBT];
   __shared__ double d0[2 * kBT][2 * kBT + 1];
   __shared__ double d1[2 * kBT][2 * kBT + 1];
@@ -121,7 +125,8 @@ __global__ void bc_potentials_kernel(KParams P, int axis, const double* __restri
   const int p1 = blockIdx.x * kBT + tx + 1, p2 = blockIdx.y * kBT + ty + 1;  // 1-based face node
   double acc0 = 0.0, acc1 = 0.0;
   const int N1 = n1, N2 = n2;
-  for (int q = 1; q <= nn; ++q) {
+  const int q_lo = blockIdx.z * per + 1, q_hi = min(nn, q_lo + per - 1);
+  for (int q = q_lo; q <= q_hi; ++q) {
     for (int t2 = 0; t2 < (N2 + kBT - 1) / kBT; ++t2)
       for (int t1 = 0; t1 < (N1 + kBT - 1) / kBT; ++t1) {
         // charge tile: cells (q1, q2) = (t1*16 + tx + 1, t2*16 + ty + 1)
@@ -178,21 +183,56 @@ __global__ void bc_potentials_kernel(KParams P, int axis, const double* __restri
       }
   }
   if (p1 <= N1 && p2 <= N2) {
-    const double scale = 1.0 / (2.0 * kTau * kEps0);
-    long long g0, g1;
-    if (axis == 0) {
-      g0 = node_index(P, 0, p1, p2);
-      g1 = node_index(P, Nx + 1, p1, p2);
-    } else if (axis == 1) {
-      g0 = node_index(P, p1, 0, p2);
-      g1 = node_index(P, p1, Ny + 1, p2);
-    } else {
-      g0 = node_index(P, p1, p2, 0);
-      g1 = node_index(P, p1, p2, Nz + 1);
-    }
-    U[g0] = acc0 * scale;
-    U[g1] = acc1 * scale;
+    const long long face = (long long)N1 * N2, at = (long long)(p2 - 1) * N1 + (p1 - 1);
+    partial[(2LL * blockIdx.z) * face + at] = acc0;
+    partial[(2LL * blockIdx.z + 1) * face + at] = acc1;
   }
+}
+
+// U on the two faces normal to `axis`: the partial sums in plane order.
+__global__ void bc_direct_sum_kernel(KParams P, int axis, int groups, const double* __restrict__ partial, double* U) {
+  const int Nx = P.nx, Ny = P.ny, Nz = P.nz;
+  const int N1 = axis == 0 ? Ny : Nx, N2 = axis == 2 ? Ny : Nz;
+  const long long face = (long long)N1 * N2, t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= face) return;
+  const int p1 = int(t % N1) + 1, p2 = int(t / N1) + 1;
+  double a0 = 0.0, a1 = 0.0;
+#pragma unroll 8
+  for (int g = 0; g < groups; ++g) {
+    a0 += partial[2LL * g * face + t];
+    a1 += partial[(2LL * g + 1) * face + t];
+  }
+  const double scale = 1.0 / (2.0 * kTau * kEps0);
+  long long g0, g1;
+  if (axis == 0) {
+    g0 = node_index(P, 0, p1, p2);
+    g1 = node_index(P, Nx + 1, p1, p2);
+  } else if (axis == 1) {
+    g0 = node_index(P, p1, 0, p2);
+    g1 = node_index(P, p1, Ny + 1, p2);
+  } else {
+    g0 = node_index(P, p1, p2, 0);
+    g1 = node_index(P, p1, p2, Nz + 1);
+  }
+  U[g0] = a0 * scale;
+  U[g1] = a1 * scale;
+}
+
+// Plane groups of one axis: about four blocks of 256 threads per SM.
+struct DirectSplit {
+  int n1, n2, nn, bx, by, per, groups;
+};
+inline DirectSplit direct_split(const KParams& P, int axis) {
+  DirectSplit S;
+  S.n1 = axis == 0 ? P.ny : P.nx;
+  S.n2 = axis == 2 ? P.ny : P.nz;
+  S.nn = axis == 0 ? P.nx : axis == 1 ? P.ny : P.nz;
+  S.bx = (S.n1 + kBT - 1) / kBT;
+  S.by = (S.n2 + kBT - 1) / kBT;
+  const long long want = std::max<long long>(1, 148LL * 4 / ((long long)S.bx * S.by));
+  S.per = int((S.nn + std::min<long long>(want, S.nn) - 1) / std::min<long long>(want, S.nn));
+  S.groups = (S.nn + S.per - 1) / S.per;
+  return S;
 }
 
 // ------------------------------------------------------------- Jacobi
@@ -1079,18 +1119,29 @@ cudaError_t launch_finish_flux(const KParams& P, const unsigned long long* Facc,
   return cudaGetLastError();
 }
 
-cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(U, 0, sizeof(double) * P.nodes, st);
+long long bc_direct_scratch(const KParams& P) {
+  long long most = 0;
+  for (int axis = 0; axis < 3; ++axis) {
+    const DirectSplit S = direct_split(P, axis);
+    most = std::max(most, 2LL * S.groups * S.n1 * S.n2);
+  }
+  return most;
+}
+
+cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, double* scratch,
+                                 cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(U, 0, sizeof(double) * P.nodes, st);  // BCpotentials.f90:36
   if (e != cudaSuccess) return e;
   const int flows[3] = {P.xflow, P.yflow, P.zflow};
   for (int axis = 0; axis < 3; ++axis) {
     if (!flows[axis]) continue;
-    int n1 = axis == 0 ? P.ny : P.nx, n2 = axis == 2 ? P.ny : P.nz;
-    dim3 grid((n1 + kBT - 1) / kBT, (n2 + kBT - 1) / kBT);
+    const DirectSplit S = direct_split(P, axis);
     note_launch();
-    bc_potentials_kernel<<<grid, dim3(kBT, kBT), 0, st>>>(P, axis, C, D, U);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    bc_potentials_kernel<<<dim3(S.bx, S.by, S.groups), dim3(kBT, kBT), 0, st>>>(P, axis, S.per, C, D, scratch);
+    if ((e = cudaGetLastError())) return e;
+    note_launch();
+    bc_direct_sum_kernel<<<grid_for((long long)S.n1 * S.n2), kThreads, 0, st>>>(P, axis, S.groups, scratch, U);
+    if ((e = cudaGetLastError())) return e;
   }
   return cudaSuccess;
 }

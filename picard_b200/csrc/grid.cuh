@@ -85,7 +85,10 @@ JacobiCoef jacobi_coef(const KParams& P);
 cudaError_t launch_finish_deposit(const KParams& P, const unsigned long long* Nacc, double* N, double* C,
                                   cudaStream_t st);
 cudaError_t launch_finish_flux(const KParams& P, const unsigned long long* Facc, double* F, cudaStream_t st);
-cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, cudaStream_t st);
+// The direct sum; scratch: bc_direct_scratch(P) doubles.
+long long bc_direct_scratch(const KParams& P);
+cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, double* scratch,
+                                 cudaStream_t st);
 // Tensor-core BCpotentials (bcpot_tc.cu): scratch sizes (bf16 split charge,
 // FP64 per-CTA partial tiles) and the launch.
 void bcpot_tc_scratch(const KParams& P, long long* cs_elems, long long* partial_elems);
@@ -97,6 +100,18 @@ cudaError_t launch_rhs(const KParams& P, const double* C, double* b, double* par
                        cudaStream_t st);
 cudaError_t launch_sweep_f64(const KParams& P, const JacobiGeom& G, const double* Uin, double* Uout, const double* b,
                              double* partial, cudaStream_t st);
+// FP64 sweeps with the iterate resident in one thread-block cluster
+// (jacobi_cluster.cu): the plan (ctas == 0: the grid does not fit), the
+// partials per sweep, and m sweeps from Uin to Uout's interior (Uin unchanged)
+// with partial[s][cluster_partials] the squared residuals of iterate s.
+struct ClusterPlan {
+  int ctas = 0, planes = 0, npt = 0;
+  size_t smem = 0;
+};
+ClusterPlan cluster_plan(const KParams& P);
+int cluster_partials(const ClusterPlan& C);
+cudaError_t launch_sweeps_cluster(const KParams& P, const ClusterPlan& C, const double* Uin, double* Uout,
+                                  const double* b, double* partial, int m, cudaStream_t st);
 cudaError_t launch_sweep_f32(const KParams& P, const JacobiGeom& G, const float* win, float* wout, const float* r,
                              double* partial, int w_zero, cudaStream_t st);
 cudaError_t launch_anchor(const KParams& P, const JacobiGeom& G, const double* Vin, double* Vout, const float* w,

@@ -72,13 +72,12 @@ constexpr int kOutflowWordsPerBlock = 64;
 // BCoutflow split around a host read of the survivor count (for callers that
 // synchronise anyway): stage 1 marks, scans and writes m, the survivors at or
 // above the new count n', to info[0]; stage 2 fills the holes below n', by
-// pointer jumping over the window [n', n) when nxt[0] and nxt[1] (n - n' ints
-// each) are given, else by following each hole's chain (outflow.cuh).
+// pointer jumping over the window [n', n) when nxt (n - n' ints) is given, else by following each hole's chain (outflow.cuh).
 struct OutflowSplit {
   int stage;
   long long np;  // stage 2: n' (*count after stage 1)
-  int* info;     // stage 1: one int
-  int* nxt[2];   // stage 2: pointer-jumping scratch, or null
+  int* info;     // [32] stage 1: m, then the words of the jumping rounds
+  int* nxt;      // stage 2: pointer-jumping scratch, or null
 };
 // BCoutflow in place, leaving the particles in the reference's order
 // (outflow.cuh); *count receives the survivors.  wrap != 0 also applies the

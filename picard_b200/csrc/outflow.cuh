@@ -171,10 +171,16 @@ __global__ void __launch_bounds__(kOutflowThreads)
 // round replaces it by the next position's entry, so after the rounds every
 // position holds the survivor its chain ends at.  The holes below n' then
 // take the survivor at the end of the chain from q + S(q), exactly as in
-// outflow_fill_kernel.
+// outflow_fill_kernel.  (The rounds go four hops at a time and stop when nothing
+// moves, so the longest chain sets their number, not the window.)
 
-// m (the survivors in the window, = the holes below n') into info[0].
+// m (the survivors in the window, = the holes below n') into info[0]; the
+// rounds' "something moved" words info[1 ..] cleared.
 __global__ void outflow_window_kernel(const uint2* words, const int* block_offsets, const int* survivors, int* info) {
+  if (threadIdx.x > 0) {
+    info[threadIdx.x] = 0;
+    return;
+  }
   const long long np = *survivors;
   info[0] = np > 0 ? int(np - kept_through(block_offsets, np - 1, words[(np - 1) >> 5])) : 0;
 }
@@ -186,18 +192,34 @@ __global__ void outflow_jump_init_kernel(long long n, const uint2* words, const 
        x += (long long)gridDim.x * blockDim.x) {
     const uint2 w = words[x >> 5];
     if ((w.x >> (x & 31)) & 1u)
-      nxt[x - np] = int(x);
+      nxt[x - np] = ~int(x);  // the chain ends here
     else
       nxt[x - np] = int(x + (np - kept_through(block_offsets, x, w)));  // in [x, n)
   }
 }
 
-__global__ void outflow_jump_kernel(const int* __restrict__ in, int* __restrict__ out, long long n,
-                                    const int* survivors) {
+// One round, in place: every entry replaced by the one four hops on, or by the
+// complement of the survivor the chain ends at.  An entry read while another thread moves it on is
+// still an entry of the same chain, and the launch before made every entry
+// visible, so a round advances each chain at least as far as on a copy.  A
+// round in which nothing moved ends the work: the rounds after it return at
+// once (*before: the word of the round before; null in the first).
+__global__ void outflow_jump_kernel(int* nxt, long long n, const int* survivors, const int* before, int* moved) {
+  if (before && *before == 0) return;
   const long long np = *survivors;
+  volatile int* v = nxt;
+  bool any = false;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n - np;
-       i += (long long)gridDim.x * blockDim.x)
-    out[i] = in[in[i] - np];
+       i += (long long)gridDim.x * blockDim.x) {
+    const int a = v[i];
+    if (a < 0) continue;  // resolved: no look at the survivor, which many chains share
+    int d = v[a - np];
+    if (d >= 0) d = v[d - np];
+    if (d >= 0) d = v[d - np];
+    any = true;
+    v[i] = d;
+  }
+  if (__syncthreads_or(any) && threadIdx.x == 0) *moved = 1;  // one store a block: the word is shared by all
 }
 
 template <class L>
@@ -213,7 +235,7 @@ __global__ void __launch_bounds__(kOutflowThreads)
     const uint2 w = words[p >> 5];
     if ((w.x >> (p & 31)) & 1u) continue;
     const long long s = p + (np - kept_through(block_offsets, p, w));
-    const long long t = (s >= np && s < n) ? (long long)term[s - np] : -1;
+    const long long t = (s >= np && s < n) ? ~(long long)term[s - np] : -1;  // unresolved entries: negative
     if (t >= np && t < n && ((words[t >> 5].x >> (t & 31)) & 1u))
       lay.move(p, t);
     else
@@ -243,27 +265,24 @@ cudaError_t launch_outflow_inplace(const L& lay, long long n, uint2* words, int*
     if (e != cudaSuccess) return e;
     if (split) {
       note_launch();
-      outflow_window_kernel<<<1, 1, 0, st>>>(words, block_offsets, count, split->info);
+      outflow_window_kernel<<<1, 32, 0, st>>>(words, block_offsets, count, split->info);
       return cudaGetLastError();
     }
   }
-  if (split && split->nxt[0] && n > split->np) {
+  if (split && split->nxt && n > split->np) {
     const long long W = n - split->np;
     const long long want = (W + 255) / 256;
     const int g = int(want < 148LL * 16 ? want : 148LL * 16);
     note_launch();
-    outflow_jump_init_kernel<<<g, 256, 0, st>>>(n, words, block_offsets, count, split->nxt[0]);
-    int* a = split->nxt[0];
-    int* b = split->nxt[1];
-    for (long long hops = 1; hops < W; hops <<= 1) {
+    outflow_jump_init_kernel<<<g, 256, 0, st>>>(n, words, block_offsets, count, split->nxt);
+    int round = 0;
+    for (long long hops = 1; hops < W; hops <<= 2, ++round) {
       note_launch();
-      outflow_jump_kernel<<<g, 256, 0, st>>>(a, b, n, count);
-      int* t = a;
-      a = b;
-      b = t;
+      outflow_jump_kernel<<<g, 256, 0, st>>>(split->nxt, n, count, round ? split->info + round : nullptr,
+                                             split->info + round + 1);
     }
     note_launch();
-    outflow_fill_jump_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_offsets, count, a, err);
+    outflow_fill_jump_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_offsets, count, split->nxt, err);
     return cudaGetLastError();
   }
   note_launch();

@@ -72,8 +72,76 @@ int read_r2(picard_ctx* c, int count) {
   return PICARD_OK;
 }
 
+// The same walk as solve_f64 with a whole batch of sweeps per launch
+// (jacobi_cluster.cu).  A launch leaves the iterate it starts from in place, so
+// the anchor needs no copy, and the accepted iterate is rebuilt from it.
+int solve_f64_cluster(picard_ctx* c, double tol, long long smax, int maxit, long long* sweeps, bool* converged) {
+  const KParams& K = c->K;
+  const int nb = cluster_partials(c->cluster);
+  double* buf[2] = {c->U, c->U1};
+  int cur = 0;  // the anchor, iterate a, is in buf[cur]
+  PICARD_CUDA(cudaMemcpyAsync(c->U1, c->U, sizeof(double) * K.nodes, cudaMemcpyDeviceToDevice, c->st));
+  auto run = [&](int m) -> int {
+    PICARD_CUDA(launch_sweeps_cluster(K, c->cluster, buf[cur], buf[1 - cur], c->b, c->cluster_partials, m, c->st));
+    c->stats.sweep_launches += m;
+    return PICARD_OK;
+  };
+  auto keep = [&]() -> int {
+    if (cur == 1) PICARD_CUDA(cudaMemcpyAsync(c->U, c->U1, sizeof(double) * K.nodes, cudaMemcpyDeviceToDevice, c->st));
+    return PICARD_OK;
+  };
+  long long a = 0;
+  int m = 64;
+  double r2_prev = 0.0, r2_last = 0.0;
+  const double tol2 = tol * tol;
+  for (;;) {
+    const int m_eff = int(std::min<long long>(m, smax - a));
+    PICARD_CUDA(cudaEventRecord(c->ev[0], c->st));
+    PICARD_TRY(run(m_eff));
+    PICARD_CUDA(cudaEventRecord(c->ev[1], c->st));
+    PICARD_CUDA(launch_reduce_sweeps(c->cluster_partials, nb, m_eff, c->r2, c->st));
+    PICARD_TRY(read_r2(c, m_eff));
+    c->stats.sweep_ms += elapsed_ms(c, 0, 1);
+    for (int t = 0; t < m_eff; ++t) {
+      const long long d = a + t;  // sweep d + 1 measured the residual of iterate d
+      const double r2 = c->h_pinned[t];
+      if (d < 1) continue;
+      r2_prev = r2_last;
+      r2_last = r2;
+      c->last_residual = std::sqrt(r2);
+      if (d + 1 <= maxit && passes(r2, tol)) {
+        if (d > a) {
+          PICARD_TRY(run(int(d - a)));
+          cur = 1 - cur;
+        }
+        *sweeps = d;
+        *converged = true;
+        return keep();
+      }
+    }
+    a += m_eff;
+    cur = 1 - cur;
+    if (a >= smax) {
+      *sweeps = a;
+      *converged = false;
+      return keep();
+    }
+    m = next_batch(r2_prev, r2_last, tol2, c->m_max);
+  }
+}
+
 // ------------------------------------------------------------- FP64 sweeps
 int solve_f64(picard_ctx* c, double tol, long long smax, int maxit, long long* sweeps, bool* converged) {
+  if (!c->cluster_planned) {
+    c->cluster = cluster_plan(c->K);
+    if (c->cluster.ctas) {
+      void* q = nullptr;
+      PICARD_TRY(dev_alloc(c, &q, sizeof(double) * (size_t)c->m_max * cluster_partials(c->cluster)));
+      c->cluster_partials = static_cast<double*>(q);
+    }
+    c->cluster_planned = true;
+  }
+  if (c->cluster.ctas) return solve_f64_cluster(c, tol, smax, maxit, sweeps, converged);
   const KParams& K = c->K;
   const int nb = c->G.nblocks;
   double* buf[2] = {c->U, c->U1};
