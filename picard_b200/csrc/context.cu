@@ -1018,6 +1018,9 @@ int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
     c->bcpot_tensor = value;
     return PICARD_OK;
   }
+  // a sweep shape asked for by hand replaces the cluster that the tuner may have picked
+  if (option >= PICARD_OPT_SWEEP_CTAS && option <= PICARD_OPT_SWEEP_FUSED) c->cluster32 = ClusterPlan();
+  if (option == PICARD_OPT_SWEEP_R_GLOBAL) c->cluster32 = ClusterPlan();
   if (option == PICARD_OPT_SWEEP_CTAS) {
     if (value < -1) return fail(PICARD_ERR_BAD_ARG, "SWEEP_CTAS must be -1, 0 or a CTA count");
     if (value == 0) {

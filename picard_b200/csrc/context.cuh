@@ -140,6 +140,7 @@ struct picard_ctx {
   // the first solve
   picard::ClusterPlan cluster;
   bool cluster_planned = false;
+  picard::ClusterPlan cluster32;       // FP32 sweeps in one cluster; ctas == 0: not chosen by the tuner
   double* cluster_partials = nullptr;  // [m_max][cluster_partials(plan)]
   double* bc_scratch = nullptr;        // direct BCpotentials, allocated on first use
 

@@ -109,6 +109,11 @@ struct ClusterPlan {
   size_t smem = 0;
 };
 ClusterPlan cluster_plan(const KParams& P);
+// The FP32 sweeps likewise (open boundaries, zc 4): m sweeps from w = 0,
+// the last increment to wout, the partials of the tile kernels.
+ClusterPlan cluster32_plan(const KParams& P, const JacobiGeom& G);
+cudaError_t launch_sweeps32_cluster(const KParams& P, const JacobiGeom& G, const ClusterPlan& C, const float* r,
+                                    float* wout, double* partial, int m, cudaStream_t st);
 int cluster_partials(const ClusterPlan& C);
 cudaError_t launch_sweeps_cluster(const KParams& P, const ClusterPlan& C, const double* Uin, double* Uout,
                                   const double* b, double* partial, int m, cudaStream_t st);

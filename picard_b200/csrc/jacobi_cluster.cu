@@ -1,5 +1,6 @@
-// jacobi_cluster.cu -- FP64 Jacobi sweeps (CalcEpotential.f90:74-96) of a grid
-// that fits the shared memory of one thread-block cluster.
+// jacobi_cluster.cu -- Jacobi sweeps (CalcEpotential.f90:74-96) of a grid that
+// fits the shared memory of one thread-block cluster: in FP64, and on the FP32
+// increment (sweeps32_cluster_kernel, further down).
 //
 // A sweep of 32^3 nodes is a third of a microsecond of FP64 work, but 4 us as a
 // launch of its own that reads the iterate from L2.  Here one cluster of up to
@@ -24,6 +25,7 @@
 
 #include "common.cuh"
 #include "grid.cuh"
+#include "pair_tile.cuh"
 #include "stencil.cuh"
 
 namespace picard {
@@ -153,6 +155,160 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps_cluster_kernel(ClusterAr
   }
 }
 
+// ------------------------------------------------ FP32 sweeps of the increment
+//
+// The same residence for the sweeps of the F32_REFINE solver (open boundaries).
+// CTA r is tile layer r of the TMA sweep kernels, four planes.  Half a warp takes a
+// row of one 32-wide tile, a lane two x-adjacent nodes in packed FP32 pairs and
+// their planes in z order, as pair_tile_sweep_body does: every node has the
+// operations of jacobi_res_f32 / jacobi_next_f32, and a tile's partial is summed
+// the same way (FP32 down each column, the 32-lane tree, the tile's eight rows in
+// order), so the bits are those of every other sweep kernel.  A launch starts from
+// w = 0, as every round of sweeps after an anchor does.
+//
+// What bounds it: the chain of shared-memory loads, four planes and the barrier.
+// us per sweep of a 24-sweep round, here and with the tile kernel's launches:
+// 16^3 1.45 / 2.0, 24^3 1.47 / 1.95, 32^3 1.62 / 1.96.  A second row pair per half
+// warp loses (40 x 36 x 30: 2.7 / 1.95, 48 x 40 x 33: 2.6 / 2.05; with every load
+// ahead of the first store 3.4), so at most 64 tile rows per layer are taken here;
+// among the grids that qualify the launch tuner decides.
+constexpr int kCl32Planes = 4;
+constexpr int kCl32Tasks = kClThreads / 16;
+
+struct Cluster32Args {
+  Stencil S;
+  JacobiCoefF J;
+  const float* r;
+  float* wout;
+  double* partial;  // [m][nblocks]
+  int m, gx, gy, nblocks;
+};
+
+__device__ __forceinline__ void store_remote(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void store_remote(uint32_t addr, unsigned long long v) {
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+// Row pitch (floats): node i at column i + 1, so that a lane's pair (odd i, i + 1)
+// starts on 8 bytes; columns up to nx + 3 are read.
+__host__ __device__ inline int cluster32_pitch(int nx) { return (nx + 5) & ~1; }
+
+__global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster32Args A) {
+  constexpr int ZC = kCl32Planes;
+  // row sums [3][tasks] (a thread may write sweep s + 1's before another has
+  // summed those of s - 1), then w [2][ZC + 2][ny + 2][pitch] in floats
+  extern __shared__ double cl32_smem[];
+  using pair = unsigned long long;
+  const Stencil& S = A.S;
+  const int cta = blockIdx.x, ctas = gridDim.x, lane = threadIdx.x & 31;
+  const int pitch = cluster32_pitch(S.nx), area = pitch * (S.ny + 2), tasks = A.gx * S.ny;
+  const int z0 = cta * ZC, kend = min(ZC, S.nz - z0);
+  double* rows = cl32_smem;
+  float* w0 = reinterpret_cast<float*>(cl32_smem + 3 * tasks);
+  const int buf = (ZC + 2) * area;
+  for (int e = threadIdx.x; e < 2 * buf; e += kClThreads) w0[e] = 0.0f;  // ghosts and the increment itself
+  // this lane's pair: which of its two nodes exist, and r
+  const int task = threadIdx.x >> 4, j = task / A.gx + 1, i0 = (task % A.gx) * 32 + 2 * (lane & 15) + 1;
+  const bool a0 = task < tasks && i0 <= S.nx, both = a0 && i0 < S.nx;
+  const int off = j * pitch + i0 + 1;
+  pair r[ZC];
+#pragma unroll
+  for (int kk = 0; kk < ZC; ++kk) {
+    const float* p = A.r + fidx(S, i0, j, z0 + 1 + kk);
+    r[kk] = pk2(a0 && kk < kend ? p[0] : 0.0f, both && kk < kend ? p[1] : 0.0f);
+  }
+  const uint32_t base = smem_addr(w0);
+  uint32_t to_below = 0, to_above = 0;  // our plane 1 -> the halo above its ZC planes; our plane ZC -> plane 0
+  if (cta > 0) to_below = remote_addr(base, cta - 1) + uint32_t(4 * (off + (ZC + 1) * area));
+  if (cta + 1 < ctas) to_above = remote_addr(base, cta + 1) + uint32_t(4 * off);
+  const pair m2 = pk2(-2.0f, -2.0f), ix2 = pk2(A.J.idx2, A.J.idx2), iy2 = pk2(A.J.idy2, A.J.idy2),
+             iz2 = pk2(A.J.idz2, A.J.idz2), naf = pk2(-A.J.af, -A.J.af);
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  // a tile's partial of sweep s from its rows, by the last warps (they have the fewest rows)
+  auto flush = [&](int s) {
+    const int tiles = A.gx * A.gy;
+    for (int t = kClThreads - 1 - threadIdx.x; t < tiles; t += kClThreads) {
+      const int bx = t % A.gx, by = t / A.gx;
+      double v = 0.0;
+      for (int w = 0; w < 8; ++w) {
+        const int row = by * 8 + w;
+        v += row < S.ny ? rows[(s % 3) * tasks + row * A.gx + bx] : 0.0;
+      }
+      A.partial[(long long)s * A.nblocks + bx + A.gx * (by + A.gy * cta)] = v;
+    }
+  };
+  for (int s = 0; s < A.m; ++s) {
+    const float* c = w0 + (s & 1) * buf + off;
+    float* n = w0 + (1 - (s & 1)) * buf + off;
+    const uint32_t nbuf = uint32_t(4 * (1 - (s & 1)) * buf);
+    pair r2 = 0ull;  // (+0.0f, +0.0f)
+    if (a0) {
+      pair wm = *reinterpret_cast<const pair*>(c), wc = *reinterpret_cast<const pair*>(c + area);
+#pragma unroll
+      for (int kk = 0; kk < ZC; ++kk) {
+        if (kk < kend) {
+          c += area;
+          n += area;
+          const pair wp = *reinterpret_cast<const pair*>(c + area);
+          pair res = r[kk];
+          if (s > 0) {
+            const pair ym = *reinterpret_cast<const pair*>(c - pitch), yp = *reinterpret_cast<const pair*>(c + pitch);
+            const float2 f = up2(wc);
+            const pair sx = add2(pk2(f.y, c[2]), pk2(c[-1], f.x)), sy = add2(yp, ym), sz = add2(wp, wm);
+            pair lap = mul2(fma2(m2, wc, sx), ix2);
+            lap = fma2(fma2(m2, wc, sy), iy2, lap);
+            lap = fma2(fma2(m2, wc, sz), iz2, lap);
+            res = sub2(res, lap);
+          }
+          const pair v = fma2(naf, res, wc);
+          if (both) {
+            *reinterpret_cast<pair*>(n) = v;
+            if (kk == 0 && to_below) store_remote(to_below + nbuf, v);
+            if (kk == ZC - 1 && to_above) store_remote(to_above + nbuf, v);
+          } else {  // the last column of an odd row: its neighbour is a ghost
+            const float x = up2(v).x;
+            res = pk2(up2(res).x, 0.0f);
+            *n = x;
+            if (kk == 0 && to_below) store_remote(to_below + nbuf, x);
+            if (kk == ZC - 1 && to_above) store_remote(to_above + nbuf, x);
+          }
+          r2 = fma2(res, res, r2);
+          wm = wc;
+          wc = wp;
+        }
+      }
+    }
+    __syncwarp();
+    cluster_arrive();
+    if (s > 0) flush(s - 1);  // its rows are complete since the last barrier
+    // block_sum_store's 32-lane tree on 16 lanes of pairs
+    const float2 f = up2(r2);
+    double v0 = (double)f.x, v1 = (double)f.y;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      v0 += __shfl_down_sync(0xffffffffu, v0, o);
+      v1 += __shfl_down_sync(0xffffffffu, v1, o);
+    }
+    if ((lane & 15) == 0 && task < tasks) rows[(s % 3) * tasks + task] = v0 + v1;
+    __syncwarp();
+    cluster_wait();
+  }
+  __syncthreads();
+  flush(A.m - 1);
+  if (!a0) return;
+  const float* last = w0 + (A.m & 1) * buf + off;
+  for (int kk = 0; kk < kend; ++kk) {
+    float* out = A.wout + fidx(S, i0, j, z0 + 1 + kk);
+    const float* v = last + (kk + 1) * area;
+    out[0] = v[0];
+    if (both) out[1] = v[1];
+  }
+}
+
 using ClusterKernel = void (*)(ClusterArgs);
 ClusterKernel cluster_kernel(int npt) {
   return npt <= 1 ? sweeps_cluster_kernel<1> : npt <= 2 ? sweeps_cluster_kernel<2>
@@ -204,6 +360,46 @@ ClusterPlan cluster_plan(const KParams& P) {
     C = ClusterPlan();
   }
   return C;
+}
+
+// The FP32 sweeps: one CTA per tile layer (2 .. 16 of four planes), a half warp
+// per tile row of it.
+ClusterPlan cluster32_plan(const KParams& P, const JacobiGeom& G) {
+  ClusterPlan C;
+  const int ctas = (int)G.grid.z, tasks = (int)G.grid.x * P.ny;
+  if (!G.tma || G.zc != kCl32Planes || ctas < 2 || ctas > 16 || tasks > kCl32Tasks) return C;
+  C.ctas = ctas;
+  C.planes = kCl32Planes;
+  C.smem = 24 * (size_t)tasks + 8 * (size_t)(kCl32Planes + 2) * cluster32_pitch(P.nx) * (P.ny + 2);
+  static_assert(24 * kCl32Tasks + 8 * (kCl32Planes + 2) * 68 * (kCl32Tasks + 2) <= kClSmem, "at most 64 x 64 nodes");
+  auto k = sweeps32_cluster_kernel;
+  cudaLaunchAttribute at[1];
+  const cudaLaunchConfig_t cfg = cluster_config(C, at, nullptr);
+  int fit = 0;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClSmem) == cudaSuccess &&
+      (ctas <= 8 || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+      cudaOccupancyMaxActiveClusters(&fit, k, &cfg) == cudaSuccess && fit > 0)
+    return C;
+  (void)cudaGetLastError();
+  return ClusterPlan();
+}
+
+cudaError_t launch_sweeps32_cluster(const KParams& P, const JacobiGeom& G, const ClusterPlan& C, const float* r,
+                                    float* wout, double* partial, int m, cudaStream_t st) {
+  Cluster32Args A;
+  A.S = make_stencil(P);
+  A.J = jacobi_coef_f(P);
+  A.r = r;
+  A.wout = wout;
+  A.partial = partial;
+  A.m = m;
+  A.gx = (int)G.grid.x;
+  A.gy = (int)G.grid.y;
+  A.nblocks = G.nblocks;
+  cudaLaunchAttribute at[1];
+  cudaLaunchConfig_t cfg = cluster_config(C, at, st);
+  note_launch();
+  return cudaLaunchKernelEx(&cfg, sweeps32_cluster_kernel, A);
 }
 
 int cluster_partials(const ClusterPlan& C) { return C.ctas * kClWarps; }

@@ -238,6 +238,12 @@ int run_sweeps_single(picard_ctx* c, int count, int rsel, double* partial_base, 
   const KParams& K = c->K;
   const int nb = c->G.nblocks;
   float* R[2] = {c->r, c->r + f32_elems(K)};
+  if (c->cluster32.ctas) {
+    const int out = 1 - *wcur;
+    PICARD_CUDA(launch_sweeps32_cluster(K, c->G, c->cluster32, R[rsel], c->w[out], partial_base, count, c->st));
+    *wcur = out;
+    return PICARD_OK;
+  }
   if (c->G.res) {
     // one resident launch at a time on the device: its CTAs must all be
     // resident together, which another cooperative grid could prevent
@@ -481,8 +487,8 @@ extern "C" int picard_gpu_calc_epotential(picard_ctx* c, double maxerr, int32_t 
 // stages, k up to the kernel's occupancy; or one stage at full occupancy),
 // each with and without programmatic dependent launch; or the
 // register-resident sweep with each CTA shape whose grid fits on the device
-// at once -- by timing a short run of sweeps of each candidate on this
-// context's own buffers.  PICARD_TUNE_LOG=1 prints the
+// at once; or all sweeps of a round in one cluster where the grid fits it -- by
+// timing a short run of sweeps of each candidate on this context's own buffers.  PICARD_TUNE_LOG=1 prints the
 // timings to stderr.  The shape does not change a
 // single bit of the results, so the choice is free to differ from process to
 // process.  Choices are cached per (grid, tile depth, device) for the life of
@@ -496,11 +502,13 @@ struct SweepShape {
   int pairs;    // TMA sweep: 1 the x-pair kernel
   int fused2;   // x-pair sweeps two per launch
   int rglobal;  // x-pair sweep, one CTA per tile: r from global memory
+  int cluster = 0;  // every sweep of a round in one cluster (jacobi_cluster.cu)
 };
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int, int>, SweepShape> g_tuned;
 
 int apply_shape(picard_ctx* c, const SweepShape& sh) {
+  c->cluster32 = sh.cluster ? cluster32_plan(c->K, c->G) : ClusterPlan();
   c->G.ctas = sh.ctas;
   c->G.pdl = sh.pdl;
   c->G.stages = sh.stages;
@@ -602,13 +610,20 @@ int tune_sweep(picard_ctx* c, bool fresh) {
     JacobiGeom g = c->G;
     if (resident_plan(c->K, g, q)) cand.push_back({0, 0, 1, q + 1, 0, 0, 0});
   }
+  if (cluster32_plan(c->K, c->G).ctas) cand.push_back({0, 1, 1, 0, c->K.nx > 32 ? 1 : 0, 0, 0, 1});
   constexpr int kReps = 24;
   std::vector<float> best(cand.size(), 1e30f);
   for (int round = 0; round < 2; ++round) {
     for (size_t q = 0; q < cand.size(); ++q) {
       PICARD_TRY(apply(cand[q]));
       float ms = 0.0f;
-      if (c->G.res) {
+      if (c->cluster32.ctas) {
+        PICARD_CUDA(launch_sweeps32_cluster(c->K, c->G, c->cluster32, c->r, c->w[0], c->partials, 2, c->st));
+        PICARD_CUDA(cudaEventRecord(c->ev[0], c->st));
+        PICARD_CUDA(launch_sweeps32_cluster(c->K, c->G, c->cluster32, c->r, c->w[0], c->partials, kReps, c->st));
+        PICARD_CUDA(cudaEventRecord(c->ev[1], c->st));
+        PICARD_CUDA(cudaEventSynchronize(c->ev[1]));
+      } else if (c->G.res) {
         std::lock_guard<std::mutex> lk(g_resident_mu);
         PICARD_CUDA(launch_sweeps_resident(c->K, c->G, c->r, nullptr, c->w[0], c->res_faces, c->res_bar,
                                            c->partials, 2, 1, c->d_err, c->st));
@@ -647,7 +662,10 @@ int tune_sweep(picard_ctx* c, bool fresh) {
     if (best[q] < best[pick]) pick = q;
   if (const char* v = std::getenv("PICARD_TUNE_LOG"); v && *v && *v != '0') {
     for (size_t q = 0; q < cand.size(); ++q) {
-      if (cand[q].res)
+      if (cand[q].cluster)
+        std::fprintf(stderr, "picard sweep tune %dx%dx%d zc=%d: one cluster  %.3f us%s\n", c->K.nx, c->K.ny, c->K.nz,
+                     c->G.zc, best[q] * 1e3, q == pick ? "  <- picked" : "");
+      else if (cand[q].res)
         std::fprintf(stderr, "picard sweep tune %dx%dx%d zc=%d: resident shape %d  %.3f us%s\n", c->K.nx, c->K.ny,
                      c->K.nz, c->G.zc, cand[q].res - 1, best[q] * 1e3, q == pick ? "  <- picked" : "");
       else
