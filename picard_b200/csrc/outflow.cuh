@@ -25,7 +25,10 @@
 //        a thread's items before any is tested, so the loads overlap);
 //   bool keep_wrap(long long p, Key key, int wrap)  -- the BCoutflow test of
 //        particle p; when wrap != 0 also wraps a survivor across periodic faces;
-//   void move(long long dst, long long src).
+//   void move(long long dst, long long src);
+//   kQuads  -- whether the keys are words that are read four at a time (16-byte
+//        aligned), with bool plain(uint32_t key): kept without a look at
+//        anything else (keep_wrap is asked about the others only).
 #pragma once
 
 #include "common.cuh"
@@ -39,6 +42,24 @@ constexpr int kOutflowItems = 8;
 constexpr int kOutflowTile = kOutflowThreads * kOutflowItems;  // particles per block
 constexpr int kOutflowWords = kOutflowTile / 32;               // keep words per block
 static_assert(kOutflowWords == kOutflowWordsPerBlock, "keep words per block");
+
+// The block's keep words and its survivors, by its first warp.
+__device__ __forceinline__ void mark_words(const unsigned* bits, uint2* words, int* block_counts) {
+  const int lane = threadIdx.x;
+  const unsigned b0 = bits[2 * lane], b1 = bits[2 * lane + 1];
+  const int c0 = __popc(b0), v = c0 + __popc(b1);
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const int before = x - v;
+  uint2* w = words + (long long)blockIdx.x * kOutflowWords;
+  w[2 * lane] = make_uint2(b0, unsigned(before));
+  w[2 * lane + 1] = make_uint2(b1, unsigned(before + c0));
+  if (lane == 31) block_counts[blockIdx.x] = x;
+}
 
 // Item q of thread t is particle base + 256 q + t, so word 8 q + warp of the
 // block holds the ballot of item q of that warp: bit l is particle 32 w + l.
@@ -62,21 +83,74 @@ __global__ void __launch_bounds__(kOutflowThreads)
     if (lane == 0) bits[q * (kOutflowThreads / 32) + warp] = m;
   }
   __syncthreads();
-  if (warp == 0) {
-    const unsigned b0 = bits[2 * lane], b1 = bits[2 * lane + 1];
-    const int c0 = __popc(b0), v = c0 + __popc(b1);
-    int x = v;
+  if (warp == 0) mark_words(bits, words, block_counts);
+}
+
+// The same for keys of one word, of which nearly all are plain: the others of a
+// tile are listed in shared memory and tested side by side.  What bounds it is
+// the read of the keys and then, dependent on it, of the outer particles' offsets,
+// for which outflow_mark_kernel waited once per vote.  us there and here: 268 M
+// particles 417 and 316 (its bytes at the copy bandwidth: 161), 11.9 M 31.5 and
+// 24.1, 16 runs of 33 k to 3 M 29 and 22 a run.  Slower still: the keys in the list
+// too and four tests a thread at a time (38 registers and 17 KB a block: 357), a
+// block over several tiles with the next one's keys ahead (665), a vote per quad
+// with half a tile per warp (375, and 22 instead of 5 on small grids).
+template <class L>
+__global__ void __launch_bounds__(kOutflowThreads)
+    outflow_mark_quad_kernel(L lay, long long n, uint2* words, int* block_counts, int wrap) {
+  static_assert(kOutflowItems == 8 && kOutflowWords == 64, "two quads a thread, two words a lane of the first warp");
+  __shared__ unsigned bits[kOutflowWords];
+  __shared__ unsigned short outer[kOutflowTile];  // particles of the tile that are not plain
+  __shared__ int listed;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long base = (long long)blockIdx.x * kOutflowTile;
+  if (threadIdx.x < kOutflowWords) {
+    const long long left = n - base - 32 * threadIdx.x;
+    bits[threadIdx.x] = left >= 32 ? 0xffffffffu : left > 0 ? (1u << int(left)) - 1u : 0u;
+  }
+  if (threadIdx.x == 0) listed = 0;
+  uint4 key[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const long long p = base + q * (kOutflowTile / 2) + 4 * threadIdx.x;
+    if (p + 3 < n) {
+      key[q] = *reinterpret_cast<const uint4*>(lay.keys() + p);
+    } else if (p < n) {  // the last, partial quad; a key past the end is never listed
+      key[q] = make_uint4(lay.load_key(p), p + 1 < n ? lay.load_key(p + 1) : 0u, p + 2 < n ? lay.load_key(p + 2) : 0u, 0u);
+    }
+  }
+  unsigned mine = 0u;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const long long left = n - (base + q * (kOutflowTile / 2) + 4 * threadIdx.x);
+    mine |= unsigned((left > 0 && !lay.plain(key[q].x)) | (left > 1 && !lay.plain(key[q].y)) << 1 |
+                     (left > 2 && !lay.plain(key[q].z)) << 2 | (left > 3 && !lay.plain(key[q].w)) << 3)
+            << (4 * q);
+  }
+  __syncthreads();
+  if (__any_sync(0xffffffffu, mine != 0u)) {
+    const int c = __popc(mine);
+    int at = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const int y = __shfl_up_sync(0xffffffffu, at, o);
+      if (lane >= o) at += y;
     }
-    const int before = x - v;
-    uint2* w = words + (long long)blockIdx.x * kOutflowWords;
-    w[2 * lane] = make_uint2(b0, unsigned(before));
-    w[2 * lane + 1] = make_uint2(b1, unsigned(before + c0));
-    if (lane == 31) block_counts[blockIdx.x] = x;
+    int first = 0;
+    if (lane == 31) first = atomicAdd(&listed, at);
+    at += __shfl_sync(0xffffffffu, first, 31) - c;
+    for (unsigned m = mine; m; m &= m - 1) {
+      const int e = __ffs(m) - 1;
+      outer[at++] = (unsigned short)((e >> 2) * (kOutflowTile / 2) + 4 * threadIdx.x + (e & 3));
+    }
   }
+  __syncthreads();
+  for (int e = threadIdx.x; e < listed; e += kOutflowThreads) {
+    const int o = outer[e];
+    if (!lay.keep_wrap(base + o, lay.load_key(base + o), wrap)) atomicAnd(&bits[o >> 5], ~(1u << (o & 31)));
+  }
+  __syncthreads();
+  if (warp == 0) mark_words(bits, words, block_counts);
 }
 
 // Survivors among particles 0 .. q (q < n); w = the keep word of q.
@@ -166,10 +240,10 @@ __global__ void __launch_bounds__(kOutflowThreads)
 // removed -- a chain steps through the window ~(n - n') / m times (m
 // survivors in the window), each step a dependent pair of loads, and the
 // longest chain sets the time.  The same chains are then resolved in
-// ceil(log2(n - n')) parallel rounds instead: every window position x holds
-// the next position of its chain, x + S(x) (itself for a survivor), and each
-// round replaces it by the next position's entry, so after the rounds every
-// position holds the survivor its chain ends at.  The holes below n' then
+// parallel rounds instead: every window position x holds the next position of
+// its chain, x + S(x) (for a survivor the complement of x), and each round
+// replaces it by the entry four hops on, so after the rounds every position
+// holds the complement of the survivor its chain ends at.  The holes below n' then
 // take the survivor at the end of the chain from q + S(q), exactly as in
 // outflow_fill_kernel.  (The rounds go four hops at a time and stop when nothing
 // moves, so the longest chain sets their number, not the window.)
@@ -260,7 +334,10 @@ cudaError_t launch_outflow_inplace(const L& lay, long long n, uint2* words, int*
   const int nb = int((n + kOutflowTile - 1) / kOutflowTile);
   if (!split || split->stage == 1) {
     note_launch();
-    outflow_mark_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_counts, wrap);
+    if constexpr (L::kQuads)
+      outflow_mark_quad_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_counts, wrap);
+    else
+      outflow_mark_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_counts, wrap);
     cudaError_t e = launch_scan_int(block_counts, block_offsets, nb, count, block_offsets + nb + 1, st);
     if (e != cudaSuccess) return e;
     if (split) {

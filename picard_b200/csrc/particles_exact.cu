@@ -531,6 +531,7 @@ struct OutflowF64 {
   KParams P;
   PartF64 a;
   using Key = double3;
+  static constexpr bool kQuads = false;
   __device__ Key load_key(long long p) const { return make_double3(a.x[p], a.y[p], a.z[p]); }
   __device__ bool keep_wrap(long long p, double3 key, int wrap) const {
     const double x = key.x, y = key.y, z = key.z;

@@ -229,12 +229,16 @@ struct OutflowC32 {
   KParams P;
   PartC32 a;
   using Key = uint32_t;
+  static constexpr bool kQuads = true;
+  __device__ const uint32_t* keys() const { return a.cell; }
   __device__ Key load_key(long long p) const { return a.cell[p]; }
-  __device__ bool keep_wrap(long long p, uint32_t cell, int wrap) const {
-    // interior cells 1 .. n-1 on every axis (packed as 2 .. n): kept, no wrap
+  // interior cells 1 .. n-1 on every axis (packed as 2 .. n): kept, no wrap
+  __device__ bool plain(uint32_t cell) const {
     const uint32_t cx = cell & kCellMaskX, cy = (cell >> kCellBitsX) & kCellMaskY,
                    cz = cell >> (kCellBitsX + kCellBitsY);
-    if (cx - 2u < uint32_t(P.nx - 1) && cy - 2u < uint32_t(P.ny - 1) && cz - 2u < uint32_t(P.nz - 1)) return true;
+    return cx - 2u < uint32_t(P.nx - 1) && cy - 2u < uint32_t(P.ny - 1) && cz - 2u < uint32_t(P.nz - 1);
+  }
+  __device__ bool keep_wrap(long long p, uint32_t cell, int wrap) const {
     C32 c;
     unpack_cell(cell, c.i, c.j, c.k);
     c.f[0] = (c.i == 0 || c.i == P.nx) ? a.fx[p] : kOffHalf;
