@@ -773,7 +773,7 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
     else if (q != PICARD_OK) return q;
     return PICARD_OK;
   };
-  for (int r = 0; r < n; ++r) ctxs[r]->spec.pending = false;
+  for (int r = 0; r < n; ++r) ctxs[r]->spec.collected = ctxs[r]->spec.queued;
   auto body = [&]() -> int {
     for (int32_t step = 1; step <= nsteps; ++step) {
       tick = now();

@@ -28,6 +28,7 @@
 #include <type_traits>
 #include <vector>
 
+#include "chain.cuh"
 #include "context.cuh"
 
 namespace picard {
@@ -471,6 +472,7 @@ struct FftJobs3 {
 };
 template <int STAGE, int LOG>
 __global__ void __launch_bounds__(kFftThreads, 2) bcfft_run_kernel(const __grid_constant__ FftJobs3 T) {
+  chain_begin();
   const long long b = blockIdx.x;
   int q = 0;
   while (q + 1 < T.n && T.j[q + 1].start[STAGE] <= b) ++q;
@@ -732,11 +734,10 @@ int stage_log(const FaceGeom& F, int stage) { return stage == 0 || stage == 3 ? 
 
 template <int STAGE>
 int launch_run_stage(FftJobs3& T, int log, long long blocks, cudaStream_t st) {
-  note_launch();
   return with_log(log, [&](auto lg) {
     constexpr int LOG = decltype(lg)::value;
-    bcfft_run_kernel<STAGE, LOG><<<(unsigned)blocks, kFftThreads, fsmem<LOG>(), st>>>(T);
-    return check_cuda(cudaGetLastError(), "bcfft_run_kernel");
+    return check_cuda(launch_chained(bcfft_run_kernel<STAGE, LOG>, (unsigned)blocks, kFftThreads, fsmem<LOG>(), st, T),
+                      "bcfft_run_kernel");
   });
 }
 // Stages [STAGE, END) of jobs [first, last) of `J`, one launch per stage and

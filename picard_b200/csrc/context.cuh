@@ -54,6 +54,10 @@ struct SpecState {
   int pad;
 };
 
+struct SpecStamps {  // behind the SpecState: device times in ns
+  unsigned long long begin, search, iterate, end;
+};
+
 // Closed-form Jacobi solve (spectral.cu): the axis bases and the compact FP64
 // interior arrays the transforms use.  Modes of an axis in the order [even |
 // odd].
@@ -65,7 +69,7 @@ struct SpectralPlan {
   SpecState* state = nullptr;
   unsigned int* counter = nullptr;              // blocks done in a reduction (re-armed by the last)
   int norm_blocks = 0;
-  bool pending = false;                         // a queued solve whose result has not been collected
+  unsigned queued = 0, collected = 0;           // solves queued and collected: at most two are under way
 };
 }  // namespace picard
 
@@ -227,8 +231,9 @@ void bcpot_fft_free(picard_ctx* c);
 long long spectral_bytes(const KParams& K);
 // Queues the whole closed-form solve on the context's stream (set-up, search,
 // iterate, periodic ghosts, copy of its SpecState to the host).
+// One more may be queued before the last is collected.
 int spec_issue(picard_ctx* c, double maxerr, int maxit);
-// After the stream has passed it: books the solve and reports its sweeps and
+// After the stream has passed it: books the oldest solve not collected and reports its sweeps and
 // status (PICARD_ERR_NOT_CONVERGED included).  Zero sweeps when none is pending.
 int spec_collect(picard_ctx* c, long long* sweeps);
 }  // namespace picard

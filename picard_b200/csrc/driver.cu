@@ -264,7 +264,7 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
       return rc;
     return PICARD_OK;
   };
-  c->spec.pending = false;
+  c->spec.collected = c->spec.queued;
   for (int32_t it = iter_start + 1; it <= iter_end; ++it) {
     const cudaEvent_t* ev = c->pev + 6 * (it & 1);
     const cudaEvent_t* before = c->pev + 6 * (1 - (it & 1));
@@ -299,9 +299,6 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
     PICARD_CUDA(cudaEventRecord(ev[2], c->st));
     PICARD_TRY(bc_potentials_async(c));  // a timeout surfaces through the solve's error check
     PICARD_CUDA(cudaEventRecord(ev[3], c->st));
-    // the step before has passed the count above; read it while the device has
-    // the deposit and the boundary potential to do
-    PICARD_TRY(settle(before));
     if (c->solver == PICARD_SOLVER_SPECTRAL) {
       PICARD_TRY(spec_issue(c, p.maxerr, p.maxit));
     } else {
@@ -314,6 +311,9 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
       if (sweeps_total) *sweeps_total += sw;
     }
     PICARD_CUDA(cudaEventRecord(ev[4], c->st));
+    // the step before has passed the count above; read it while the device has the
+    // whole solve to do
+    PICARD_TRY(settle(before));
     PICARD_TRY(picard_gpu_calc_efield(c));
     // AdvanceVelocity; in the CELL32 layout, when another step follows, fused
     // with that step's AdvancePosition (one pass over the particles)

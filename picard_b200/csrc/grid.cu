@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "grid.cuh"
 #include "stencil.cuh"
@@ -53,6 +54,7 @@ __device__ inline int mirror(int i, int n, int open) {
 // N_s = n2p_s * acc * 2^-40 at every node (ParticlesGridify.f90:98-121 with the
 // folds of 149-278), C = sum_s q_s N_s (288-293).
 __global__ void finish_deposit_kernel(KParams P, const unsigned long long* Nacc, double* N, double* Cout) {
+  chain_begin();
   long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P.nodes) return;
   int i = int(g % P.nxp), j = int((g / P.nxp) % P.nyp), k = int(g / ((long long)P.nxp * P.nyp));
@@ -970,7 +972,8 @@ __global__ void reduce_sweeps_kernel(const double* partial, int nb, double* r2) 
 // CalcEfield.f90:27-34 + BCfields.f90:31-90 on one rank: interior central
 // differences, open-face ghosts zero, periodic ghosts mirrored.  Writes the
 // FP64 planes (Ex, Ey, Ez) and the FP32 float4 copy used by the CELL32 gather.
-__global__ void efield_kernel(KParams P, const double* __restrict__ U, double* E, float4* E32) {
+__global__ void efield_kernel(KParams P, const double* U, double* E, float4* E32) {
+  chain_begin();
   long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P.nodes) return;
   int i = int(g % P.nxp), j = int((g / P.nxp) % P.nyp), k = int(g / ((long long)P.nxp * P.nyp));
@@ -1108,9 +1111,7 @@ JacobiCoefF jacobi_coef_f(const KParams& P) {
 
 cudaError_t launch_finish_deposit(const KParams& P, const unsigned long long* Nacc, double* N, double* C,
                                   cudaStream_t st) {
-  note_launch();
-  finish_deposit_kernel<<<grid_for(P.nodes), kThreads, 0, st>>>(P, Nacc, N, C);
-  return cudaGetLastError();
+  return launch_chained(finish_deposit_kernel, grid_for(P.nodes), kThreads, 0, st, P, Nacc, N, C);
 }
 
 cudaError_t launch_finish_flux(const KParams& P, const unsigned long long* Facc, double* F, cudaStream_t st) {
@@ -1442,9 +1443,7 @@ cudaError_t launch_reduce_sweeps(const double* partial, int nb, int m, double* r
 }
 
 cudaError_t launch_efield(const KParams& P, const double* U, double* E, float4* E32, cudaStream_t st) {
-  note_launch();
-  efield_kernel<<<grid_for(P.nodes), kThreads, 0, st>>>(P, U, E, E32);
-  return cudaGetLastError();
+  return launch_chained(efield_kernel, grid_for(P.nodes), kThreads, 0, st, P, U, E, E32);
 }
 
 cudaError_t launch_bc_fields(const KParams& P, double* E, float4* E32, cudaStream_t st) {

@@ -31,6 +31,7 @@
 //        anything else (keep_wrap is asked about the others only).
 #pragma once
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -66,6 +67,7 @@ __device__ __forceinline__ void mark_words(const unsigned* bits, uint2* words, i
 template <class L>
 __global__ void __launch_bounds__(kOutflowThreads)
     outflow_mark_kernel(L lay, long long n, uint2* words, int* block_counts, int wrap) {
+  chain_begin();
   __shared__ unsigned bits[kOutflowWords];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long base = (long long)blockIdx.x * kOutflowTile;
@@ -98,6 +100,7 @@ __global__ void __launch_bounds__(kOutflowThreads)
 template <class L>
 __global__ void __launch_bounds__(kOutflowThreads)
     outflow_mark_quad_kernel(L lay, long long n, uint2* words, int* block_counts, int wrap) {
+  chain_begin();
   static_assert(kOutflowItems == 8 && kOutflowWords == 64, "two quads a thread, two words a lane of the first warp");
   __shared__ unsigned bits[kOutflowWords];
   __shared__ unsigned short outer[kOutflowTile];  // particles of the tile that are not plain
@@ -116,7 +119,8 @@ __global__ void __launch_bounds__(kOutflowThreads)
     if (p + 3 < n) {
       key[q] = *reinterpret_cast<const uint4*>(lay.keys() + p);
     } else if (p < n) {  // the last, partial quad; a key past the end is never listed
-      key[q] = make_uint4(lay.load_key(p), p + 1 < n ? lay.load_key(p + 1) : 0u, p + 2 < n ? lay.load_key(p + 2) : 0u, 0u);
+      key[q] = make_uint4(lay.load_key(p), p + 1 < n ? lay.load_key(p + 1) : 0u, p + 2 < n ? lay.load_key(p + 2) : 0u,
+                          0u);
     }
   }
   unsigned mine = 0u;
@@ -170,6 +174,7 @@ template <class L>
 __global__ void __launch_bounds__(kOutflowThreads)
     outflow_fill_kernel(L lay, long long n, const uint2* words, const int* block_offsets, const int* survivors,
                         int* err) {
+  chain_begin();
   const long long np = *survivors;
   const long long base = (long long)blockIdx.x * kOutflowTile;
   if (base >= np) return;
@@ -333,12 +338,15 @@ cudaError_t launch_outflow_inplace(const L& lay, long long n, uint2* words, int*
   }
   const int nb = int((n + kOutflowTile - 1) / kOutflowTile);
   if (!split || split->stage == 1) {
-    note_launch();
-    if constexpr (L::kQuads)
-      outflow_mark_quad_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_counts, wrap);
-    else
-      outflow_mark_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_counts, wrap);
-    cudaError_t e = launch_scan_int(block_counts, block_offsets, nb, count, block_offsets + nb + 1, st);
+    auto mark = [] {
+      if constexpr (L::kQuads)
+        return outflow_mark_quad_kernel<L>;
+      else
+        return outflow_mark_kernel<L>;
+    }();
+    cudaError_t e = launch_chained(mark, nb, kOutflowThreads, 0, st, lay, n, words, block_counts, wrap);
+    if (e != cudaSuccess) return e;
+    e = launch_scan_int(block_counts, block_offsets, nb, count, block_offsets + nb + 1, st);
     if (e != cudaSuccess) return e;
     if (split) {
       note_launch();
@@ -362,9 +370,7 @@ cudaError_t launch_outflow_inplace(const L& lay, long long n, uint2* words, int*
     outflow_fill_jump_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_offsets, count, split->nxt, err);
     return cudaGetLastError();
   }
-  note_launch();
-  outflow_fill_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_offsets, count, err);
-  return cudaGetLastError();
+  return launch_chained(outflow_fill_kernel<L>, nb, kOutflowThreads, 0, st, lay, n, words, block_offsets, count, err);
 }
 
 }  // namespace

@@ -11,6 +11,7 @@
 #include <climits>
 #include <cmath>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "outflow.cuh"
@@ -413,6 +414,7 @@ __device__ inline void interior_cell(const KParams& P, long long c, int& ii, int
 }
 
 __global__ void produce_count_kernel(KParams P, int iteration, int* counts) {
+  chain_begin();
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long cells = (long long)P.nx * P.ny * P.nz;
   if (c >= cells) return;
@@ -433,6 +435,7 @@ __global__ void produce_count_kernel(KParams P, int iteration, int* counts) {
 template <class Store>
 __global__ void produce_emit_kernel(KParams P, int iteration, const int* offsets, const int* count, long long capacity,
                                     int* err, Store store) {
+  chain_begin();
   long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   long long cells = (long long)P.nx * P.ny * P.nz;
   if (c >= cells) return;
@@ -581,6 +584,7 @@ inline int inflow_items(long long candidates) {
 __global__ void __launch_bounds__(kThreads) inflow_stage_kernel(KParams P, InflowTable T, InflowReach R, int iteration,
                                                                 long long total, int items, int* block_counts,
                                                                 double* stage, int8_t* stage_sp, long long stride) {
+  chain_begin();
   constexpr int kWords = kInflowItems * kThreads / 32;
   static_assert(kWords == 64, "two words per lane of the scanning warp");
   __shared__ int warp_sums[32];
@@ -645,6 +649,7 @@ __global__ void __launch_bounds__(kThreads) inflow_place_kernel(int tile, const 
                                                                 const int* count, long long capacity, int* err,
                                                                 const double* stage, const int8_t* stage_sp,
                                                                 long long stride, Store store) {
+  chain_begin();
   for (int r = threadIdx.x; r < block_counts[blockIdx.x]; r += blockDim.x) {
     const long long q = (long long)blockIdx.x * tile + r;
     const double x[3] = {stage[q], stage[q + stride], stage[q + 2 * stride]};
@@ -1281,12 +1286,11 @@ cudaError_t launch_inflow_c32(const KParams& P, const InflowTable& T, int iterat
 
 cudaError_t launch_produce_count(const KParams& P, int iteration, int* counts, cudaStream_t st) {
   long long cells = (long long)P.nx * P.ny * P.nz;
-  note_launch();
-  produce_count_kernel<<<grid_for(cells), kThreads, 0, st>>>(P, iteration, counts);
-  return cudaGetLastError();
+  return launch_chained(produce_count_kernel, grid_for(cells), kThreads, 0, st, P, iteration, counts);
 }
 
 __global__ void add_count_kernel(int* count, const int* add, long long capacity) {
+  chain_begin();
   long long v = (long long)*count + *add;
   *count = int(v < capacity ? v : capacity);
 }
@@ -1303,16 +1307,15 @@ static cudaError_t inflow_fused(const KParams& P, const InflowTable& T, int iter
   cudaError_t e;
   const int items = inflow_items(total), tile = items * kThreads;
   const long long stride = (long long)nb * tile;
-  note_launch();
-  inflow_stage_kernel<<<nb, kThreads, 0, st>>>(P, T, R, iteration, total, items, block_counts, S.x, S.sp, stride);
+  e = launch_chained(inflow_stage_kernel, nb, kThreads, 0, st, P, T, R, iteration, total, items, block_counts, S.x, S.sp,
+                     stride);
+  if (e != cudaSuccess) return e;
   e = launch_scan_int(block_counts, block_offsets, nb, block_offsets + nb, block_offsets + nb + 1, st);
   if (e != cudaSuccess) return e;
-  note_launch();
-  inflow_place_kernel<<<nb, kThreads, 0, st>>>(tile, block_counts, block_offsets, count, capacity, err, S.x, S.sp, stride,
-                                               store);
-  note_launch();
-  add_count_kernel<<<1, 1, 0, st>>>(count, block_offsets + nb, capacity);
-  return cudaGetLastError();
+  e = launch_chained(inflow_place_kernel<Store>, nb, kThreads, 0, st, tile, block_counts, block_offsets, count, capacity,
+                     err, S.x, S.sp, stride, store);
+  if (e != cudaSuccess) return e;
+  return launch_chained(add_count_kernel, 1, 1, 0, st, count, block_offsets + nb, capacity);
 }
 
 cudaError_t launch_inflow_fused_c32(const KParams& P, const InflowTable& T, int iteration, PartC32 out, int* count,
@@ -1333,23 +1336,19 @@ long long inflow_stage_slots(long long candidates) { return (long long)inflow_bl
 cudaError_t launch_produce_emit_f64(const KParams& P, int iteration, const int* offsets, PartF64 out, int* count,
                                     long long capacity, int* err, cudaStream_t st) {
   long long cells = (long long)P.nx * P.ny * P.nz;
-  note_launch();
-  produce_emit_kernel<<<grid_for(cells), kThreads, 0, st>>>(P, iteration, offsets, count, capacity, err,
-                                                            StoreF64{out});
-  note_launch();
-  add_count_kernel<<<1, 1, 0, st>>>(count, offsets + cells, capacity);
-  return cudaGetLastError();
+  cudaError_t e = launch_chained(produce_emit_kernel<StoreF64>, grid_for(cells), kThreads, 0, st, P, iteration, offsets, count,
+                                 capacity, err, StoreF64{out});
+  if (e != cudaSuccess) return e;
+  return launch_chained(add_count_kernel, 1, 1, 0, st, count, offsets + cells, capacity);
 }
 
 cudaError_t launch_produce_emit_c32(const KParams& P, int iteration, const int* offsets, PartC32 out, int* count,
                                     long long capacity, int* err, cudaStream_t st) {
   long long cells = (long long)P.nx * P.ny * P.nz;
-  note_launch();
-  produce_emit_kernel<<<grid_for(cells), kThreads, 0, st>>>(P, iteration, offsets, count, capacity, err,
-                                                            StoreC32{P, out});
-  note_launch();
-  add_count_kernel<<<1, 1, 0, st>>>(count, offsets + cells, capacity);
-  return cudaGetLastError();
+  cudaError_t e = launch_chained(produce_emit_kernel<StoreC32>, grid_for(cells), kThreads, 0, st, P, iteration, offsets, count,
+                                 capacity, err, StoreC32{P, out});
+  if (e != cudaSuccess) return e;
+  return launch_chained(add_count_kernel, 1, 1, 0, st, count, offsets + cells, capacity);
 }
 
 static int persistent_grid(long long n) {

@@ -12,6 +12,7 @@
 
 #include <cmath>
 
+#include "chain.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "outflow.cuh"
@@ -62,6 +63,7 @@ __device__ inline int block_scan_excl(int v, int& total) {
 }
 
 __global__ void scan_tiles_kernel(const int* in, int* out, int n, int* tile_sums) {
+  chain_begin();
   long long base = (long long)blockIdx.x * kScanTile + (long long)threadIdx.x * kScanItems;
   int v[kScanItems];
   int s = 0;
@@ -83,6 +85,7 @@ __global__ void scan_tiles_kernel(const int* in, int* out, int n, int* tile_sums
 }
 
 __global__ void scan_add_kernel(int* out, int n, const int* tile_offsets) {
+  chain_begin();
   long long base = (long long)blockIdx.x * kScanTile;
   int add = tile_offsets[blockIdx.x];
   for (int q = threadIdx.x; q < kScanTile; q += blockDim.x) {
@@ -889,20 +892,16 @@ int scan_scratch_ints(int n) {
 cudaError_t launch_scan_int(const int* in, int* out, int n, int* total, int* scratch, cudaStream_t st) {
   if (n <= 0) return cudaMemsetAsync(total, 0, sizeof(int), st);
   if (n <= kScanTile) {
-    note_launch();
-    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(in, out, n, total);
-    return cudaGetLastError();
+    return launch_chained(scan_tiles_kernel, 1, kScanThreads, 0, st, in, out, n, total);
   }
   int nb = (n + kScanTile - 1) / kScanTile;
   int* sums = scratch;
   int* offs = scratch + nb + 1;
-  note_launch();
-  scan_tiles_kernel<<<nb, kScanThreads, 0, st>>>(in, out, n, sums);
-  cudaError_t e = launch_scan_int(sums, offs, nb, total, offs + nb + 1, st);
+  cudaError_t e = launch_chained(scan_tiles_kernel, nb, kScanThreads, 0, st, in, out, n, sums);
   if (e != cudaSuccess) return e;
-  note_launch();
-  scan_add_kernel<<<nb, kScanThreads, 0, st>>>(out, n, offs);
-  return cudaGetLastError();
+  e = launch_scan_int(sums, offs, nb, total, offs + nb + 1, st);
+  if (e != cudaSuccess) return e;
+  return launch_chained(scan_add_kernel, nb, kScanThreads, 0, st, out, n, offs);
 }
 
 cudaError_t launch_advance_position_c32(const KParams& P, PartC32 a, long long n, double dt, cudaStream_t st) {
@@ -949,12 +948,6 @@ cudaError_t launch_deposit_c32(const KParams& P, PartC32 a, long long n, unsigne
                                unsigned long long* Facc, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (!Facc) {
-    // Eight particles per lane spread a warp's lanes over more cells (fewer
-    // bank conflicts) and flush a box less often; four where that box would be
-    // mostly empty (few particles per cell) or the array has no two chunks of
-    // eight for every resident warp.  Both, us per ParticlesGridify: 64 per
-    // cell, 67 M particles 687 against 786; 26 per cell, 11.9 M 154 / 162; 24
-    // per cell, 1.56 M 46 / 43; 10 per cell, 8.0 M 172 / 139.
     // Particles per lane.  Eight spread a warp's lanes over more cells (fewer
     // bank conflicts) and flush a box less often, four where that box would be
     // mostly empty (few particles per cell), two where the array has not two

@@ -41,7 +41,10 @@ struct F32Solve {
 
 // CalcEpotential's set-up and wrap-up around the solve loop.
 constexpr int kPinnedB2 = kMaxSweepsPerRound + 8;  // slot of ||b||^2 in ctx->h_pinned (past the r2 copies)
-constexpr int kPinnedSpec = kMaxSweepsPerRound + 16;  // slots of a queued closed-form solve's SpecState
+constexpr int kPinnedSpec = kMaxSweepsPerRound + 16;  // slots of two queued closed-form solves' SpecStates
+constexpr int kSpecSlots = 20;
+constexpr size_t kSpecBytes = sizeof(SpecState) + sizeof(SpecStamps);
+static_assert(kSpecBytes <= kSpecSlots * sizeof(double) && 16 + 2 * kSpecSlots <= 64, "the mailbox ends 64 slots on");
 struct EpotSetup {
   double bnorm = 0.0, tol = 0.0, sigma = 1.0;
   long long smax = 0;

@@ -40,6 +40,7 @@
 #include <cstring>
 #include <vector>
 
+#include "chain.cuh"
 #include "context.cuh"
 #include "picard_gpu.h"
 #include "solve_f32.cuh"
@@ -76,6 +77,16 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return t;
 }
 
+// A queued solve's times on the device's clock, behind its SpecState: start of the
+// set-up, of the search and of the iterate, and the latest end of a block of the
+// last pass.  (Events would keep the kernels on either side of them apart.)
+__device__ __forceinline__ SpecStamps* stamps_of(SpecState* state) { return reinterpret_cast<SpecStamps*>(state + 1); }
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long v;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
+  return v;
+}
+
 // b = -C/(dV eps0) and r_0 = b - L U over the interior, compact x-fastest
 // (CalcEpotential.f90:50-54, 83-92; periodic axes read the wrapped interior
 // instead of the ghost), ||b||^2, and from it, in the last block, the start of
@@ -83,11 +94,13 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 // (CalcEpotential.f90:55-61).
 template <class T>
 __global__ void __launch_bounds__(kSpecThreads) spec_begin_kernel(KParams P, double idx2, double idy2, double idz2,
-                                                                  double binv, const double* __restrict__ C,
-                                                                  const double* __restrict__ U, double* __restrict__ R,
+                                                                  double binv, const double* C,
+                                                                  const double* U, double* R,
                                                                   double maxerr, int maxit,
                                                                   double* __restrict__ partial, unsigned int* counter,
                                                                   SpecState* state) {
+  chain_begin();
+  if (blockIdx.x == 0 && threadIdx.x == 0) *stamps_of(state) = SpecStamps{global_ns(), 0, 0, 0};
   const T n = T(P.nx) * T(P.ny) * T(P.nz);
   double b2 = 0.0;
   for (T t = T(blockIdx.x) * blockDim.x + threadIdx.x; t < n; t += T(gridDim.x) * blockDim.x) {
@@ -186,11 +199,12 @@ __device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double
 // shared-memory as FP64 cycles), in-place butterflies and a pass of its own for
 // the update; 24^3: 28 us against 55 us.
 template <bool INV, bool X, bool APPLY>
-__global__ void __launch_bounds__(256, 2) spec_axis_kernel(const double* __restrict__ in, double* __restrict__ out,
+__global__ void __launch_bounds__(256, 2) spec_axis_kernel(const double* in, double* out,
                                                            const double* __restrict__ Pe,
                                                            const double* __restrict__ Po, int n, int ne, int no, int s,
-                                                           long long I, int rows, KParams P, double* __restrict__ U,
-                                                           const SpecState* __restrict__ state) {
+                                                           long long I, int rows, KParams P, double* U,
+                                                           SpecState* state) {
+  chain_begin();
   if (APPLY && state->trivial) return;  // zero sweeps: U stays
   // row strides 4 mod 16 doubles: the 16 lanes of a half-warp read 16 banks
   __shared__ double sh[2 * kAxTile * (kAxK + 4) + 2 * kAxK * (kAxTile + 4)];
@@ -339,6 +353,7 @@ __global__ void __launch_bounds__(256, 2) spec_axis_kernel(const double* __restr
           }
         }
     }
+    if (APPLY && tid == 0) atomicMax(&stamps_of(state)->end, global_ns());
   } else {
 #pragma unroll
     for (int fa = 0; fa < 4; ++fa)
@@ -435,13 +450,15 @@ __device__ void spec_advance(SpecState& Q, const double* f) {
 // fixed order; the last block to finish sums them, re-arms the counter and
 // moves the search on.  A finished search returns at once.
 template <class T>
-__global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* __restrict__ Rh, int nx, int ny,
+__global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* Rh, int nx, int ny,
                                                                   int nz, const double* __restrict__ omx,
                                                                   const double* __restrict__ omy,
                                                                   const double* __restrict__ omz,
                                                                   double* __restrict__ partial, unsigned int* counter,
                                                                   SpecState* state) {
+  chain_begin();
   if (state->done) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && stamps_of(state)->search == 0) stamps_of(state)->search = global_ns();
   const long long d0 = state->d0, step = state->step;
   const int count = state->count, doubling = state->phase == kSpecDoubling;
   const double g2_skip = state->g2_skip;
@@ -533,11 +550,13 @@ __global__ void __launch_bounds__(kSpecThreads) spec_norms_kernel(const double* 
 // -expm1(d log1p(-omg))/omg (no cancellation near g = 1); a mode with
 // omg == 0 (every axis periodic, the constant mode) takes d.
 template <class T>
-__global__ void spec_scale_kernel(double* __restrict__ Rh, int nx, int ny, int nz, const double* __restrict__ omx,
+__global__ void spec_scale_kernel(double* Rh, int nx, int ny, int nz, const double* __restrict__ omx,
                                   const double* __restrict__ omy, const double* __restrict__ omz, double af,
-                                  const SpecState* __restrict__ state) {
+                                  SpecState* state) {
+  chain_begin();
   const long long d = state->d;
   if (state->trivial) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) stamps_of(state)->iterate = global_ns();
   const T n = T(nx) * T(ny) * T(nz);
   for (T q = T(blockIdx.x) * blockDim.x + threadIdx.x; q < n; q += T(gridDim.x) * blockDim.x) {
     int mx, my, mz;
@@ -628,20 +647,17 @@ cudaError_t axis_pass(picard_ctx* c, int d, bool forward, const double* in, doub
   const int rows = d == 0 ? ny * nz : 0;
   auto tiles = [](long long v) { return (unsigned)((v + kAxTile - 1) / kAxTile); };
   const dim3 grid = d == 0 ? dim3(tiles(A.ne), tiles(rows)) : dim3(tiles(I), tiles(A.ne), d == 1 ? nz : 1);
-  note_launch();
   if (d == 0 && forward)
-    spec_axis_kernel<false, true, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
-                                                                  c->K, nullptr, S.state);
-  else if (d == 0)
-    spec_axis_kernel<true, true, true><<<grid, 256, 0, c->st>>>(in, nullptr, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
-                                                                c->K, c->U, S.state);
-  else if (forward)
-    spec_axis_kernel<false, false, false><<<grid, 256, 0, c->st>>>(in, out, A.Pe, A.Po, n, A.ne, A.no, A.s, I, rows,
-                                                                   c->K, nullptr, S.state);
-  else
-    spec_axis_kernel<true, false, false><<<grid, 256, 0, c->st>>>(in, out, A.PeT, A.PoT, n, A.ne, A.no, A.s, I, rows,
-                                                                  c->K, nullptr, S.state);
-  return cudaGetLastError();
+    return launch_chained(spec_axis_kernel<false, true, false>, grid, 256, 0, c->st, in, out, A.PeT, A.PoT, n, A.ne, A.no,
+                          A.s, I, rows, c->K, nullptr, S.state);
+  if (d == 0)
+    return launch_chained(spec_axis_kernel<true, true, true>, grid, 256, 0, c->st, in, nullptr, A.Pe, A.Po, n, A.ne, A.no,
+                          A.s, I, rows, c->K, c->U, S.state);
+  if (forward)
+    return launch_chained(spec_axis_kernel<false, false, false>, grid, 256, 0, c->st, in, out, A.Pe, A.Po, n, A.ne, A.no,
+                          A.s, I, rows, c->K, nullptr, S.state);
+  return launch_chained(spec_axis_kernel<true, false, false>, grid, 256, 0, c->st, in, out, A.PeT, A.PoT, n, A.ne, A.no,
+                        A.s, I, rows, c->K, nullptr, S.state);
 }
 
 // Forward: Qz Qy Qx of T[0] into T[1] (x, y, z passes ping-ponging T[0] and
@@ -708,7 +724,7 @@ int spectral_alloc(picard_ctx* c) {
   S.norm_blocks = std::min(stream_blocks(n), 148 * 4);
   PICARD_TRY(dev_alloc(c, &p, sizeof(double) * (size_t)S.norm_blocks * kSpecPoints));
   S.partial = static_cast<double*>(p);
-  PICARD_TRY(dev_alloc(c, &p, sizeof(SpecState)));
+  PICARD_TRY(dev_alloc(c, &p, kSpecBytes));
   S.state = static_cast<SpecState*>(p);
   PICARD_TRY(dev_alloc(c, &p, sizeof(unsigned int)));  // zeroed
   S.counter = static_cast<unsigned int*>(p);
@@ -728,57 +744,39 @@ int spec_issue(picard_ctx* c, double maxerr, int maxit) {
   const JacobiCoef J = jacobi_coef(K);
   const double ix = 1.0 / J.dx2, iy = 1.0 / J.dy2, iz = 1.0 / J.dz2, binv = 1.0 / (K.dV * kEps0);
   const int nb = stream_blocks(n);  // at most 32 norm_blocks partials
-  PICARD_CUDA(cudaEventRecord(c->ev[0], c->st));
-  note_launch();
-  if (fits32(n))
-    spec_begin_kernel<unsigned><<<nb, kSpecThreads, 0, c->st>>>(K, ix, iy, iz, binv, c->C, c->U, S.T[0], maxerr, maxit,
-                                                                 S.partial, S.counter, S.state);
-  else
-    spec_begin_kernel<long long><<<nb, kSpecThreads, 0, c->st>>>(K, ix, iy, iz, binv, c->C, c->U, S.T[0], maxerr, maxit,
-                                                                  S.partial, S.counter, S.state);
-  PICARD_CUDA(cudaGetLastError());
+  if (S.queued - S.collected > 1) return fail(PICARD_ERR_STATE, "two closed-form solves are waiting to be collected");
+  const int slot = S.queued & 1;
+  auto* begin = fits32(n) ? spec_begin_kernel<unsigned> : spec_begin_kernel<long long>;
+  PICARD_CUDA(launch_chained(begin, nb, kSpecThreads, 0, c->st, K, ix, iy, iz, binv, c->C, c->U, S.T[0], maxerr, maxit,
+                             S.partial, S.counter, S.state));
   PICARD_CUDA(transform(c, true));
-  PICARD_CUDA(cudaEventRecord(c->ev[1], c->st));
-  for (int e = max_evaluations(maxit); e > 0; --e) {
-    note_launch();
-    if (fits32(n))
-      spec_norms_kernel<unsigned><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
-                                                                              S.om[2], S.partial, S.counter, S.state);
-    else
-      spec_norms_kernel<long long><<<S.norm_blocks, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
-                                                                               S.om[2], S.partial, S.counter, S.state);
-    PICARD_CUDA(cudaGetLastError());
-  }
-  PICARD_CUDA(cudaEventRecord(c->ev[2], c->st));
-  note_launch();
-  if (fits32(n))
-    spec_scale_kernel<unsigned><<<nb, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1], S.om[2],
-                                                                 J.af, S.state);
-  else
-    spec_scale_kernel<long long><<<nb, kSpecThreads, 0, c->st>>>(S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1], S.om[2],
-                                                                  J.af, S.state);
-  PICARD_CUDA(cudaGetLastError());
+  auto* norms = fits32(n) ? spec_norms_kernel<unsigned> : spec_norms_kernel<long long>;
+  for (int e = max_evaluations(maxit); e > 0; --e)
+    PICARD_CUDA(launch_chained(norms, S.norm_blocks, kSpecThreads, 0, c->st, S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1],
+                               S.om[2], S.partial, S.counter, S.state));
+  auto* scale = fits32(n) ? spec_scale_kernel<unsigned> : spec_scale_kernel<long long>;
+  PICARD_CUDA(launch_chained(scale, nb, kSpecThreads, 0, c->st, S.T[1], K.nx, K.ny, K.nz, S.om[0], S.om[1], S.om[2],
+                             J.af, S.state));
   PICARD_CUDA(transform(c, false));
-  PICARD_CUDA(cudaEventRecord(c->ev[3], c->st));
   PICARD_CUDA(launch_refresh_periodic(c->K, c->U, c->st));
-  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned + kPinnedSpec, S.state, sizeof(SpecState), cudaMemcpyDeviceToHost, c->st));
-  c->stats.d2h_bytes += sizeof(SpecState);
-  S.pending = true;
+  PICARD_CUDA(cudaMemcpyAsync(c->h_pinned + kPinnedSpec + slot * kSpecSlots, S.state, kSpecBytes,
+                              cudaMemcpyDeviceToHost, c->st));
+  c->stats.d2h_bytes += kSpecBytes;
+  ++S.queued;
   return PICARD_OK;
 }
 
 int spec_collect(picard_ctx* c, long long* sweeps) {
   *sweeps = 0;
-  if (!c->spec.pending) return PICARD_OK;
-  c->spec.pending = false;
+  if (c->spec.queued == c->spec.collected) return PICARD_OK;
+  const int slot = c->spec.collected++ & 1;
   SpecState Q;
-  std::memcpy(&Q, c->h_pinned + kPinnedSpec, sizeof(Q));
-  float f0 = 0.f, f1 = 0.f;
-  cudaEventElapsedTime(&f0, c->ev[0], c->ev[1]);
-  cudaEventElapsedTime(&f1, c->ev[2], c->ev[3]);
+  SpecStamps ns;
+  std::memcpy(&Q, c->h_pinned + kPinnedSpec + slot * kSpecSlots, sizeof(Q));
+  std::memcpy(&ns, c->h_pinned + kPinnedSpec + slot * kSpecSlots + sizeof(Q) / sizeof(double), sizeof(ns));
   if (!Q.trivial) {
     c->stats.spectral_transforms += 2;
-    c->stats.spectral_transform_ms += f0 + f1;
+    c->stats.spectral_transform_ms += 1e-6 * double((ns.search - ns.begin) + (ns.end - ns.iterate));
   }
   *sweeps = Q.d;
   return epot_account(c, Q.bnorm, Q.trivial ? Q.bnorm : std::sqrt(Q.r2_hit), Q.smax, Q.d, Q.converged != 0);
