@@ -42,10 +42,10 @@ cudaError_t launch_inflow_c32(const KParams& P, const InflowTable& T, int iterat
 // Fused inflow (fast path): candidates are generated, advanced by dt and kept
 // only if BCoutflow would keep them; survivors are appended at *count in
 // candidate order.  block_counts holds inflow_blocks(candidates) ints,
-// block_offsets that many + 2 + scan_scratch_ints(that many).  With a
+// block_offsets that many + 2 + scan_scratch_ints(that many).  The
 // staging area (inflow_stage_slots(candidates) slots: six doubles in planes
-// of that stride and a species byte) every candidate is generated once;
-// without one (x == nullptr) twice, counted and then emitted.
+// of that stride and a species byte) takes the survivors until their places are
+// known, so that every candidate is generated once.
 struct InflowStage {
   double* x = nullptr;
   int8_t* sp = nullptr;

@@ -278,9 +278,10 @@ __global__ void outflow_jump_init_kernel(long long n, const uint2* words, const 
 }
 
 // One round, in place: every entry replaced by the one four hops on, or by the
-// complement of the survivor the chain ends at.  An entry read while another thread moves it on is
-// still an entry of the same chain, and the launch before made every entry
-// visible, so a round advances each chain at least as far as on a copy.  A
+// complement of the survivor the chain ends at.  An entry read while another
+// thread moves it on is still an entry of the same chain, and the launch before
+// made every entry visible, so a round advances each chain at least as far as on a
+// copy.  A
 // round in which nothing moved ends the work: the rounds after it return at
 // once (*before: the word of the round before; null in the first).
 __global__ void outflow_jump_kernel(int* nxt, long long n, const int* survivors, const int* before, int* moved) {
