@@ -594,9 +594,9 @@ __global__ void deposit_c32_kernel(KParams P, PartC32 a, long long n, unsigned l
 // are exact and order-independent: N is bit-identical to the warp-aggregated
 // kernel's.
 //
-// What bounds it is the shared-memory pipe (16 atomics per particle, each
-// warp-level atomic taking as many wavefronts as lanes meet in one bank) and
-// instruction issue.  So
+// What bounds it is the shared-memory pipe (93 % busy at 64 per cell: 16 atomics
+// per particle, four wavefronts per warp-level atomic, more where lanes meet in
+// one bank) and instruction issue (52 %).  So
 // - a lane takes PER consecutive particles (16-byte loads) rather than every
 //   32nd: at one time the lanes stand in several cells;
 // - lane l visits the eight corners in the order q ^ (l & 7), so lanes that
