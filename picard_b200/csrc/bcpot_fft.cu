@@ -770,7 +770,7 @@ int bc_potentials_fft(picard_ctx* c) {
   PICARD_TRY(bcpot_fft_alloc(c));
   BcFft* B = c->bcfft;
   if (!B->ready) PICARD_TRY(prepare(c));
-  PICARD_CUDA(cudaMemsetAsync(c->U, 0, sizeof(double) * c->K.nodes, c->st));  // BCpotentials.f90:36
+  PICARD_CUDA(launch_zero(c->U, c->K.nodes, c->st));  // BCpotentials.f90:36
   std::vector<FftJob> jobs;
   for (int a = 0; a < 3; ++a)
     if (B->ax[a].Dh) jobs.push_back(make_job(c, B->ax[a]));
@@ -826,7 +826,7 @@ int bc_potentials_batch(picard_ctx** ctxs, int n, cudaStream_t bst, cudaEvent_t*
     PICARD_TRY(bcpot_fft_alloc(c));
     BcFft* B = c->bcfft;
     if (!B->ready) PICARD_TRY(prepare(c));
-    PICARD_CUDA(cudaMemsetAsync(c->U, 0, sizeof(double) * c->K.nodes, c->st));  // BCpotentials.f90:36
+    PICARD_CUDA(launch_zero(c->U, c->K.nodes, c->st));  // BCpotentials.f90:36
     PICARD_CUDA(cudaEventRecord(rev[r], c->st));
     PICARD_CUDA(cudaStreamWaitEvent(bst, rev[r], 0));
     fft_runs.push_back(r);

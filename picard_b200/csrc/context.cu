@@ -979,7 +979,7 @@ int picard_gpu_particles_transfer(picard_ctx* c) {
 static int deposit(picard_ctx* c, bool with_flux) {
   const long long nn = c->K.nodes;
   const int S = c->prm.species;
-  PICARD_CUDA(cudaMemsetAsync(c->Nacc, 0, sizeof(unsigned long long) * nn * S, c->st));
+  PICARD_CUDA(launch_zero(c->Nacc, (long long)nn * S, c->st));
   unsigned long long* Facc = nullptr;
   if (with_flux) {
     if (!c->Facc) PICARD_TRY(dalloc(c, c->Facc, (size_t)3 * S * nn));

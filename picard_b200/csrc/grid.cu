@@ -53,6 +53,15 @@ __device__ inline int mirror(int i, int n, int open) {
 
 // N_s = n2p_s * acc * 2^-40 at every node (ParticlesGridify.f90:98-121 with the
 // folds of 149-278), C = sum_s q_s N_s (288-293).
+// n zero words of 8 bytes (p 16-byte aligned), in the chain: a copy-engine memset
+// of a small array costs some 5 us between kernels, this 1.
+__global__ void __launch_bounds__(kThreads) zero_kernel(unsigned long long* p, long long n) {
+  chain_begin();
+  const long long stride = (long long)gridDim.x * blockDim.x, first = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long q = first; q < n >> 1; q += stride) reinterpret_cast<ulonglong2*>(p)[q] = ulonglong2{0ull, 0ull};
+  if (first == 0 && (n & 1)) p[n - 1] = 0ull;
+}
+
 __global__ void finish_deposit_kernel(KParams P, const unsigned long long* Nacc, double* N, double* Cout) {
   chain_begin();
   long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1440,6 +1449,12 @@ cudaError_t launch_reduce_sweeps(const double* partial, int nb, int m, double* r
   note_launch();
   reduce_sweeps_kernel<<<m, 256, 0, st>>>(partial, nb, r2);
   return cudaGetLastError();
+}
+
+cudaError_t launch_zero(void* p, long long n, cudaStream_t st) {
+  const long long blocks = (n / 2 + kThreads - 1) / kThreads;
+  return launch_chained(zero_kernel, int(blocks < 1 ? 1 : blocks < 148 * 8 ? blocks : 148 * 8), kThreads, 0, st,
+                        static_cast<unsigned long long*>(p), n);
 }
 
 cudaError_t launch_efield(const KParams& P, const double* U, double* E, float4* E32, cudaStream_t st) {

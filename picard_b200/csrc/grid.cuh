@@ -125,6 +125,8 @@ cudaError_t launch_finalize(const KParams& P, const double* V, const float* w, d
                             cudaStream_t st);
 cudaError_t launch_refresh_periodic(const KParams& P, double* U, cudaStream_t st);
 cudaError_t launch_reduce_sweeps(const double* partial, int nb, int m, double* r2, cudaStream_t st);
+// n words of 8 bytes from p (16-byte aligned) set to zero.
+cudaError_t launch_zero(void* p, long long n, cudaStream_t st);
 cudaError_t launch_efield(const KParams& P, const double* U, double* E, float4* E32, cudaStream_t st);
 cudaError_t launch_bc_fields(const KParams& P, double* E, float4* E32, cudaStream_t st);
 cudaError_t launch_energy_field(const KParams& P, const double* E, double* partial, double* out, cudaStream_t st);

@@ -690,6 +690,7 @@ __global__ void __launch_bounds__(256, kDepCtas) deposit_tile_c32_kernel(KParams
   static_assert(PER == 2 || PER == 4 || PER == 8, "loads of two or four particles");
   constexpr int V = PER < 4 ? PER : 4, kGroups = PER / V;
   constexpr unsigned kAll = (1u << PER) - 1u;
+  chain_begin();
   extern __shared__ unsigned int dep_tile[];  // per warp: [2][kDepTile] low and high 20-bit halves
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned int* lo = dep_tile + warp * 2 * kDepTile;
@@ -962,11 +963,9 @@ cudaError_t launch_deposit_c32(const KParams& P, PartC32 a, long long n, unsigne
     const long long chunk = (long long)kDepWarps * 32 * per;
     const long long chunks = (n + chunk - 1) / chunk, full = 148LL * kDepCtas;
     const int grid = int(chunks < full ? chunks : full);
-    note_launch();
     // the window reaches as far along x as the particles of one warp at this density, and a cell to either side
     const long long span = (chunk / kDepWarps) * cells / n + 2;
-    kernel<<<grid, 256, smem, st>>>(P, a, n, Nacc, uint32_t(span < 15 ? span : 15));
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, 256, smem, st, P, a, n, Nacc, uint32_t(span < 15 ? span : 15));
   }
   note_launch();
   deposit_c32_kernel<<<persistent_grid(n), kThreads, 0, st>>>(P, a, n, Nacc, Facc);
