@@ -11,8 +11,8 @@
 // overlap away.
 // A step of run_fused in us, with ordinary launches and with these (and the reading
 // of the step before moved behind the queued solve): 16^3 at 8 particles per cell
-// 238 and 180, 24^3 at 8 325 and 258, 32^3 at 32 296 and 246, 77^3 at 26 1078 and
-// 1032.  On large grids the gaps do not count (256 x 128 x 128: 1 % of a step).
+// 238 and 179, 24^3 at 8 325 and 252, 32^3 at 32 296 and 246, 77^3 at 26 1078 and
+// 1007.  On large grids the gaps do not count (256 x 128 x 128: 1 % of a step).
 //
 // What such a kernel reads of its predecessors' results is not declared
 // __restrict__: a load through the read-only path is meant for data that does not
