@@ -168,12 +168,22 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps_cluster_kernel(ClusterAr
 //
 // What bounds it: the chain of shared-memory loads, four planes and the barrier.
 // us per sweep of a 24-sweep round, here and with the tile kernel's launches:
-// 16^3 1.45 / 2.0, 24^3 1.47 / 1.95, 32^3 1.62 / 1.96.  A second row pair per half
+// 16^3 1.45 / 2.0, 24^3 1.65 / 1.95, 32^3 1.74 / 1.96 (with the row sums stored ahead
+// of the arrival instead 1.54, 1.71 and 1.85).  A second row pair per half
 // warp loses (40 x 36 x 30: 2.7 / 1.95, 48 x 40 x 33: 2.6 / 2.05; with every load
 // ahead of the first store 3.4), so at most 64 tile rows per layer are taken here;
 // among the grids that qualify the launch tuner decides.
 constexpr int kCl32Planes = 4;
 constexpr int kCl32Tasks = kClThreads / 16;
+// A row's sum of sweep s is stored after its thread's arrival at that sweep's
+// barrier, in the barrier's shadow, so only the arrival of sweep s + 1 makes it
+// visible: in sweep s, after their own arrival, the summing threads take the rows of
+// sweep s - kRowLag.  The slot they read is written again in sweep s - kRowLag +
+// kRowSlots, by a thread that has passed the barrier of the sweep before, which the
+// summing threads reach only when they have read.
+constexpr int kRowLag = 2;
+constexpr int kRowSlots = 4;
+static_assert(kRowLag >= 2 && kRowSlots >= kRowLag + 2, "a barrier between store and read, and between read and store");
 
 struct Cluster32Args {
   Stencil S;
@@ -197,8 +207,7 @@ __host__ __device__ inline int cluster32_pitch(int nx) { return (nx + 5) & ~1; }
 
 __global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster32Args A) {
   constexpr int ZC = kCl32Planes;
-  // row sums [3][tasks] (a thread may write sweep s + 1's before another has
-  // summed those of s - 1), then w [2][ZC + 2][ny + 2][pitch] in floats
+  // row sums [kRowSlots][tasks], then w [2][ZC + 2][ny + 2][pitch] in floats
   extern __shared__ double cl32_smem[];
   using pair = unsigned long long;
   const Stencil& S = A.S;
@@ -206,7 +215,7 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster
   const int pitch = cluster32_pitch(S.nx), area = pitch * (S.ny + 2), tasks = A.gx * S.ny;
   const int z0 = cta * ZC, kend = min(ZC, S.nz - z0);
   double* rows = cl32_smem;
-  float* w0 = reinterpret_cast<float*>(cl32_smem + 3 * tasks);
+  float* w0 = reinterpret_cast<float*>(cl32_smem + kRowSlots * tasks);
   const int buf = (ZC + 2) * area;
   for (int e = threadIdx.x; e < 2 * buf; e += kClThreads) w0[e] = 0.0f;  // ghosts and the increment itself
   // this lane's pair: which of its two nodes exist, and r
@@ -236,7 +245,7 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster
       double v = 0.0;
       for (int w = 0; w < 8; ++w) {
         const int row = by * 8 + w;
-        v += row < S.ny ? rows[(s % 3) * tasks + row * A.gx + bx] : 0.0;
+        v += row < S.ny ? rows[(s % kRowSlots) * tasks + row * A.gx + bx] : 0.0;
       }
       A.partial[(long long)s * A.nblocks + bx + A.gx * (by + A.gy * cta)] = v;
     }
@@ -284,7 +293,7 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster
     }
     __syncwarp();
     cluster_arrive();
-    if (s > 0) flush(s - 1);  // its rows are complete since the last barrier
+    if (s >= kRowLag) flush(s - kRowLag);
     // block_sum_store's 32-lane tree on 16 lanes of pairs
     const float2 f = up2(r2);
     double v0 = (double)f.x, v1 = (double)f.y;
@@ -293,12 +302,12 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps32_cluster_kernel(Cluster
       v0 += __shfl_down_sync(0xffffffffu, v0, o);
       v1 += __shfl_down_sync(0xffffffffu, v1, o);
     }
-    if ((lane & 15) == 0 && task < tasks) rows[(s % 3) * tasks + task] = v0 + v1;
+    if ((lane & 15) == 0 && task < tasks) rows[(s % kRowSlots) * tasks + task] = v0 + v1;
     __syncwarp();
     cluster_wait();
   }
   __syncthreads();
-  flush(A.m - 1);
+  for (int s = max(0, A.m - kRowLag); s < A.m; ++s) flush(s);
   if (!a0) return;
   const float* last = w0 + (A.m & 1) * buf + off;
   for (int kk = 0; kk < kend; ++kk) {
@@ -370,8 +379,8 @@ ClusterPlan cluster32_plan(const KParams& P, const JacobiGeom& G) {
   if (!G.tma || G.zc != kCl32Planes || ctas < 2 || ctas > 16 || tasks > kCl32Tasks) return C;
   C.ctas = ctas;
   C.planes = kCl32Planes;
-  C.smem = 24 * (size_t)tasks + 8 * (size_t)(kCl32Planes + 2) * cluster32_pitch(P.nx) * (P.ny + 2);
-  static_assert(24 * kCl32Tasks + 8 * (kCl32Planes + 2) * 68 * (kCl32Tasks + 2) <= kClSmem, "at most 64 x 64 nodes");
+  C.smem = sizeof(double) * kRowSlots * (size_t)tasks + 8 * (size_t)(kCl32Planes + 2) * cluster32_pitch(P.nx) * (P.ny + 2);
+  static_assert(8 * kRowSlots * kCl32Tasks + 8 * (kCl32Planes + 2) * 68 * (kCl32Tasks + 2) <= kClSmem, "at most 64 x 64 nodes");
   auto k = sweeps32_cluster_kernel;
   cudaLaunchAttribute at[1];
   const cudaLaunchConfig_t cfg = cluster_config(C, at, nullptr);
