@@ -203,6 +203,10 @@ __device__ __forceinline__ void fft_block(double2* x, const double2* __restrict_
   fft_pass<LOG, 0, INV, BLOAD, BSTORE>(x, tw, load, store);
 }
 
+// The stages of a run are chained launches (chain.cuh), so the bodies below read C
+// and the stage buffers W, S and V by ordinary loads; the read-only path is for
+// the twiddles and the slice transforms, which no kernel of the chain writes.
+
 // Geometry of one face pair: A the normal axis, P and Q the tangential axes.
 struct FaceGeom {
   int nA, nP, nQ;
@@ -229,8 +233,8 @@ __device__ inline int circ_off(int t, int L, int n, bool& ok) {
 // kernel rows (s, tQ) of slices s0 + a (a < count), tQ = by < LQ, from D.
 // Output W[(a * rowsQ + q) * HP + kP], kP < HP.
 template <int LOG>
-__device__ void bcfft_rows_body(const FaceGeom& F, int mode, const double* __restrict__ src, int s0, int count,
-                                const double2* __restrict__ tw, double2* __restrict__ W, int bx, int by) {
+__device__ void bcfft_rows_body(const FaceGeom& F, int mode, const double* src, int s0, int count,
+                                const double2* __restrict__ tw, double2* W, int bx, int by) {
   extern __shared__ double2 smem[];
   constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int q = by;
@@ -298,9 +302,8 @@ __device__ __forceinline__ int plane_at(int t, int nA) { return t & 1 ? nA - 1 -
 // mode 1 (kernel transforms): slice by < count of W, real part times scale to
 // Dh[(s0 + by) * HP * LQ + kP * LQ + kQ].
 template <int LOG>
-__device__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* __restrict__ W, int s0, int count,
-                                double scale, const double2* __restrict__ tw, double* __restrict__ Dh,
-                                double2* __restrict__ S, int bx, int by) {
+__device__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* W, int s0, int count, double scale,
+                                const double2* __restrict__ tw, double* Dh, double2* S, int bx, int by) {
   extern __shared__ double2 smem[];
   constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int k0 = bx * B;
@@ -315,7 +318,7 @@ __device__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* __re
     const int a = mode == 0 ? plane_at(t, F.nA) : t;
     const double2* w = W + (long long)a * rowsQ * F.HP + k0;
     auto load = [&](int b, int q) {
-      return k0 + b < F.HP && q < rowsQ ? __ldg(w + (long long)q * F.HP + b) : make_double2(0.0, 0.0);
+      return k0 + b < F.HP && q < rowsQ ? w[(long long)q * F.HP + b] : make_double2(0.0, 0.0);
     };
     if (t > t_lo) __syncthreads();  // the plane before has read its last shared element
     if (mode == 0) {
@@ -355,8 +358,8 @@ __device__ void bcfft_cols_body(const FaceGeom& F, int mode, const double2* __re
 // Q of columns kP in [bx B, bx B + B) of face f = by; V[(f*nQ + q)*HP + kP] for
 // q < nQ.
 template <int LOG>
-__device__ void bcfft_invq_body(const FaceGeom& F, const double2* __restrict__ S, const double2* __restrict__ tw,
-                                double2* __restrict__ V, int bx, int by) {
+__device__ void bcfft_invq_body(const FaceGeom& F, const double2* S, const double2* __restrict__ tw, double2* V,
+                                int bx, int by) {
   extern __shared__ double2 smem[];
   constexpr int L = 1 << LOG, B = kFftElems >> LOG;
   const int k0 = bx * B, f = by;
@@ -369,7 +372,7 @@ __device__ void bcfft_invq_body(const FaceGeom& F, const double2* __restrict__ S
           const double2* s = S + (long long)f * plane + (long long)(k0 + b) * L + kq;
 #pragma unroll 4
           for (int g = 0; g < F.G; ++g) {
-            const double2 e = __ldg(s + (long long)g * 2 * plane);
+            const double2 e = s[(long long)g * 2 * plane];
             v.x += e.x;
             v.y += e.y;
           }
@@ -385,8 +388,8 @@ __device__ void bcfft_invq_body(const FaceGeom& F, const double2* __restrict__ S
 // by, m in [bx B, bx B + B) (the spectrum's upper half from Hermitian
 // symmetry): two real rows as the real and imaginary part of one transform.
 template <int LOG>
-__device__ void bcfft_invp_body(const FaceGeom& F, const double2* __restrict__ V, const double2* __restrict__ tw,
-                                double* __restrict__ U, int bx, int by) {
+__device__ void bcfft_invp_body(const FaceGeom& F, const double2* V, const double2* __restrict__ tw, double* U,
+                                int bx, int by) {
   extern __shared__ double2 smem[];
   constexpr int L = 1 << LOG, B = kFftElems >> LOG, HP = L / 2 + 1;
   const int q0 = 2 * bx * B, f = by;
@@ -399,7 +402,7 @@ __device__ void bcfft_invp_body(const FaceGeom& F, const double2* __restrict__ V
         if (q < F.nQ) {
           const bool up = k >= HP;
           const double2* r = V + ((long long)f * F.nQ + q) * HP + (up ? L - k : k);
-          double2 v = __ldg(r), w = q + 1 < F.nQ ? __ldg(r + HP) : make_double2(0.0, 0.0);
+          double2 v = r[0], w = q + 1 < F.nQ ? r[HP] : make_double2(0.0, 0.0);
           if (up) v.y = -v.y, w.y = -w.y;
           z = make_double2(v.x - w.y, v.y + w.x);  // v + i w
         }
