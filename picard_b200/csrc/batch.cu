@@ -773,7 +773,6 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
     else if (q != PICARD_OK) return q;
     return PICARD_OK;
   };
-  for (int r = 0; r < n; ++r) ctxs[r]->spec.collected = ctxs[r]->spec.queued;
   auto body = [&]() -> int {
     for (int32_t step = 1; step <= nsteps; ++step) {
       tick = now();
@@ -972,7 +971,13 @@ int batch_run_impl(picard_ctx** ctxs, int32_t n, const int32_t* it0, int32_t nst
                  n, ph[0], ph[1], ph[2], rounds, ticks, launches, g_batch_ctas);
   if (rc == PICARD_OK) rc = check_cuda(cudaStreamSynchronize(bst), "batch stream");
   cleanup();
-  if (rc != PICARD_OK) return rc;
+  if (rc != PICARD_OK) {
+    // what the runs have under way is read all the same: each one's next solve is
+    // the next one collected
+    const std::string why = picard_gpu_last_error();
+    for (int r = 0; r < n; ++r) spec_drain(ctxs[r], sweeps_total ? sweeps_total + r : nullptr);
+    return fail(rc, why);
+  }
   if (nc) return fail(PICARD_ERR_NOT_CONVERGED, "at least one Jacobi solve hit 2*maxit+1 sweeps");
   return PICARD_OK;
 }

@@ -236,6 +236,10 @@ int spec_issue(picard_ctx* c, double maxerr, int maxit);
 // After the stream has passed it: books the oldest solve not collected and reports its sweeps and
 // status (PICARD_ERR_NOT_CONVERGED included).  Zero sweeps when none is pending.
 int spec_collect(picard_ctx* c, long long* sweeps);
+// After a loop that ended early: waits for the stream and books every solve not
+// collected (their sweeps are added to *sweeps_total, which may be null).  Outside
+// the loops no solve is ever left to collect.  May change the last error's text.
+void spec_drain(picard_ctx* c, int64_t* sweeps_total);
 }  // namespace picard
 
 #define PICARD_CUDA(expr)                                          \

@@ -244,13 +244,14 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
   const bool source = has_neutral_source(K);
   bool nc = false;
   bool advanced = false;  // the previous step's push already advanced the positions
-  bool open = false;      // the previous step's events and closed-form solve are still to be read
+  const cudaEvent_t* open = nullptr;  // events of a step whose times and closed-form solve are still to be read
   // A step is queued up to its velocity push without waiting for its solve; what
   // the host has to know of it is read at the next step's particle count, so the
   // device has work while the host goes from one step to the next.
-  auto settle = [&](const cudaEvent_t* ev) -> int {
+  auto settle = [&]() -> int {
     if (!open) return PICARD_OK;
-    open = false;
+    const cudaEvent_t* ev = open;
+    open = nullptr;
     for (int ph = 0; ph < 5; ++ph) {
       float ms = 0.0f;
       if (cudaEventElapsedTime(&ms, ev[ph], ev[ph + 1]) == cudaSuccess) c->stats.phase_ms[ph] += ms;
@@ -264,10 +265,8 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
       return rc;
     return PICARD_OK;
   };
-  c->spec.collected = c->spec.queued;
-  for (int32_t it = iter_start + 1; it <= iter_end; ++it) {
+  auto step = [&](int32_t it) -> int {
     const cudaEvent_t* ev = c->pev + 6 * (it & 1);
-    const cudaEvent_t* before = c->pev + 6 * (1 - (it & 1));
     PICARD_CUDA(cudaEventRecord(ev[0], c->st));
     // AdvancePosition on the particles present before BCinflow
     if (!advanced) PICARD_TRY(picard_gpu_advance_position(c, p.dt));
@@ -313,7 +312,7 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
     PICARD_CUDA(cudaEventRecord(ev[4], c->st));
     // the step before has passed the count above; read it while the device has the
     // whole solve to do
-    PICARD_TRY(settle(before));
+    PICARD_TRY(settle());
     PICARD_TRY(picard_gpu_calc_efield(c));
     // AdvanceVelocity; in the CELL32 layout, when another step follows, fused
     // with that step's AdvancePosition (one pass over the particles)
@@ -323,12 +322,23 @@ int picard_gpu_run_fused(picard_ctx* c, int32_t iter_start, int32_t iter_end, in
     else
       PICARD_TRY(picard_gpu_advance_velocity(c, p.dt));
     PICARD_CUDA(cudaEventRecord(ev[5], c->st));
-    open = true;
+    open = ev;
     c->stats.steps += 1;
     c->stats.particle_steps += c->num_local;
+    return PICARD_OK;
+  };
+  int rc = PICARD_OK;
+  for (int32_t it = iter_start + 1; it <= iter_end && rc == PICARD_OK; ++it) rc = step(it);
+  if (rc == PICARD_OK) rc = check_dev_err_public(c);  // waits for the stream; a wait that gave up in the last step
+  if (rc == PICARD_OK) rc = settle();
+  if (rc != PICARD_OK) {
+    // what the step that failed left under way is read all the same, so that the
+    // context's next solve is the next one collected
+    const std::string why = picard_gpu_last_error();
+    if (cudaStreamSynchronize(c->st) == cudaSuccess) (void)settle();
+    spec_drain(c, sweeps_total);
+    return fail(rc, why);
   }
-  PICARD_TRY(check_dev_err_public(c));  // waits for the stream; a wait that gave up in the last step
-  PICARD_TRY(settle(c->pev + 6 * (iter_end & 1)));
   if (nc) return fail(PICARD_ERR_NOT_CONVERGED, "at least one Jacobi solve hit 2*maxit+1 sweeps");
   return PICARD_OK;
 }

@@ -460,8 +460,12 @@ extern "C" int picard_gpu_calc_epotential(picard_ctx* c, double maxerr, int32_t 
   if (c->solver == PICARD_SOLVER_SPECTRAL) {
     long long done = 0;
     PICARD_TRY(spec_issue(c, maxerr, maxit));
-    PICARD_CUDA(cudaStreamSynchronize(c->st));
-    const int rc = spec_collect(c, &done);
+    int rc = check_cuda(cudaStreamSynchronize(c->st), "cudaStreamSynchronize(c->st)");
+    if (rc != PICARD_OK) {
+      c->spec.collected = c->spec.queued;
+      return rc;
+    }
+    rc = spec_collect(c, &done);
     if (sweeps_out) *sweeps_out = int32_t(done);
     return rc;
   }

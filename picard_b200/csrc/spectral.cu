@@ -782,4 +782,14 @@ int spec_collect(picard_ctx* c, long long* sweeps) {
   return epot_account(c, Q.bnorm, Q.trivial ? Q.bnorm : std::sqrt(Q.r2_hit), Q.smax, Q.d, Q.converged != 0);
 }
 
+void spec_drain(picard_ctx* c, int64_t* sweeps_total) {
+  if (c->spec.queued == c->spec.collected) return;
+  if (cudaStreamSynchronize(c->st) != cudaSuccess) c->spec.collected = c->spec.queued;  // their results never came
+  while (c->spec.queued != c->spec.collected) {
+    long long sw = 0;
+    (void)spec_collect(c, &sw);
+    if (sweeps_total) *sweeps_total += sw;
+  }
+}
+
 }  // namespace picard
