@@ -339,7 +339,13 @@ typedef enum picard_option {
    * (picard_gpu_sort_particles) in the ParticlesTransfer slot of every
    * iteration divisible by k; 0 (the default): never.  The per-subroutine
    * loops never sort (their particles stay in the reference's order). */
-  PICARD_OPT_SORT_EVERY = 9
+  PICARD_OPT_SORT_EVERY = 9,
+  /* 1: every sweep of a round in one thread-block cluster, on grids of 5 .. 63
+   * planes with at most 64 tile rows (ny times the 32-wide tiles of a row), else
+   * PICARD_ERR_STATE (the launch tuner picks it where it measures faster);
+   * 0, or any other sweep knob above set to a value it takes: off.  Never
+   * changes a result bit. */
+  PICARD_OPT_SWEEP_CLUSTER = 10
 } picard_option;
 /* Reads an option's current value (SWEEP_CTAS: 0 means one CTA per tile). */
 PICARD_API int picard_gpu_get_option(picard_ctx* ctx, int32_t option, int32_t* value);

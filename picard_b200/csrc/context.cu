@@ -1059,6 +1059,10 @@ int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
     if (c->G.rglobal) c->G.pairs = 1, c->G.fused2 = 0;
     return PICARD_OK;
   }
+  if (option == PICARD_OPT_SWEEP_CLUSTER) {
+    if (value != 0 && value != 1) return fail(PICARD_ERR_BAD_ARG, "SWEEP_CLUSTER must be 0 or 1");
+    return set_cluster(c, value);
+  }
   if (option == PICARD_OPT_SORT_EVERY) {
     if (value < 0) return fail(PICARD_ERR_BAD_ARG, "SORT_EVERY must be >= 0");
     c->sort_every = value;
@@ -1085,6 +1089,7 @@ int picard_gpu_get_option(picard_ctx* c, int32_t option, int32_t* value) {
     case PICARD_OPT_WAIT_TEST: *value = c->wait_test; return PICARD_OK;
     case PICARD_OPT_SWEEP_R_GLOBAL: *value = c->G.rglobal; return PICARD_OK;
     case PICARD_OPT_SORT_EVERY: *value = c->sort_every; return PICARD_OK;
+    case PICARD_OPT_SWEEP_CLUSTER: *value = c->cluster32.ctas != 0; return PICARD_OK;
   }
   return fail(PICARD_ERR_BAD_ARG, "unknown option");
 }

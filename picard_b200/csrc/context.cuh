@@ -206,6 +206,7 @@ int dev_alloc(picard_ctx* c, void** p, size_t bytes);
 int tune_sweep(picard_ctx* c, bool fresh);
 // PICARD_OPT_SWEEP_RESIDENT: 0 off, q + 1 resident with CTA shape q.
 int set_resident(picard_ctx* c, int value);
+int set_cluster(picard_ctx* c, int value);
 int resident_option_value(const picard_ctx* c);
 // Stable counting sort of the context's particles by cell; synchronises once
 // to read the run count.

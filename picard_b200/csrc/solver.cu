@@ -561,6 +561,19 @@ int set_resident(picard_ctx* c, int value) {
   return apply_shape(c, sh);
 }
 
+int set_cluster(picard_ctx* c, int value) {
+  if (value == 0) {
+    c->cluster32 = ClusterPlan();
+    return PICARD_OK;
+  }
+  if (!c->G.tma || !c->w[0]) return fail(PICARD_ERR_STATE, "cluster sweeps need open boundaries and the F32_REFINE solver");
+  const ClusterPlan C = cluster32_plan(c->K, c->G);
+  if (!C.ctas) return fail(PICARD_ERR_STATE, "the sweeps of this grid do not fit one cluster");
+  c->cluster32 = C;
+  c->G.res = 0;
+  return PICARD_OK;
+}
+
 int resident_option_value(const picard_ctx* c) {
   if (!c->G.res) return 0;
   for (int q = 0; q < kResidentShapes; ++q) {
