@@ -1008,8 +1008,7 @@ int picard_gpu_particles_gridify_all(picard_ctx* c) {
   return deposit(c, true);
 }
 
-int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
-  if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
+static int set_option(picard_ctx* c, int32_t option, int32_t value) {
   if (option == PICARD_OPT_BCPOT_TENSOR) {
     if (value < PICARD_BCPOT_DIRECT || value > PICARD_BCPOT_FFT)
       return fail(PICARD_ERR_BAD_ARG, "BCPOT_TENSOR must be 0 (direct), 1 (tensor cores) or 2 (FFT)");
@@ -1018,9 +1017,6 @@ int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
     c->bcpot_tensor = value;
     return PICARD_OK;
   }
-  // a sweep shape asked for by hand replaces the cluster that the tuner may have picked
-  if (option >= PICARD_OPT_SWEEP_CTAS && option <= PICARD_OPT_SWEEP_FUSED) c->cluster32 = ClusterPlan();
-  if (option == PICARD_OPT_SWEEP_R_GLOBAL) c->cluster32 = ClusterPlan();
   if (option == PICARD_OPT_SWEEP_CTAS) {
     if (value < -1) return fail(PICARD_ERR_BAD_ARG, "SWEEP_CTAS must be -1, 0 or a CTA count");
     if (value == 0) {
@@ -1074,6 +1070,17 @@ int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
     return PICARD_OK;
   }
   return fail(PICARD_ERR_BAD_ARG, "unknown option");
+}
+
+int picard_gpu_set_option(picard_ctx* c, int32_t option, int32_t value) {
+  if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
+  PICARD_TRY(set_option(c, option, value));
+  // a sweep shape asked for by hand replaces the cluster that the tuner may have
+  // picked (SWEEP_CTAS 0 has just asked the tuner)
+  const bool shape = (option >= PICARD_OPT_SWEEP_CTAS && option <= PICARD_OPT_SWEEP_FUSED) ||
+                     option == PICARD_OPT_SWEEP_R_GLOBAL;
+  if (shape && !(option == PICARD_OPT_SWEEP_CTAS && value == 0)) c->cluster32 = ClusterPlan();
+  return PICARD_OK;
 }
 
 int picard_gpu_get_option(picard_ctx* c, int32_t option, int32_t* value) {
