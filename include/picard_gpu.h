@@ -157,7 +157,9 @@ PICARD_API int picard_gpu_footprint(const picard_params* p, int32_t layout, int3
  * a process that creates and releases many contexts (parameter sweeps, the
  * serving loop) maps memory again for every one.  This keeps up to `bytes` of
  * freed memory in the pool of `device` for reuse (the serving loop sets its
- * budget), and up to 64 MB of it in freed pinned host memory.  No counterpart in the reference (its arrays are static). */
+ * budget), and as much, up to 64 MB, of freed pinned host memory, which the
+ * devices share (the largest of their values counts).  No counterpart in the
+ * reference (its arrays are static). */
 PICARD_API int picard_gpu_pool_keep(int32_t device, uint64_t bytes);
 
 /* Particles in the reference layout: real_particles(8, n) column-major

@@ -13,11 +13,11 @@
 
 #include "context.cuh"
 #include "picard_gpu.h"
+#include "pinned.cuh"
 
 using namespace picard;
 
 #include <atomic>
-#include <mutex>
 #include <thread>
 
 namespace picard {
@@ -147,65 +147,18 @@ InflowTable make_inflow_table(const picard_params& p) {
 
 namespace {
 
-// Pinned host memory of the process's contexts, in blocks of two sizes: a
-// context's mailbox and a piece of a field on its way to the host.  Allocating
-// or freeing pinned memory takes milliseconds and waits for the device, so freed
-// blocks are kept: four staging blocks while any context lives, and beyond that
-// what picard_gpu_pool_keep allows (at most kPinnedKeepMost), which also bounds
-// what stays after the last context is gone.  Any thread, any device.
-constexpr size_t kPinnedBlock[2] = {36 << 10, 4 << 20};
-constexpr size_t kPinnedKeepMost = 64 << 20;
-struct PinnedPool {
-  std::mutex mu;
-  std::vector<void*> idle[2];
-  size_t keep = 0;
-  long long contexts = 0;
-
-  size_t idle_bytes() const { return idle[0].size() * kPinnedBlock[0] + idle[1].size() * kPinnedBlock[1]; }
-  void trim() {  // with mu held
-    const size_t allowed = keep + (contexts > 0 ? 4 * kPinnedBlock[1] : 0);
-    for (int cls = 1; cls >= 0; --cls)
-      while (!idle[cls].empty() && idle_bytes() > allowed) {
-        cudaFreeHost(idle[cls].back());
-        idle[cls].pop_back();
-      }
-  }
-  void* get(int cls) {
-    {
-      std::lock_guard<std::mutex> lk(mu);
-      if (!idle[cls].empty()) {
-        void* p = idle[cls].back();
-        idle[cls].pop_back();
-        return p;
-      }
-    }
+struct CudaPinned {
+  static void* alloc(size_t bytes) {
     void* p = nullptr;
-    if (cudaHostAlloc(&p, kPinnedBlock[cls], cudaHostAllocPortable) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return nullptr;
-    }
-    return p;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return p;
+    (void)cudaGetLastError();
+    return nullptr;
   }
-  void put(int cls, void* p) {
-    if (!p) return;
-    std::lock_guard<std::mutex> lk(mu);
-    idle[cls].push_back(p);
-    trim();
-  }
-  void context(int d) {
-    std::lock_guard<std::mutex> lk(mu);
-    contexts += d;
-    trim();
-  }
-  void set_keep(size_t bytes) {
-    std::lock_guard<std::mutex> lk(mu);
-    keep = std::min(bytes, kPinnedKeepMost);
-    trim();
-  }
+  static void free(void* p) { cudaFreeHost(p); }
 };
 // never destroyed: blocks kept at exit go with the process, after the driver
-PinnedPool& pinned() {
-  static PinnedPool* p = new PinnedPool();
+PinnedPool<CudaPinned>& pinned() {
+  static auto* p = new PinnedPool<CudaPinned>();
   return *p;
 }
 
@@ -435,7 +388,7 @@ int picard_gpu_pool_keep(int32_t device, uint64_t bytes) {
   cudaMemPool_t pool;
   PICARD_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
   PICARD_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes));
-  pinned().set_keep((size_t)bytes);
+  pinned().set_keep(device, (size_t)bytes);
   return PICARD_OK;
 }
 
