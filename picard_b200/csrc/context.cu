@@ -4,11 +4,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <vector>
 
 #include "context.cuh"
@@ -723,24 +723,45 @@ int picard_gpu_get_field(picard_ctx* c, int32_t which, double* out) {
   // Pieces of up to 4 MB through pinned memory, the components brought into the
   // reference order on the device; up to four host threads copy them on, each
   // with its own pinned block, so the pieces of one are under way while another's
-  // are copied.  (One pageable copy into a scratch array and a loop over it took
+  // are copied; one that gets no pinned block copies its pieces through pageable
+  // memory.  (One pageable copy into a scratch array and a loop over it took
   // 32 ms for U and 80 ms for N of 256 x 128 x 128.)
   const long long total = (long long)ncomp * n, piece = (long long)(kPinnedBlock[1] / sizeof(double));
   const long long pieces = (total + piece - 1) / piece;
   const int fs = which == PICARD_FIELD_F ? c->prm.species : 0;
   const int workers = int(std::min<long long>(4, (pieces + 1) / 2));
-  std::vector<int> status(std::max(workers, 1), PICARD_OK);
-  std::vector<std::string> message(status.size());
+  std::array<int, 4> status{};  // PICARD_OK
+  std::array<std::string, 4> message;
   std::atomic<long long> next{0};
+  // elements [first, first + count) without pinned memory: their nodes of every plane, put in order here
+  auto copy_pageable = [&](std::vector<double>& h, long long first, long long count) -> cudaError_t {
+    const long long g0 = first / ncomp, nodes = (first + count - 1) / ncomp + 1 - g0;
+    h.resize((size_t)(ncomp * nodes));
+    cudaError_t e = cudaSuccess;
+    for (int pl = 0; pl < ncomp && e == cudaSuccess; ++pl)
+      e = cudaMemcpyAsync(h.data() + pl * nodes, dev + pl * n + g0, sizeof(double) * nodes, cudaMemcpyDeviceToHost, c->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->st);
+    if (e != cudaSuccess) return e;
+    for (int pl = 0; pl < ncomp; ++pl)
+      for (long long g = 0; g < nodes; ++g) {
+        const long long at = (long long)ref_index(which, c->prm.species, pl, g0 + g);
+        if (at >= first && at < first + count) out[at] = h[(size_t)(pl * nodes + g)];
+      }
+    return cudaSuccess;
+  };
   auto work = [&](int w) {
     auto run = [&]() -> int {
       double* stage = static_cast<double*>(pinned().get(1));
-      if (!stage) return fail(PICARD_ERR_CUDA, "no pinned host memory");
+      std::vector<double> h;  // where there is no pinned block
       cudaEvent_t done = nullptr;
       int rc = check_cuda(cudaEventCreateWithFlags(&done, cudaEventDisableTiming), "cudaEventCreate");
       for (long long q; rc == PICARD_OK && (q = next.fetch_add(1)) < pieces;) {
         const long long first = q * piece, count = std::min(piece, total - first);
         cudaError_t e;
+        if (!stage) {
+          rc = check_cuda(copy_pageable(h, first, count), "field copy");
+          continue;
+        }
         if (ncomp == 1) {
           e = cudaMemcpyAsync(stage, dev + first, sizeof(double) * count, cudaMemcpyDeviceToHost, c->st);
         } else {
@@ -770,16 +791,17 @@ int picard_gpu_get_field(picard_ctx* c, int32_t which, double* out) {
     }
     if (device != c->device) cudaSetDevice(device);
   };
-  std::vector<std::thread> others;
+  std::array<std::thread, 3> others;
   for (int w = 1; w < workers; ++w) {
     try {
-      others.emplace_back(work, w);
-    } catch (const std::system_error&) {
+      others[w - 1] = std::thread(work, w);
+    } catch (const std::exception&) {
       break;  // fewer threads share the pieces
     }
   }
   work(0);
-  for (std::thread& th : others) th.join();
+  for (std::thread& th : others)
+    if (th.joinable()) th.join();
   for (size_t w = 0; w < status.size(); ++w)
     if (status[w] != PICARD_OK) return fail(status[w], message[w].empty() ? "field copy" : message[w]);
   c->stats.d2h_bytes += (int64_t)(sizeof(double) * total);
