@@ -177,6 +177,12 @@ PICARD_API int picard_gpu_set_field(picard_ctx* ctx, int32_t which, const double
 
 /* ------------------------------------------- one entry per reference routine */
 
+/* The calls queue their work on the context's stream and return; those that hand
+ * something to the host (a count, the sweeps, an energy, a field) or check the
+ * device's error word wait for it.  picard_gpu_particles_initialize,
+ * picard_gpu_bc_inflow and, when no species has a source,
+ * picard_gpu_particles_produce do neither: an error of work queued before them is
+ * returned by the next call that waits. */
 PICARD_API int picard_gpu_calc_distance(picard_ctx* ctx);                       /* CalcDistance.f90:1-95        */
 PICARD_API int picard_gpu_particles_initialize(picard_ctx* ctx);                /* ParticlesInitialize.f90:2-125*/
 PICARD_API int picard_gpu_bc_inflow(picard_ctx* ctx, int32_t iteration);        /* BCinflow.f90:2-476           */
@@ -260,8 +266,9 @@ typedef struct picard_stats {
   int64_t kernel_launches;
   int64_t solves;          /* CalcEpotential calls                          */
   int64_t sweeps;          /* Jacobi iterations accepted, summed over solves */
-  int64_t sweep_launches;  /* sweep kernels run (replays and overshoot too)  */
-  double sweep_ms;         /* device time of those sweep launches            */
+  int64_t sweep_launches;  /* sweeps run by kernels (replays and overshoot
+                              too; one launch may run two or a whole batch)  */
+  double sweep_ms;         /* device time of those sweeps                    */
   int64_t anchor_launches; /* FP64 anchor passes (F32_REFINE solver)         */
   double anchor_ms;
   double last_residual;    /* ||b - L U|| of the last accepted iterate       */

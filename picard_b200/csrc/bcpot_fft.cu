@@ -186,13 +186,15 @@ __device__ __forceinline__ void fft_pass(double2* x, const double2* __restrict__
   }
 }
 
-// What bounds the stages: latency at small sizes, the 128-register blocks' two
-// per SM at large ones (DRAM at an eighth of its rate).  Before, a stage was a
+// What bounds the stages: latency at small sizes; at large ones the shared-memory
+// pipe of the row transforms (75 % busy, an eighth of it conflicts) and, in the
+// contraction, global loads that two blocks of 128 registers per SM do not hide
+// (DRAM at a quarter of its rate).  Before, a stage was a
 // generic radix-4 Stockham transform that crossed shared memory at every
 // radix, in natural element order (30-44 % of its wavefronts were bank
 // conflicts), with one real row per complex transform and a launch per face
-// pair.  BCpotentials in us, before and now: 24^3 117 and 30, 77^3 378 and 99,
-// 128^3 654 and 206, 256 x 128 x 128 1159 and 350, 200 x 140 x 140 2258 and 622.
+// pair.  BCpotentials in us, before and now: 24^3 117 and 24, 77^3 378 and 93,
+// 128^3 654 and 190, 256 x 128 x 128 1159 and 332, 200 x 140 x 140 2258 and 628.
 //
 // B = 2048 / L transforms of length L = 2^LOG (8 .. 2048) by the block: inputs
 // load(b, i), outputs store(u, b, i, value), natural order, no scaling.  A
@@ -528,7 +530,14 @@ int pair_blocks(const FaceGeom& F, int rows) { return (rows + 2 * (kFftElems >> 
 
 // Whether the face pairs go through the row and contraction stages together:
 // while their row transforms fit the L2 cache with room to spare.  Else one
-// after another, so that each contraction finds its own row transforms in L2.
+// after another, so that each contraction finds its own row transforms in L2 and has
+// three times the plane groups (face_geom).  BCpotentials in us, one after another
+// and together: 64^3 (14 MB) 87 / 50, 64 x 128 x 100 (38 MB) 138 / 99, 60 x 60 x 250
+// (45 MB) 173 / 163, 96^3 (54 MB) 141 / 117; above the line 100 x 200 x 80 (94 MB)
+// 242 / 395, 120 x 120 x 150 (106 MB) 262 / 414, 256 x 128 x 128 (164 MB) 332 / 355.
+// Pairs of equal transform lengths, which share their launches, gain from going
+// together up to 97 MB (128^3 190 / 163), pairs of unequal ones lose from 54 MB on
+// (100 x 130 x 60 177 / 248).
 bool faces_together(const KParams& K) {
   auto half = [](int n) { return pow2_at_least(2 * n - 1) / 2 + 1LL; };
   const long long elems = (long long)K.nx * K.nz * half(K.ny) + (long long)K.ny * K.nz * half(K.nx) +
@@ -563,7 +572,10 @@ FaceGeom face_geom(const KParams& K, int axis) {
   F.face1 = F.base + (long long)F.nA * F.sA;     // plane nA + 1
   // plane groups of the contraction: two blocks per SM, counting the other face
   // pairs of a launch; on small grids no more than eight partials, which the
-  // inverse along Q sums before it starts
+  // inverse along Q sums before it starts.  BCpotentials in us with at most 4 / 8 /
+  // 16 / 32 groups: 24^3 29.2 / 29.1 / 29.7 / 32.5, 40^3 48 / 37.6 / 38.4 / 43.9, 64^3 59
+  // / 50.2 / 44.4 / 50.0, 128^3 405 / 252 / 185 / 190 (72^3 and 96^3 fill the SMs with
+  // eight)
   const int share = col_blocks(F) * (faces_together(K) ? 3 : 1);
   F.G = std::max(1, std::min(std::min(F.nA, F.nA <= 64 ? 8 : 32), 2 * 148 / share));
   return F;

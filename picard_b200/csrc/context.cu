@@ -724,8 +724,8 @@ int picard_gpu_get_field(picard_ctx* c, int32_t which, double* out) {
   // reference order on the device; up to four host threads copy them on, each
   // with its own pinned block, so the pieces of one are under way while another's
   // are copied; one that gets no pinned block copies its pieces through pageable
-  // memory.  (One pageable copy into a scratch array and a loop over it took
-  // 32 ms for U and 80 ms for N of 256 x 128 x 128.)
+  // memory.  (U of 256 x 128 x 128 2.5 ms, N 6.2; one pageable copy into a
+  // scratch array and a loop over it took 21 and 79.)
   const long long total = (long long)ncomp * n, piece = (long long)(kPinnedBlock[1] / sizeof(double));
   const long long pieces = (total + piece - 1) / piece;
   const int fs = which == PICARD_FIELD_F ? c->prm.species : 0;

@@ -51,8 +51,6 @@ __device__ inline int mirror(int i, int n, int open) {
   return i < 1 ? i + n : i - n;
 }
 
-// N_s = n2p_s * acc * 2^-40 at every node (ParticlesGridify.f90:98-121 with the
-// folds of 149-278), C = sum_s q_s N_s (288-293).
 // n zero words of 8 bytes (p 16-byte aligned), in the chain: a copy-engine memset
 // of a small array costs some 5 us between kernels, this 1.
 __global__ void __launch_bounds__(kThreads) zero_kernel(unsigned long long* p, long long n) {
@@ -62,6 +60,8 @@ __global__ void __launch_bounds__(kThreads) zero_kernel(unsigned long long* p, l
   if (first == 0 && (n & 1)) p[n - 1] = 0ull;
 }
 
+// N_s = n2p_s * acc * 2^-40 at every node (ParticlesGridify.f90:98-121 with the
+// folds of 149-278), C = sum_s q_s N_s (288-293).
 __global__ void finish_deposit_kernel(KParams P, const unsigned long long* Nacc, double* N, double* Cout) {
   chain_begin();
   long long g = (long long)blockIdx.x * blockDim.x + threadIdx.x;

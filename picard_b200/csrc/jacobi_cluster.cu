@@ -16,9 +16,10 @@
 // reciprocals of the squared spacings instead of dividing by them.  Its squares
 // are summed per warp in a fixed order, one partial per warp and sweep.
 //
-// What bounds it: FP64 issue on 16 SMs and the barrier.  32^3 (16 CTAs, two nodes
-// a thread): 1.33 us per sweep against 4.07 us of kernel time and 3.3 us of host
-// time for one launch per sweep.
+// What bounds it: the shared-memory pipe of 16 SMs (71 % busy), their issue slots
+// (50 %; FP64 23 %) and the fence and wait of the barrier (the first stall).  32^3 (16
+// CTAs, two nodes a thread): 1.33 us per sweep against 4.07 us of kernel time and 3.3
+// us of host time for one launch per sweep.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -166,7 +167,8 @@ __global__ void __launch_bounds__(kClThreads, 1) sweeps_cluster_kernel(ClusterAr
 // order), so the bits are those of every other sweep kernel.  A launch starts from
 // w = 0, as every round of sweeps after an anchor does.
 //
-// What bounds it: the chain of shared-memory loads, four planes and the barrier.
+// What bounds it: the chain of shared-memory loads through four planes (that pipe 59 %
+// busy) and the barrier (its wait and fence are the first stalls).
 // us per sweep of a 24-sweep round, here and with the tile kernel's launches:
 // 16^3 1.45 / 2.0, 24^3 1.65 / 1.95, 32^3 1.74 / 1.96 (with the row sums stored ahead
 // of the arrival instead 1.54, 1.71 and 1.85).  A second row pair per half

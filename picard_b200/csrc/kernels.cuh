@@ -72,7 +72,8 @@ constexpr int kOutflowWordsPerBlock = 64;
 // BCoutflow split around a host read of the survivor count (for callers that
 // synchronise anyway): stage 1 marks, scans and writes m, the survivors at or
 // above the new count n', to info[0]; stage 2 fills the holes below n', by
-// pointer jumping over the window [n', n) when nxt (n - n' ints) is given, else by following each hole's chain (outflow.cuh).
+// pointer jumping over the window [n', n) when nxt (n - n' ints) is given, else
+// by following each hole's chain (outflow.cuh).
 struct OutflowSplit {
   int stage;
   long long np;  // stage 2: n' (*count after stage 1)

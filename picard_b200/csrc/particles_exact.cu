@@ -221,8 +221,8 @@ struct StoreC32 {
 // Candidate indices of one BCinflow call are decoded in 32-bit arithmetic.
 constexpr long long kMaxInflowCandidates = 0xFFFFFFFFLL;
 
-// Guard cell g of the inflow enumeration, and the axis of its face; the launchers keep every candidate
-// index (and so g) below 2^32, so the decode divides in 32 bits.
+// Guard cell g of the inflow enumeration, and the axis of its face; the launchers
+// keep every candidate index (and so g) below 2^32, so the decode divides in 32 bits.
 __device__ inline int inflow_cell(const KParams& P, const InflowTable& T, uint32_t g, int& ii, int& jj, int& kk,
                                   double& x0, double& y0, double& z0) {
   int f = 0;
@@ -569,13 +569,17 @@ struct OutflowF64 {
 // scan of the block counts, the place pass stores them at *count + the block's
 // offset + their rank.
 //
-// What bounds it: the integer decode of the candidates.  Listing first matters
+// What bounds it: instruction issue (55 % of the slots, FP64 6 %), most of it the
+// integer decode of the candidates.  Listing first matters
 // as much as the early test itself: with a test ahead of the draws but 256
 // candidates a block, nearly every block still waited for one lane's logarithm
 // and sine.  256 x 128 x 128, 10.7 M candidates: 164 us, 267 with the test
 // alone, 612 when every candidate drew its velocity.
-// A block takes `items` candidates per thread: 1 on small grids, so that the
-// device fills, up to 8.
+// A block takes `items` candidates per thread, one for every four blocks an SM that
+// the candidates would fill: 1 on small grids, so that the device fills, up to 8.
+// us with 1 / 2 / 4 / 8 candidates a thread: 16^3 (16 k candidates) 8.1 / 9.2 / 10.9 /
+// 14.2, 32^3 (222 k) 16.5 / 13.8 / 14.5 / 18.4, 48^3 (390 k) 21.8 / 20.7 / 17.0 / 19.8,
+// 77^3 (970 k) 43 / 34 / 29 / 27, 256 x 128 x 128 (5.4 M) 198 / 145 / 109 / 90.
 constexpr int kInflowItems = 8;
 inline int inflow_items(long long candidates) {
   const long long q = candidates / (148LL * 4 * kThreads);
@@ -880,12 +884,12 @@ __device__ __forceinline__ long long fixed_f64(double F, double scale) {
 // species outside 1 .. species, and positions farther than half a cell outside
 // the domain, are skipped.  VEC: the arrays allow 16-byte loads.
 //
-// What bounds it: instruction issue (65 % of the slots; FP64 arithmetic, then
-// 16 shared atomics a particle).  8 M particles on 64^3: 198 us, against 1687
+// What bounds it: instruction issue (70 % of the slots; FP64 arithmetic, then
+// 16 shared atomics a particle).  8 M particles on 64^3: 193 us, against 1684
 // for one particle per lane with warp aggregation by match_any and two
 // partial-mask reductions per corner, three fmod calls and eleven divisions; 1
-// M on 32^3 47 and 218, 2 M on 90^3 (under three per cell) 129 and 648, 4 M in
-// no order 234 and 1424.  Two particles per lane at 64 registers beat four (80
+// M on 32^3 44 and 218, 2 M on 90^3 (under three per cell) 126 and 648, 4 M in
+// no order 221 and 1424.  Two particles per lane at 64 registers beat four (80
 // registers 248 us, 106 registers 261) and eight (128 registers, 521).
 constexpr int kTileF64 = 768;   // entries per warp (two u32 halves)
 constexpr int kTileWarps = 8;

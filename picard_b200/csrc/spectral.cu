@@ -191,9 +191,11 @@ __device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double
 // [k]), B = data.  APPLY (x, inverse): adds the outputs to U's interior instead
 // of storing them.
 //
-// What bounds it: FP64 (4.3 GFLOP of products for both transforms of 256 x 128
-// x 128, 0.12 ms at 37 TFLOP/s), the fragments being read from shared memory
-// once per 4 x 4 tiles (64 of 256 cycles); small grids are bound by the launch.
+// What bounds it: the inverse passes the FP64 tensor pipe (53 % busy, its throttle
+// the first stall), the forward ones the latency of the staging loads, which two
+// blocks of 128 registers per SM do not hide (35 to 39 % busy, long scoreboard);
+// small grids the launch.  4.3 GFLOP of products for both transforms of 256 x 128 x
+// 128 are 0.12 ms at 37 TFLOP/s.
 // Both transforms of 256 x 128 x 128 with the update of U: 286 us in 6 launches,
 // against 498 us in 19 for products with 4 x 4 outputs per thread (as many
 // shared-memory as FP64 cycles), in-place butterflies and a pass of its own for
