@@ -169,8 +169,7 @@ int dalloc(picard_ctx* c, T*& p, size_t n) {
   // stream-ordered: creating or destroying a context does not synchronise
   // the device, so contexts of concurrent runs come and go independently
   cudaError_t e = cudaMallocAsync(&q, bytes, c->st);
-  if (e != cudaSuccess)
-    return fail(PICARD_ERR_CUDA, "cudaMallocAsync(" + std::to_string(bytes) + " B): " + cudaGetErrorString(e));
+  if (e != cudaSuccess) return check_cuda(e, ("cudaMallocAsync(" + std::to_string(bytes) + " B)").c_str());
   c->allocs.push_back(q);
   e = cudaMemsetAsync(q, 0, bytes, c->st);
   if (e != cudaSuccess) return check_cuda(e, "cudaMemsetAsync");

@@ -136,8 +136,10 @@ int solve_f64(picard_ctx* c, double tol, long long smax, int maxit, long long* s
     c->cluster = cluster_plan(c->K);
     if (c->cluster.ctas) {
       void* q = nullptr;
-      PICARD_TRY(dev_alloc(c, &q, sizeof(double) * (size_t)c->m_max * cluster_partials(c->cluster)));
-      c->cluster_partials = static_cast<double*>(q);
+      if (dev_alloc(c, &q, sizeof(double) * (size_t)c->m_max * cluster_partials(c->cluster)) == PICARD_OK)
+        c->cluster_partials = static_cast<double*>(q);
+      else
+        c->cluster = ClusterPlan();  // no room for its partial sums: one launch per sweep needs none
     }
     c->cluster_planned = true;
   }
