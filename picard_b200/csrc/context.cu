@@ -320,8 +320,13 @@ int bc_potentials_async(picard_ctx* c) {
     PICARD_CUDA(launch_bc_potentials_tc(c->K, c->C, c->D, c->U, c->tc_cs, c->tc_partial, c->d_err, c->st));
     return PICARD_OK;
   }
-  if (!c->bc_scratch) PICARD_TRY(dalloc(c, c->bc_scratch, (size_t)bc_direct_scratch(c->K)));
-  PICARD_CUDA(launch_bc_potentials(c->K, c->C, c->D, c->U, c->bc_scratch, c->st));
+  const long long want = bc_direct_scratch(c->K);
+  if (!c->bc_scratch && dalloc(c, c->bc_scratch, (size_t)want) != PICARD_OK) {
+    // no room: the right-hand side's array, which the next solve writes before it reads it
+    PICARD_CUDA(launch_bc_potentials(c->K, c->C, c->D, c->U, c->b, c->K.nodes, c->st));
+    return PICARD_OK;
+  }
+  PICARD_CUDA(launch_bc_potentials(c->K, c->C, c->D, c->U, c->bc_scratch, want, c->st));
   return PICARD_OK;
 }
 

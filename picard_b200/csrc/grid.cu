@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "chain.cuh"
@@ -229,19 +230,21 @@ __global__ void bc_direct_sum_kernel(KParams P, int axis, int groups, const doub
   U[g1] = a1 * scale;
 }
 
-// Plane groups of one axis: about four blocks of 256 threads per SM.
+// Plane groups of one axis: about four blocks of 256 threads per SM, and no more
+// than `room` doubles of partial sums hold (one group always fits a node array).
 struct DirectSplit {
   int n1, n2, nn, bx, by, per, groups;
 };
-inline DirectSplit direct_split(const KParams& P, int axis) {
+inline DirectSplit direct_split(const KParams& P, int axis, long long room) {
   DirectSplit S;
   S.n1 = axis == 0 ? P.ny : P.nx;
   S.n2 = axis == 2 ? P.ny : P.nz;
   S.nn = axis == 0 ? P.nx : axis == 1 ? P.ny : P.nz;
   S.bx = (S.n1 + kBT - 1) / kBT;
   S.by = (S.n2 + kBT - 1) / kBT;
-  const long long want = std::max<long long>(1, 148LL * 4 / ((long long)S.bx * S.by));
-  S.per = int((S.nn + std::min<long long>(want, S.nn) - 1) / std::min<long long>(want, S.nn));
+  const long long want =
+      std::max<long long>(1, std::min({148LL * 4 / ((long long)S.bx * S.by), (long long)S.nn, room / (2LL * S.n1 * S.n2)}));
+  S.per = int((S.nn + want - 1) / want);
   S.groups = (S.nn + S.per - 1) / S.per;
   return S;
 }
@@ -1132,20 +1135,20 @@ cudaError_t launch_finish_flux(const KParams& P, const unsigned long long* Facc,
 long long bc_direct_scratch(const KParams& P) {
   long long most = 0;
   for (int axis = 0; axis < 3; ++axis) {
-    const DirectSplit S = direct_split(P, axis);
+    const DirectSplit S = direct_split(P, axis, LLONG_MAX);
     most = std::max(most, 2LL * S.groups * S.n1 * S.n2);
   }
   return most;
 }
 
 cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, double* scratch,
-                                 cudaStream_t st) {
+                                 long long room, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(U, 0, sizeof(double) * P.nodes, st);  // BCpotentials.f90:36
   if (e != cudaSuccess) return e;
   const int flows[3] = {P.xflow, P.yflow, P.zflow};
   for (int axis = 0; axis < 3; ++axis) {
     if (!flows[axis]) continue;
-    const DirectSplit S = direct_split(P, axis);
+    const DirectSplit S = direct_split(P, axis, room);
     note_launch();
     bc_potentials_kernel<<<dim3(S.bx, S.by, S.groups), dim3(kBT, kBT), 0, st>>>(P, axis, S.per, C, D, scratch);
     if ((e = cudaGetLastError())) return e;

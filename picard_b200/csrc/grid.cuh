@@ -85,10 +85,11 @@ JacobiCoef jacobi_coef(const KParams& P);
 cudaError_t launch_finish_deposit(const KParams& P, const unsigned long long* Nacc, double* N, double* C,
                                   cudaStream_t st);
 cudaError_t launch_finish_flux(const KParams& P, const unsigned long long* Facc, double* F, cudaStream_t st);
-// The direct sum; scratch: bc_direct_scratch(P) doubles.
+// The direct sum; scratch: bc_direct_scratch(P) doubles, or fewer (`room` of them, a
+// node array's at least), with fewer plane groups then.
 long long bc_direct_scratch(const KParams& P);
 cudaError_t launch_bc_potentials(const KParams& P, const double* C, const double* D, double* U, double* scratch,
-                                 cudaStream_t st);
+                                 long long room, cudaStream_t st);
 // Tensor-core BCpotentials (bcpot_tc.cu): scratch sizes (bf16 split charge,
 // FP64 per-CTA partial tiles) and the launch.
 void bcpot_tc_scratch(const KParams& P, long long* cs_elems, long long* partial_elems);
