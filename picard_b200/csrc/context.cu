@@ -470,7 +470,7 @@ int picard_gpu_create(const picard_params* p, int32_t layout, int32_t solver, pi
       return bail(rc);
   }
   const long long nn = s.nodes;
-  if ((rc = dalloc(c, c->d_count, 2)) || (rc = dalloc(c, c->d_info, 32)) ||
+  if ((rc = dalloc(c, c->d_count, 2)) || (rc = dalloc(c, c->d_info, (1 + kJumpRounds) * kInfoStride)) ||
       (rc = dalloc(c, c->Nacc, nn * s.species)) || (rc = dalloc(c, c->N, nn * s.species)) ||
       (rc = dalloc(c, c->C, nn)) || (rc = dalloc(c, c->U, nn)) || (rc = dalloc(c, c->E, 3 * nn)) ||
       (rc = dalloc(c, c->D, s.dsize)) || (rc = dalloc(c, c->b, nn)) || (rc = dalloc(c, c->U1, nn)))
@@ -916,7 +916,7 @@ int picard_gpu_particles_produce(picard_ctx* c, int32_t iteration) {
 // position allocated on first use.  A chain takes about window/survivors
 // dependent loads (the longest several times that), the jumping a few rounds
 // over the window: with the reference's default parameters (30^3, a window of
-// 738,000) the walk took 312 us, the jumping takes 160.
+// 738,000) the walk took 312 us, the jumping takes 75.
 int picard_gpu_bc_outflow(picard_ctx* c) {
   if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
   const long long n = c->num_local;

@@ -86,7 +86,7 @@ struct picard_ctx {
   picard::PartC32 c32 = {};
   int* d_count = nullptr;    // live particle count
   int* d_err = nullptr;      // error word, right after the count
-  int* d_info = nullptr;     // [32] small device results (BCoutflow: window survivors, jump rounds)
+  int* d_info = nullptr;     // small device results (BCoutflow: window survivors, jump rounds)
   long long num_local = 0;   // host mirror of *d_count
 
   // node arrays (plane-major, see common.cuh)

@@ -74,10 +74,12 @@ constexpr int kOutflowWordsPerBlock = 64;
 // above the new count n', to info[0]; stage 2 fills the holes below n', by
 // pointer jumping over the window [n', n) when nxt (n - n' ints) is given, else
 // by following each hole's chain (outflow.cuh).
+constexpr int kJumpRounds = 16;   // four hops each: a window of 2^32 positions
+constexpr int kInfoStride = 32;   // ints between two words of OutflowSplit::info: a cache line
 struct OutflowSplit {
   int stage;
   long long np;  // stage 2: n' (*count after stage 1)
-  int* info;     // [32] stage 1: m, then the words of the jumping rounds
+  int* info;     // [(1 + kJumpRounds) * kInfoStride] stage 1: m, then the words of the jumping rounds
   int* nxt;      // stage 2: pointer-jumping scratch, or null
 };
 // BCoutflow in place, leaving the particles in the reference's order

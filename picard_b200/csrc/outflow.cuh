@@ -250,19 +250,20 @@ __global__ void __launch_bounds__(kOutflowThreads)
 // replaces it by the entry four hops on, so after the rounds every position
 // holds the complement of the survivor its chain ends at.  The holes below n' then
 // take the survivor at the end of the chain from q + S(q), exactly as in
-// outflow_fill_kernel.  The rounds go four hops at a time, and those after one in
-// which nothing moved return at once (256 x 128 x 128, a window of 10.7 M: 7 rounds
-// of 12, 515 us).  That takes a survivor at the end of the window, which the loops
-// with a neutral source have (its particles are the last): a removed position
-// behind the last survivor stands for itself and counts as moved.  Leaving those out
-// gained nothing: without a source the longest chain is about as long as the window
-// (32^3: 9 rounds of 3.5 us either way).
+// outflow_fill_kernel.  The rounds go four hops at a time and those after one in
+// which nothing moved return at once, so the longest chain sets their number.  What
+// a round read of the one before and what it writes for the next lie in cache lines
+// of their own: as neighbouring ints, the blocks' stores held up the loads of the
+// blocks that start, and a round of 0.7 to 4 M positions took 40 to 55 us.  BCoutflow
+// in us with a plain two-hop copy per round, with neighbouring words and now: 64^3 at
+// 32 per cell (a window of 0.8 M) 221, 431 and 181; 128^3 at 16 (1.6 M) 342, 493 and
+// 275; 192 x 128 x 128 at 32 with a source (4.3 M) 626, 668 and 517; 32^3 140, 114, 114.
 
 // m (the survivors in the window, = the holes below n') into info[0]; the
-// rounds' "something moved" words info[1 ..] cleared.
+// rounds' "something moved" words, kInfoStride apart, cleared.
 __global__ void outflow_window_kernel(const uint2* words, const int* block_offsets, const int* survivors, int* info) {
   if (threadIdx.x > 0) {
-    info[threadIdx.x] = 0;
+    if (threadIdx.x <= kJumpRounds) info[threadIdx.x * kInfoStride] = 0;
     return;
   }
   const long long np = *survivors;
@@ -300,6 +301,7 @@ __global__ void outflow_jump_kernel(int* nxt, long long n, const int* survivors,
     int d = v[a - np];
     if (d >= 0) d = v[d - np];
     if (d >= 0) d = v[d - np];
+    if (d == a) continue;  // removed, with no survivor behind it: no hole's chain comes here
     any = true;
     v[i] = d;
   }
@@ -368,8 +370,9 @@ cudaError_t launch_outflow_inplace(const L& lay, long long n, uint2* words, int*
     int round = 0;
     for (long long hops = 1; hops < W; hops <<= 2, ++round) {
       note_launch();
-      outflow_jump_kernel<<<g, 256, 0, st>>>(split->nxt, n, count, round ? split->info + round : nullptr,
-                                             split->info + round + 1);
+      outflow_jump_kernel<<<g, 256, 0, st>>>(split->nxt, n, count,
+                                             round ? split->info + round * kInfoStride : nullptr,
+                                             split->info + (round + 1) * kInfoStride);
     }
     note_launch();
     outflow_fill_jump_kernel<<<nb, kOutflowThreads, 0, st>>>(lay, n, words, block_offsets, count, split->nxt, err);
