@@ -818,40 +818,6 @@ __device__ inline int fold_index(int i, int n, int open) {
   return int(r < 0 ? r + n : r) + 1;
 }
 
-// Warp-aggregated fixed-point deposit of 8 weights (each in [0, 2^40]) at
-// the nodes of `key`'s stencil.  Lanes with equal keys are summed with
-// 32-bit warp reductions of the weights split at bit 18, then one lane per
-// group issues the 8 atomics.
-__device__ inline void deposit8(unsigned long long key, bool active, const long long w[8], const long long nodes[8],
-                                unsigned long long* plane) {
-  unsigned act = __ballot_sync(0xffffffffu, active);
-  if (!active) return;
-  unsigned grp = __match_any_sync(act, key);
-  int lane = threadIdx.x & 31;
-  int leader = __ffs(grp) - 1;
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    long long v = w[q];
-    // Weights are in [-2^40, 2^40]; bias them into [0, 2^41] for the split.
-    unsigned long long u = (unsigned long long)(v + (1LL << kDepositShift));
-    unsigned lo = unsigned(u & 0x3FFFFu), hi = unsigned(u >> 18);
-    unsigned slo = __reduce_add_sync(grp, lo);
-    unsigned shi = __reduce_add_sync(grp, hi);
-    if (lane == leader) {
-      long long cnt = __popc(grp);
-      long long sum = (long long)(((unsigned long long)shi << 18) + (unsigned long long)slo) - cnt * (1LL << kDepositShift);
-      atomicAdd(plane + nodes[q], (unsigned long long)sum);
-    }
-  }
-}
-
-// Grouping key of a particle's stencil: base node (offset by 2, 20 bits per
-// axis) and species.
-__device__ inline unsigned long long stencil_key(int i, int j, int k, int s) {
-  auto c = [](int v) { v += 2; return (unsigned long long)(v < 0 ? 0 : (v > 0xFFFFF ? 0xFFFFF : v)); };
-  return (c(i) | (c(j) << 20) | (c(k) << 40)) << 4 | (unsigned long long)s;
-}
-
 // True when x lies within half a cell of [L_min, L_max] (NaN: false).  There
 // the CIC base node is 0 .. n and both stencil nodes lie inside the
 // ghost-padded box, with non-negative weights.  The reference deposits after
@@ -1080,36 +1046,25 @@ cudaError_t launch_deposit_tile_f64(const KParams& P, const double* x, const dou
   return cudaGetLastError();
 }
 
-__global__ void deposit_f64_kernel(KParams P, PartF64 a, long long n, unsigned long long* Nacc,
-                                   unsigned long long* Facc) {
-  long long stride = (long long)gridDim.x * blockDim.x;
-  long long n_round = ((n + 31) / 32) * 32;
-  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n_round; p += stride) {
-    bool active = p < n;
-    long long w[8] = {0, 0, 0, 0, 0, 0, 0, 0}, nodes[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    double Fw[8];
-    int s = 0;
-    unsigned long long key = ~0ull;
-    if (active) {
-      Cic64 c;
-      cic64(P, a.x[p], a.y[p], a.z[p], c);
-      s = a.sp[p];
-      for (int q = 0; q < 8; ++q) {
-        Fw[q] = c.F[q] / P.dV;
-        w[q] = fixed_f64(c.F[q], kDepositScale / P.dV);
-        int i = fold_index(c.i + kOff[q][0], P.nx, P.xflow), j = fold_index(c.j + kOff[q][1], P.ny, P.yflow),
-            k = fold_index(c.k + kOff[q][2], P.nz, P.zflow);
-        nodes[q] = node_index(P, i, j, k);
-      }
-      key = stencil_key(c.i, c.j, c.k, s);
-    }
-    deposit8(key, active, w, nodes, Nacc + (long long)s * P.nodes);
-    if (Facc && active) {
-      double vel[3] = {a.vx[p], a.vy[p], a.vz[p]};
-      for (int c = 0; c < 3; ++c)
-        for (int q = 0; q < 8; ++q)
-          atomicAdd(Facc + ((long long)s * 3 + c) * P.nodes + nodes[q],
-                    (unsigned long long)__double2ll_rn(Fw[q] * vel[c] * kFluxScale));
+// The flux of GridifyAll (ParticlesGridifyAll.f90:65-160): w v in fixed point, 24
+// atomics a particle straight to global memory, which bound it; its N comes from the
+// tiles above.  GridifyAll's two passes in us, against one kernel with both sums (N
+// aggregated by match_any; 89 registers since the remainders are FMAs, 64 before):
+// 1.05 M particles on 32^3 177 (290, 208), 8.4 M on 64^3 1165 (2075, 1370), 18 M on
+// 100 x 90 x 128 2080 (5230, 3300).
+__global__ void __launch_bounds__(256, 4) flux_f64_kernel(KParams P, PartF64 a, long long n, unsigned long long* Facc) {
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
+    Cic64 c;
+    cic64(P, a.x[p], a.y[p], a.z[p], c);
+    const double vel[3] = {a.vx[p], a.vy[p], a.vz[p]};
+    unsigned long long* plane = Facc + (long long)a.sp[p] * 3 * P.nodes;
+    for (int q = 0; q < 8; ++q) {
+      const int i = fold_index(c.i + kOff[q][0], P.nx, P.xflow), j = fold_index(c.j + kOff[q][1], P.ny, P.yflow),
+                k = fold_index(c.k + kOff[q][2], P.nz, P.zflow);
+      const long long node = node_index(P, i, j, k);
+      const double F = c.F[q] / P.dV;
+      for (int d = 0; d < 3; ++d)
+        atomicAdd(plane + (long long)d * P.nodes + node, (unsigned long long)__double2ll_rn(F * vel[d] * kFluxScale));
     }
   }
 }
@@ -1392,9 +1347,10 @@ cudaError_t launch_advance_velocity_f64(const KParams& P, PartF64 a, long long n
 cudaError_t launch_deposit_f64(const KParams& P, PartF64 a, long long n, unsigned long long* Nacc,
                                unsigned long long* Facc, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  if (!Facc) return launch_deposit_tile_f64<false>(P, a.x, a.y, a.z, a.sp, n, Nacc, st);
+  const cudaError_t e = launch_deposit_tile_f64<false>(P, a.x, a.y, a.z, a.sp, n, Nacc, st);
+  if (e != cudaSuccess || !Facc) return e;
   note_launch();
-  deposit_f64_kernel<<<persistent_grid(n), kThreads, 0, st>>>(P, a, n, Nacc, Facc);
+  flux_f64_kernel<<<persistent_grid(n), kThreads, 0, st>>>(P, a, n, Facc);
   return cudaGetLastError();
 }
 

@@ -523,7 +523,10 @@ __device__ inline void cic_fixed_c32(const C32& c, long long w[8], double F[8]) 
   }
 }
 
-// Warp-aggregated fixed-point deposit (see particles_exact.cu deposit8).
+// Warp-aggregated fixed-point deposit of 8 weights (each in [0, 2^40]) at the
+// nodes of `key`'s stencil: lanes with equal keys are summed with 32-bit warp
+// reductions of the weights split at bit 18, then one lane per group issues the 8
+// atomics.
 __device__ inline void deposit8(unsigned long long key, bool active, const long long w[8], const long long nodes[8],
                                 unsigned long long* plane) {
   unsigned act = __ballot_sync(0xffffffffu, active);
