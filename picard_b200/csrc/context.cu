@@ -909,14 +909,15 @@ int picard_gpu_particles_produce(picard_ctx* c, int32_t iteration) {
 
 // BCoutflow.f90:5-87, in place and in the reference's order (outflow.cuh)
 //
-// In two stages around a read of the survivor count n': when the window
-// [n', n) holds 2^14 positions or more and at least four times its survivors --
-// right after BCinflow has appended every candidate -- its chains are resolved
-// by pointer jumping (outflow.cuh), with scratch of one int per window
-// position allocated on first use.  A chain takes about window/survivors
-// dependent loads (the longest several times that), the jumping a few rounds
-// over the window: with the reference's default parameters (30^3, a window of
-// 738,000) the walk took 312 us, the jumping takes 75.
+// In two stages around a read of the survivor count n' and of m, the survivors of the
+// window [n', n): its chains are followed one by one, or resolved by pointer jumping
+// (outflow.cuh; scratch of one int per window position, allocated on first use).  The
+// jumping launches some ten kernels, which a call that the host waits for pays in
+// full: about 100 us up to windows of 2 x 10^5.  The walk takes longer with the window
+// and, at equal windows, with the survivors its chains pass.  us of the call, walk and
+// jumping: few survivors, W 42 k, m 50 76 / 94; 85 k, 112 91 / 103; 131 k, 30 98 / 97; 209 k,
+// 53 155 / 116; 526 k, 138 242 / 145; many, W 16 k, m 400 164 / 98; 55 k, 1,340 190 / 102; 170 k,
+// 4,290 186 / 109; 738 k, 18.8 k (the reference's default parameters) 283 / 162.
 int picard_gpu_bc_outflow(picard_ctx* c) {
   if (!c) return fail(PICARD_ERR_BAD_ARG, "ctx is NULL");
   const long long n = c->num_local;
@@ -928,7 +929,7 @@ int picard_gpu_bc_outflow(picard_ctx* c) {
   const long long np = c->num_local, window = n - np, m = c->h_pinned_i[6];
   sp.stage = 2;
   sp.np = np;
-  if (window >= (1LL << 14) && window >= 4 * m) {
+  if (window >= 4 * m && (window >= (1LL << 17) || (window >= (1LL << 14) && 128 * m >= window))) {
     if (c->jump_cap < window) {
       const long long cap = std::min<long long>(c->capacity, std::max<long long>(window, 2 * c->jump_cap));
       if (c->jump) {

@@ -1,5 +1,6 @@
 """BCoutflow's fill by pointer jumping (outflow.cuh), whose rounds end when nothing
-moves: windows of 2^14 positions and more with their survivors at the front, in the
+moves, and, for windows under 2^17 positions with few survivors, by following the
+chains: windows of 2^14 positions and more with their survivors at the front, in the
 middle, at the very end, alone, in one run, at random, or none at all -- so that the
 removed positions behind the last survivor, which stand for themselves, are many, few
 or none, and chains of one hop and of thousands are resolved.
@@ -16,17 +17,17 @@ pytestmark = pytest.mark.gpu
 KEPT = 20_000
 
 
-@pytest.mark.parametrize("window", [1 << 14, 50_001, 100_000])
+@pytest.mark.parametrize("window", [1 << 14, 50_001, 100_000, 1 << 17, 200_003])
 @pytest.mark.parametrize("where", ["none", "first", "last", "middle", "front_run", "end_run", "random", "sparse"])
 def test_jumping_leaves_the_reference_order(where, window):
     pl = small_plasma(n=8, ppc=1, seed=3)
-    pl.max_per_proc = 200_000
+    pl.max_per_proc = 300_000
     p, o, g = make(pl, **F64)
     rng = np.random.default_rng(window)
     n = KEPT + window
     at = {"none": [], "first": [0], "last": [window - 1], "middle": [window // 2],
           "front_run": np.arange(300), "end_run": np.arange(window - 300, window),
-          "random": np.sort(rng.permutation(window)[:window // 5]), "sparse": np.sort(rng.permutation(window)[:40])}[where]
+          "random": np.sort(rng.permutation(window)[:min(window // 5, KEPT)]), "sparse": np.sort(rng.permutation(window)[:40])}[where]
     alive = np.zeros(n, bool)
     alive[:KEPT] = True
     alive[KEPT + np.asarray(at, int)] = True
