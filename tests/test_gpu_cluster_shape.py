@@ -67,3 +67,23 @@ def test_a_grid_that_does_not_fit_is_refused(dims, kw, flows):
         assert e.value.code == capi.ERR_STATE
         assert s.get_option(capi.OPT_SWEEP_CLUSTER) == 0
         s.set_option(capi.OPT_SWEEP_CLUSTER, 0)
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 16), (33, 17, 9), (30, 64, 63)])
+def test_every_sweep_of_a_round_has_its_residual(dims, monkeypatch, capfd):
+    """Rounds of 1, 3, 5 and 7 sweeps (2 maxit + 1, no stop): the solver's log of a
+    round, with the sum of its residuals to the last bit, for both kernels."""
+    p = boxed(*dims)
+    C = blobs(O.OracleState(p), p, seed=3, width=20.0)
+    monkeypatch.setenv("PICARD_SOLVE_LOG", "1")
+    logs = []
+    with Simulation(p, derive=False, **REFINE) as s:
+        for on in (1, 0):
+            s.set_option(capi.OPT_SWEEP_CLUSTER, on)
+            capfd.readouterr()
+            for maxit in (0, 1, 2, 3):
+                s.set_field(capi.FIELD_C, C)
+                s.set_field(capi.FIELD_U, np.zeros_like(C))
+                assert s.calc_epotential(maxerr=1e-30, maxit=maxit) == 2 * maxit + 1
+            logs.append([x for x in capfd.readouterr().err.splitlines() if x.startswith("picard solve")])
+    assert len(logs[0]) == 4 and logs[0] == logs[1]
